@@ -489,20 +489,27 @@ struct Launcher {
 
     // iteration t of a check period (t = 0 first): the Halpern weight uses t;
     // tz: a check or the final selection reads this iteration's T(z)
-    void iteration(long long t, cudaStream_t s, bool tz) {
+    // chained: the iteration before it was launched just before
+    void iteration(long long t, cudaStream_t s, bool tz, bool chained = true) {
         const int first = t == 0 ? 1 : 0;
         fi32.hk = fi64.hk = static_cast<int>(t);
         fi32.tz = fi64.tz = tz ? 1 : 0;
+        // the first pass of a period follows the restart kernel in full order
+        const bool p = chained && !first;
         if (prec == PDHG_PREC_FP64_EXACT) {
-            launch_exact_primal(ei, first, s);
-            launch_exact_dual(ei, first, s);
+            launch_exact_primal(ei, first, s, p && c.lp.m > 0);
+            launch_exact_dual(ei, first, s, c.lp.n > 0);
             c.launches += 2;
         } else if (prec == PDHG_PREC_MIXED) {
-            c.launches += launch_fast_primal(fi32, first, s, &c.fork);
-            c.launches += launch_fast_dual(fi32, first, s, &c.fork);
+            const bool one = fast_early(fi32);
+            fi32.early = one ? 1 : 0;
+            c.launches += launch_fast_primal(fi32, first, s, &c.fork, p && one);
+            c.launches += launch_fast_dual(fi32, first, s, &c.fork, one);
         } else {
-            c.launches += launch_fast_primal(fi64, first, s, &c.fork);
-            c.launches += launch_fast_dual(fi64, first, s, &c.fork);
+            const bool one = fast_early(fi64);
+            fi64.early = one ? 1 : 0;
+            c.launches += launch_fast_primal(fi64, first, s, &c.fork, p && one);
+            c.launches += launch_fast_dual(fi64, first, s, &c.fork, one);
         }
     }
     void check(long long period, cudaStream_t s) {
@@ -761,7 +768,7 @@ int run_loop(Ctx& c, Launcher& L, const pdhg_options& o, long long budget, long 
     while (p < n_periods && p * period < traced && !c.mail->done) {
         poll_stop();
         for (long long t = 0; t < period; ++t) {
-            L.iteration(t, c.stream, t == period - 1);
+            L.iteration(t, c.stream, t == period - 1, false);
             const long long k = iter0 + p * period + t;
             if (k < o.trace_iters) {
                 int rc = trace_copy(c, L.prec, k, o);
@@ -837,7 +844,7 @@ int run_loop(Ctx& c, Launcher& L, const pdhg_options& o, long long budget, long 
         poll_stop();
         if (!stop_sent) {
             for (long long t = 0; t < tail; ++t) {
-                L.iteration(t, c.stream, t == tail - 1);
+                L.iteration(t, c.stream, t == tail - 1, iter0 + n_periods * period >= o.trace_iters);
                 const long long k = iter0 + n_periods * period + t;
                 if (k < o.trace_iters) {
                     int rc = trace_copy(c, L.prec, k, o);

@@ -286,8 +286,9 @@ struct ExactIter {
     Iterates<double> it;
     DevState* st;
 };
-void launch_exact_primal(const ExactIter& a, int first, cudaStream_t s);
-void launch_exact_dual(const ExactIter& a, int first, cudaStream_t s);
+// early (here and below): the pass follows the pass before it directly
+void launch_exact_primal(const ExactIter& a, int first, cudaStream_t s, bool early = false);
+void launch_exact_dual(const ExactIter& a, int first, cudaStream_t s, bool early = false);
 
 struct ExactCheck {
     DevCsr A, AT, Ao, ATo;
@@ -313,6 +314,7 @@ struct FastIter {
     DevState* st;
     int hk = 0;  // the iteration's index in its check period (Halpern weight)
     int tz = 1;  // Halpern: this iteration stores T(z) (lean mode: only before a check / the end)
+    int early = 0;  // fast_early: the kernels that may be launched early
 };
 // A pass's short-row, long-row and row-slice kernels touch disjoint rows and
 // only read the gathered vector, so they may run side by side: with a
@@ -325,12 +327,16 @@ struct PassFork {
 };
 template <class T>
 int launch_fast_primal(const FastIter<T>& a, int first, cudaStream_t s,
-                       const PassFork* f = nullptr);  // kernels launched
+                       const PassFork* f = nullptr, bool early = false);  // kernels launched
 template <class T>
 int launch_fast_dual(const FastIter<T>& a, int first, cudaStream_t s,
-                     const PassFork* f = nullptr);
+                     const PassFork* f = nullptr, bool early = false);
 template <class T>
 int fast_launches_per_iteration(const FastIter<T>& a);
+// Whether the passes may follow one another early (FastIter::early): one kernel
+// each, of a small or middling LP.
+template <class T>
+bool fast_early(const FastIter<T>& a);
 // Once per device, before the first launch and outside any stream capture:
 // records how many CTAs of the persistent iteration kernels are resident per
 // device (their grids). 0 on success.

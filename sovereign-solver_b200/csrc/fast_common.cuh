@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "pass.cuh"
 
 namespace pdhg {
 namespace {
@@ -234,19 +235,19 @@ struct Vec16<double> {
 // sits in column k + off, so the W entries are consecutive: one vector load
 // when `va` (the gathered vector aligned with the row's values), else W
 // scalar loads at computed addresses. Otherwise the columns come from `c`.
-template <class T>
+template <class T, bool EARLY>
 __device__ __forceinline__ typename Vec16<T>::type gather16(const T* __restrict__ xg, int k, int off,
                                                             bool va) {
-    if (va) return __ldg(reinterpret_cast<const typename Vec16<T>::type*>(xg + k + off));
+    if (va) return gather_ld<EARLY>(reinterpret_cast<const typename Vec16<T>::type*>(xg + k + off));
     typename Vec16<T>::type g;
     if constexpr (std::is_same<T, float>::value) {
-        g.x = __ldg(xg + k + off);
-        g.y = __ldg(xg + k + off + 1);
-        g.z = __ldg(xg + k + off + 2);
-        g.w = __ldg(xg + k + off + 3);
+        g.x = gather_ld<EARLY>(xg + k + off);
+        g.y = gather_ld<EARLY>(xg + k + off + 1);
+        g.z = gather_ld<EARLY>(xg + k + off + 2);
+        g.w = gather_ld<EARLY>(xg + k + off + 3);
     } else {
-        g.x = __ldg(xg + k + off);
-        g.y = __ldg(xg + k + off + 1);
+        g.x = gather_ld<EARLY>(xg + k + off);
+        g.y = gather_ld<EARLY>(xg + k + off + 1);
     }
     return g;
 }
@@ -254,10 +255,10 @@ __device__ __forceinline__ typename Vec16<T>::type gather16(const T* __restrict_
 // Long-row dot product, one CTA: 128-bit loads of values and column indices
 // on the aligned body (four of each in flight per thread), scalar head and
 // tail. The matrix is streamed (evict-first, ld.global.cs) so that the
-// gathered vector keeps its L2 lines; gathers go through the read-only path.
+// gathered vector keeps its L2 lines; gathers as gather_ld says.
 // DENSE: the columns are k + off (no index loads); the sum order is the same
 // either way.
-template <class T, bool DENSE = false>
+template <class T, bool DENSE = false, bool EARLY = false>
 __device__ __forceinline__ T long_row_dot(const int32_t* __restrict__ ci,
                                           const T* __restrict__ v, const T* __restrict__ xg,
                                           int b, int e, int off = 0) {
@@ -270,7 +271,7 @@ __device__ __forceinline__ T long_row_dot(const int32_t* __restrict__ ci,
     const bool va = DENSE && ((bA + off) & (W - 1)) == 0;
     auto col = [&](int k) { return DENSE ? k + off : __ldcs(ci + k); };
     T acc = T(0);
-    for (int k = b + threadIdx.x; k < bA; k += kBlock) acc += __ldcs(v + k) * __ldg(xg + col(k));
+    for (int k = b + threadIdx.x; k < bA; k += kBlock) acc += __ldcs(v + k) * gather_ld<EARLY>(xg + col(k));
     const int nvec = (e - bA) / W;
     const V* vv = reinterpret_cast<const V*>(v + bA);
     const I* cc = reinterpret_cast<const I*>(ci + bA);
@@ -286,7 +287,7 @@ __device__ __forceinline__ T long_row_dot(const int32_t* __restrict__ ci,
             const bool ok = q + u * kBlock < nvec;
             const int qq = ok ? q + u * kBlock : 0;
             w[u] = ok ? __ldcs(vv + qq) : V{};
-            if (DENSE) g[u] = ok ? gather16<T>(xg, bA + W * qq, off, va) : V{};
+            if (DENSE) g[u] = ok ? gather16<T, EARLY>(xg, bA + W * qq, off, va) : V{};
             else c[u] = ok ? __ldcs(cc + qq) : I{};
         }
 #pragma unroll
@@ -296,17 +297,17 @@ __device__ __forceinline__ T long_row_dot(const int32_t* __restrict__ ci,
                 if (DENSE) {
                     acc += w[u].x * g[u].x + w[u].y * g[u].y + w[u].z * g[u].z + w[u].w * g[u].w;
                 } else {
-                    acc += w[u].x * __ldg(xg + c[u].x) + w[u].y * __ldg(xg + c[u].y) +
-                           w[u].z * __ldg(xg + c[u].z) + w[u].w * __ldg(xg + c[u].w);
+                    acc += w[u].x * gather_ld<EARLY>(xg + c[u].x) + w[u].y * gather_ld<EARLY>(xg + c[u].y) +
+                           w[u].z * gather_ld<EARLY>(xg + c[u].z) + w[u].w * gather_ld<EARLY>(xg + c[u].w);
                 }
             } else {
                 if (DENSE) acc += w[u].x * g[u].x + w[u].y * g[u].y;
-                else acc += w[u].x * __ldg(xg + c[u].x) + w[u].y * __ldg(xg + c[u].y);
+                else acc += w[u].x * gather_ld<EARLY>(xg + c[u].x) + w[u].y * gather_ld<EARLY>(xg + c[u].y);
             }
         }
     }
     for (int k = bA + nvec * W + threadIdx.x; k < e; k += kBlock)
-        acc += __ldcs(v + k) * __ldg(xg + col(k));
+        acc += __ldcs(v + k) * gather_ld<EARLY>(xg + col(k));
     return block_total(acc);
 }
 
@@ -317,16 +318,11 @@ __device__ __forceinline__ T long_row_dot(const int32_t* __restrict__ ci,
 #endif
 constexpr int kWarpUnroll = PDHG_WARP_UNROLL;
 
-// Load used for the x / y gathers of warp_row_dot (a build knob).
-#ifndef PDHG_GATHER
-#define PDHG_GATHER __ldg
-#endif
-
 // The same dot by one warp (rows of kLongRow..kHugeRow entries): 128-bit loads
 // of values and indices, kWarpUnroll of each in flight per lane, then a
 // shuffle reduction -- no block barrier, so a CTA's eight warps finish
 // independently. Every lane returns the total.
-template <class T>
+template <class T, bool EARLY = false>
 __device__ __forceinline__ T warp_row_dot(const int32_t* __restrict__ ci,
                                           const T* __restrict__ v, const T* __restrict__ xg,
                                           int b, int e, int off = kNotDense) {
@@ -340,7 +336,7 @@ __device__ __forceinline__ T warp_row_dot(const int32_t* __restrict__ ci,
     if (bA > e) bA = e;
     auto col = [&](int k) { return dense ? k + off : __ldcs(ci + k); };
     T acc = T(0);
-    for (int k = b + lane; k < bA; k += 32) acc += __ldcs(v + k) * PDHG_GATHER(xg + col(k));
+    for (int k = b + lane; k < bA; k += 32) acc += __ldcs(v + k) * gather_ld<EARLY>(xg + col(k));
     const int nvec = (e - bA) / W;
     const V* vv = reinterpret_cast<const V*>(v + bA);
     // rounds of up to kWarpUnroll vectors per lane in flight; the last round
@@ -360,8 +356,8 @@ __device__ __forceinline__ T warp_row_dot(const int32_t* __restrict__ ci,
 #pragma unroll
             for (int u = 0; u < kWarpUnroll; ++u)
                 if (q + 32 * u < nvec)
-                    acc += w[u].x * PDHG_GATHER(xg + c[u].x) + w[u].y * PDHG_GATHER(xg + c[u].y) +
-                           w[u].z * PDHG_GATHER(xg + c[u].z) + w[u].w * PDHG_GATHER(xg + c[u].w);
+                    acc += w[u].x * gather_ld<EARLY>(xg + c[u].x) + w[u].y * gather_ld<EARLY>(xg + c[u].y) +
+                           w[u].z * gather_ld<EARLY>(xg + c[u].z) + w[u].w * gather_ld<EARLY>(xg + c[u].w);
         }
     } else {
         const int2* ci2 = reinterpret_cast<const int2*>(ci + bA);
@@ -378,11 +374,11 @@ __device__ __forceinline__ T warp_row_dot(const int32_t* __restrict__ ci,
 #pragma unroll
             for (int u = 0; u < kWarpUnroll; ++u)
                 if (q + 32 * u < nvec)
-                    acc += w[u].x * PDHG_GATHER(xg + c[u].x) + w[u].y * PDHG_GATHER(xg + c[u].y);
+                    acc += w[u].x * gather_ld<EARLY>(xg + c[u].x) + w[u].y * gather_ld<EARLY>(xg + c[u].y);
         }
     }
     for (int k = bA + nvec * W + lane; k < e; k += 32)
-        acc += __ldcs(v + k) * PDHG_GATHER(xg + col(k));
+        acc += __ldcs(v + k) * gather_ld<EARLY>(xg + col(k));
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     return acc;
 }
@@ -469,6 +465,57 @@ __device__ __forceinline__ EpiIn<T> epi_load(const Iterates<T>& it, const PV<T>&
         else in.ps = fresh ? T(0) : __ldcs(it.ysum + r);
     }
     return in;
+}
+
+// The same in two parts for the kernels launched early: what no iteration
+// changes (c, the bounds, the Halpern anchors, which only a restart moves),
+// loaded before the wait for the pass before, and what the passes write.
+template <class T, bool PRIMAL>
+__device__ __forceinline__ EpiIn<T> epi_load_fixed(const Iterates<T>& it, const PV<T>& pv, int r) {
+    EpiIn<T> in{};
+    if (PRIMAL) {
+        in.a = __ldcs(pv.c + r);
+        in.lo = pv.ub ? pv.lo_u : __ldcs(pv.lo + r);
+        in.hi = pv.ub ? pv.hi_u : __ldcs(pv.hi + r);
+        if (it.halpern) in.ps = __ldcs(it.xa + r);
+    } else {
+        in.lo = __ldcs(pv.rlo + r);
+        in.hi = __ldcs(pv.rhi + r);
+        if (it.halpern) in.ps = __ldcs(it.ya + r);
+    }
+    return in;
+}
+template <class T, bool PRIMAL>
+__device__ __forceinline__ void epi_load_moving(EpiIn<T>& in, const Iterates<T>& it, int r, int first, bool fresh,
+                                                const Hw<T>& hw) {
+    if (PRIMAL) {
+        if (it.lean) {
+            in.b = hw.wp == T(0) ? in.ps : halpern_mix<T>(hw.wp, coherent_ld(it.xbar + r), in.ps);
+            return;
+        }
+        in.b = coherent_ld(it.x + r);
+        if (it.halpern) return;
+        if constexpr (std::is_same<T, float>::value) in.ps = first ? T(0) : coherent_ld(it.psx + r);
+        else in.ps = fresh ? T(0) : coherent_ld(it.xsum + r);
+    } else {
+        in.a = coherent_ld(it.y + r);
+        in.b = coherent_ld(it.s + r);
+        if (it.halpern) return;
+        if constexpr (std::is_same<T, float>::value) in.ps = first ? T(0) : coherent_ld(it.psy + r);
+        else in.ps = fresh ? T(0) : coherent_ld(it.ysum + r);
+    }
+}
+// ... both at once, past the wait (EARLY) or in a kernel without one
+template <class T, bool PRIMAL, bool EARLY>
+__device__ __forceinline__ EpiIn<T> pass_operands(const Iterates<T>& it, const PV<T>& pv, int r, int first,
+                                                  bool fresh, const Hw<T>& hw) {
+    if constexpr (EARLY) {
+        EpiIn<T> in = epi_load_fixed<T, PRIMAL>(it, pv, r);
+        epi_load_moving<T, PRIMAL>(in, it, r, first, fresh, hw);
+        return in;
+    } else {
+        return epi_load<T, PRIMAL>(it, pv, r, first, fresh, hw);
+    }
 }
 
 // primal: x+ = proj(x - tau (c - aty)), x_bar = 2x+ - x, sum += x+

@@ -22,6 +22,7 @@
 
 #include "engine.cuh"
 #include "ordered.cuh"
+#include "pass.cuh"
 
 namespace pdhg {
 
@@ -98,10 +99,41 @@ __host__ __device__ inline int blocks_for(int64_t n) {
 // One PDHG iteration (src/l1/pdhg.cpp:295-331)
 // ---------------------------------------------------------------------------
 
+// The row's dot of an iteration's pass (row_dot's order and rounding) with the
+// loads that do not depend on the pass before ahead of `wait`: a thread row's
+// first kHeld entries, a warp row's first two rounds. g reads the gathered
+// vector.
+constexpr int kHeld = 8;
+template <class G, class W>
+__device__ __forceinline__ double pass_row_dot(const RowTask& t, const DevCsr& M, G g, double init, W wait) {
+    const int b = M.rp[t.row], e = M.rp[t.row + 1];
+    const int32_t* __restrict__ ci = M.ci;
+    const double* __restrict__ v = M.v64;
+    if (!t.warp) {
+        int c[kHeld];
+        double w[kHeld];
+#pragma unroll
+        for (int u = 0; u < kHeld; ++u) {
+            c[u] = b + u < e ? ci[b + u] : 0;
+            w[u] = b + u < e ? v[b + u] : 0.0;
+        }
+        wait();
+        double acc = init, p[kHeld];
+#pragma unroll
+        for (int u = 0; u < kHeld; ++u) p[u] = b + u < e ? __dmul_rn(w[u], g(c[u])) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kHeld; ++u)
+            if (b + u < e) acc = __dadd_rn(acc, p[u]);
+        return b + kHeld < e ? ordered_dot(b + kHeld, e, ci, v, g, acc) : acc;
+    }
+    return ordered_dot_warp_pipelined(b, e, ci, v, g, init, warp_stage2(), wait);
+}
+
 // K1: per column j -- grad = c - A^T y (pdhg.cpp:296-297: grad starts at c,
 // then every row adds val * (-y_r) in row order), x_new = proj(x - tau grad),
 // x_bar = 2 x_new - x, Cesaro sum.
 __global__ void __launch_bounds__(kBlock) ex_primal(ExactIter a, int first) {
+    pass_begin();
     DevState* st = a.st;
     if (first && blockIdx.x == 0 && threadIdx.x == 0) st->restart = 0;  // consumed by ex_restart
     if (st->done) return;
@@ -109,37 +141,50 @@ __global__ void __launch_bounds__(kBlock) ex_primal(ExactIter a, int first) {
     if (t.row < 0) return;
     const int j = t.row;
     const double* y = a.it.y;
-    const double g = row_dot(t, a.AT, [y](int i) { return -y[i]; }, a.P.c[j]);
+    const double tau = st->tau, lo = a.P.lo[j], hi = a.P.hi[j];
+    const bool fresh = first && st->fresh;
+    double xo = 0.0, sum = 0.0;
+    const double g = pass_row_dot(t, a.AT, [y](int i) { return -coherent_ld(y + i); }, a.P.c[j], [&]() {
+        pass_wait();
+        if (!t.lead) return;
+        xo = coherent_ld(a.it.x + j);
+        sum = fresh ? 0.0 : coherent_ld(a.it.xsum + j);
+    });
     if (!t.lead) return;
-    const double xo = a.it.x[j];
-    const double xn = clampd(__dadd_rn(xo, __dmul_rn(-st->tau, g)), a.P.lo[j], a.P.hi[j]);
+    const double xn = clampd(__dadd_rn(xo, __dmul_rn(-tau, g)), lo, hi);
     a.it.xbar[j] = __dadd_rn(2.0 * xn, -xo);  // scale(2.0) then axpy(-1.0, x)
     a.it.x[j] = xn;
-    const bool fresh = first && st->fresh;
-    a.it.xsum[j] = fresh ? xn : __dadd_rn(a.it.xsum[j], xn);
+    a.it.xsum[j] = fresh ? xn : __dadd_rn(sum, xn);
 }
 
 // K2: per row i -- s_new = proj(s - tau y), s_bar = 2 s_new - s,
 // k = -(A x_bar) + s_bar, y += sigma k (pdhg.cpp:302-318), Cesaro sum.
 __global__ void __launch_bounds__(kBlock) ex_dual(ExactIter a, int first) {
+    pass_begin();
     DevState* st = a.st;
     if (st->done) return;
     const RowTask t = row_task(a.A, blockIdx.x);
     if (t.row < 0) return;
     const int i = t.row;
     const double* xbar = a.it.xbar;
-    const double sum = row_dot(t, a.A, [xbar](int j) { return xbar[j]; }, 0.0);
+    const double tau = st->tau, sigma = st->sigma, lo = a.P.rlo[i], hi = a.P.rhi[i];
+    const bool fresh = first && st->fresh;
+    double yo = 0.0, so = 0.0, ysum = 0.0;
+    const double sum = pass_row_dot(t, a.A, [xbar](int j) { return coherent_ld(xbar + j); }, 0.0, [&]() {
+        pass_wait();
+        if (!t.lead) return;
+        yo = coherent_ld(a.it.y + i);
+        so = coherent_ld(a.it.s + i);
+        ysum = fresh ? 0.0 : coherent_ld(a.it.ysum + i);
+    });
     if (!t.lead) return;
-    const double yo = a.it.y[i];
-    const double so = a.it.s[i];
-    const double sn = clampd(__dadd_rn(so, __dmul_rn(-st->tau, yo)), a.P.rlo[i], a.P.rhi[i]);
+    const double sn = clampd(__dadd_rn(so, __dmul_rn(-tau, yo)), lo, hi);
     const double sbar = __dadd_rn(2.0 * sn, -so);
     const double kb = __dadd_rn(-sum, sbar);
-    const double yn = __dadd_rn(yo, __dmul_rn(st->sigma, kb));
+    const double yn = __dadd_rn(yo, __dmul_rn(sigma, kb));
     a.it.y[i] = yn;
     a.it.s[i] = sn;
-    const bool fresh = first && st->fresh;
-    a.it.ysum[i] = fresh ? yn : __dadd_rn(a.it.ysum[i], yn);
+    a.it.ysum[i] = fresh ? yn : __dadd_rn(ysum, yn);
 }
 
 // ---------------------------------------------------------------------------
@@ -867,11 +912,11 @@ inline int grid64(int64_t n) { return static_cast<int>((n + kBlock - 1) / kBlock
 
 int exact_check_grid(const DevCsr& A, const DevCsr& AT) { return mat_blocks(A) + mat_blocks(AT); }
 
-void launch_exact_primal(const ExactIter& a, int first, cudaStream_t s) {
-    if (a.AT.rows > 0) ex_primal<<<mat_blocks(a.AT), kBlock, 0, s>>>(a, first);
+void launch_exact_primal(const ExactIter& a, int first, cudaStream_t s, bool early) {
+    if (a.AT.rows > 0) launch_pass(ex_primal, mat_blocks(a.AT), early, s, a, first);
 }
-void launch_exact_dual(const ExactIter& a, int first, cudaStream_t s) {
-    if (a.A.rows > 0) ex_dual<<<mat_blocks(a.A), kBlock, 0, s>>>(a, first);
+void launch_exact_dual(const ExactIter& a, int first, cudaStream_t s, bool early) {
+    if (a.A.rows > 0) launch_pass(ex_dual, mat_blocks(a.A), early, s, a, first);
 }
 void launch_exact_check(const ExactCheck& a, cudaStream_t s) {
     const int g1 = mat_blocks(a.A) + mat_blocks(a.AT);

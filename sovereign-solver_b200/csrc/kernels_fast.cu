@@ -123,23 +123,24 @@ __device__ __forceinline__ T mul_rn(T a, T b) {
 
 // The dot of long row `row` over entries [b, e), by one CTA (block-uniform)
 // or one warp (warp-uniform); a dense row computes its columns.
-template <class T>
+template <class T, bool EARLY>
 __device__ __forceinline__ T cta_row_dot(const DevCsr& M, const T* vals, const T* xg, int row, int b,
                                          int e) {
     const int off = M.dense_off ? __ldg(M.dense_off + row) : kNotDense;
-    if (off != kNotDense) return long_row_dot<T, true>(M.ci, vals, xg, b, e, off);
-    return long_row_dot<T>(M.ci, vals, xg, b, e);
+    if (off != kNotDense) return long_row_dot<T, true, EARLY>(M.ci, vals, xg, b, e, off);
+    return long_row_dot<T, false, EARLY>(M.ci, vals, xg, b, e);
 }
-template <class T>
+template <class T, bool EARLY>
 __device__ __forceinline__ T warp_dot(const DevCsr& M, const T* vals, const T* xg, int row, int b,
                                       int e) {
-    return warp_row_dot<T>(M.ci, vals, xg, b, e, M.dense_off ? __ldg(M.dense_off + row) : kNotDense);
+    return warp_row_dot<T, EARLY>(M.ci, vals, xg, b, e, M.dense_off ? __ldg(M.dense_off + row) : kNotDense);
 }
 
 // PRIMAL = true: rows of A^T gather y; false: rows of A gather x_bar.
-template <class T, int VW, bool PRIMAL>
+template <class T, int VW, bool PRIMAL, bool EARLY>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? PDHG_SHORT_MIN_CTAS : PDHG_SHORT_MIN_CTAS_F64)
     fast_iter(FastIter<T> a, int first, int reset) {
+    if (EARLY) pass_begin();
     DevState* st = a.st;
     iter_reset(st, reset);
     if (st->done) return;
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? PDHG_SHORT_MIN_CTAS :
     const int r = (blockIdx.x * kBlock + threadIdx.x) / VW;
     if (r >= M.rows) return;
     EpiIn<T> in{};
-    if (lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
+    if (!EARLY && lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
     int b, e;
     if (M.rp_stride > 0) {  // rows of one length: the extent is computed
         b = r * M.rp_stride;
@@ -164,32 +165,50 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? PDHG_SHORT_MIN_CTAS :
         e = __ldcs(M.rp + r + 1);
     }
     if (e - b > M.short_max) return;  // fast_iter_long handles it
-    T acc = T(0);
+    if (EARLY && lane == 0) in = epi_load_fixed<T, PRIMAL>(a.it, pv, r);
     if (VW == 1 && M.rp_stride == 2 && pair_aligned<T>(M.ci, vals)) {
         // two entries per row (the columns of a transportation LP): one
         // 8-byte index load and one vector value load, the same sum order as
         // the loop below
         const int2 c2 = __ldcs(reinterpret_cast<const int2*>(M.ci + b));
         const typename Pair<T>::type v2 = __ldcs(reinterpret_cast<const typename Pair<T>::type*>(vals + b));
-        const T g0 = __ldg(xg + c2.x), g1 = __ldg(xg + c2.y);
-        acc = fma_rn<T>(v2.y, g1, mul_rn<T>(v2.x, g0));
-        epi_store<T, PRIMAL>(a.it, r, acc, in, tau, sigma, hw, a.tz);
+        if (EARLY) {
+            pass_wait();
+            epi_load_moving<T, PRIMAL>(in, a.it, r, first, fresh, hw);
+        }
+        const T g0 = gather_ld<EARLY>(xg + c2.x), g1 = gather_ld<EARLY>(xg + c2.y);
+        epi_store<T, PRIMAL>(a.it, r, fma_rn<T>(v2.y, g1, mul_rn<T>(v2.x, g0)), in, tau, sigma, hw, a.tz);
         return;
     }
     // rounds of four entries per lane: the index and value loads of a round
-    // are all in flight before its gathers, the gathers before the adds
-    for (int k0 = b + lane; k0 < e; k0 += 4 * VW) {
-        int c[4];
-        T v[4];
+    // are all in flight before its gathers, the gathers before the adds; the
+    // first round's are loaded before the wait for the pass before
+    T acc = T(0);
+    int k0 = b + lane;
+    int c[4];
+    T v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int k = k0 + u * VW;
+        c[u] = k < e ? __ldcs(M.ci + k) : 0;
+        v[u] = k < e ? __ldcs(vals + k) : T(0);
+    }
+    if (EARLY) {
+        pass_wait();
+        if (lane == 0) epi_load_moving<T, PRIMAL>(in, a.it, r, first, fresh, hw);
+    }
+    for (;;) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u * VW < e) acc += v[u] * gather_ld<EARLY>(xg + c[u]);
+        k0 += 4 * VW;
+        if (k0 >= e) break;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int k = k0 + u * VW;
             c[u] = k < e ? __ldcs(M.ci + k) : 0;
             v[u] = k < e ? __ldcs(vals + k) : T(0);
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (k0 + u * VW < e) acc += v[u] * __ldg(xg + c[u]);
     }
     if (VW > 1) acc = group_sum(acc, VW);
     if (lane == 0) epi_store<T, PRIMAL>(a.it, r, acc, in, tau, sigma, hw, a.tz);
@@ -250,10 +269,11 @@ constexpr int uniform_min_ctas() {
     return sizeof(T) == 8 ? PDHG_UNIFORM_MIN_CTAS_F64 : (E == 2 ? PDHG_UNIFORM_MIN_CTAS : PDHG_UNIFORM_MIN_CTAS_E4);
 }
 
-template <class T, int E, int VW, bool PRIMAL>
+template <class T, int E, int VW, bool PRIMAL, bool EARLY>
 __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     fast_iter_uniform(FastIter<T> a, int first, int reset) {
     constexpr int S = E * VW;
+    if (EARLY) pass_begin();
     DevState* st = a.st;
     iter_reset(st, reset);
     if (st->done) return;
@@ -269,22 +289,27 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     int r = (blockIdx.x * kBlock + static_cast<int>(threadIdx.x)) / VW;
     if (r >= M.rows) return;  // group-uniform
     EpiIn<T> in{};
-    if (lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
+    if (!EARLY && lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
+    if (EARLY && lane == 0) in = epi_load_fixed<T, PRIMAL>(a.it, pv, r);
     int c[E];
     T v[E];
     load_idx<E>(M.ci + static_cast<int64_t>(r) * S + lane * E, c);
     load_vals<T, E>(vals + static_cast<int64_t>(r) * S + lane * E, v);
+    if (EARLY) {
+        pass_wait();
+        if (lane == 0) epi_load_moving<T, PRIMAL>(in, a.it, r, first, fresh, hw);
+    }
     for (;;) {
         T g[E];
 #pragma unroll
-        for (int q = 0; q < E; ++q) g[q] = __ldg(xg + c[q]);
+        for (int q = 0; q < E; ++q) g[q] = gather_ld<EARLY>(xg + c[q]);
         const int rn = r + groups;
         const bool more = rn < M.rows;  // group-uniform
         EpiIn<T> nin{};
         int nc[E];
         T nv[E];
         if (more) {
-            if (lane == 0) nin = epi_load<T, PRIMAL>(a.it, pv, rn, first, fresh, hw);
+            if (lane == 0) nin = pass_operands<T, PRIMAL, EARLY>(a.it, pv, rn, first, fresh, hw);
             load_idx<E>(M.ci + static_cast<int64_t>(rn) * S + lane * E, nc);
             load_vals<T, E>(vals + static_cast<int64_t>(rn) * S + lane * E, nv);
         }
@@ -307,14 +332,14 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
 // One CTA work item of L (block-uniform): the dot of its entries, then for a
 // whole row its update, for a segment its partial and ticket (and the row's
 // update when this CTA completes the row).
-template <class T, bool PRIMAL>
+template <class T, bool PRIMAL, bool EARLY>
 __device__ __forceinline__ void cta_item(const FastIter<T>& a, const DevCsr& M, const RowItems& L,
                                          int idx, int first, bool fresh, T tau, T sigma, Hw<T> hw) {
     const T* __restrict__ vals = mvals<T>(M);
     const T* __restrict__ xg = PRIMAL ? a.it.y : a.it.xbar;
     const PV<T> pv = pvec<T>(a.P);
     const int4 w = __ldg(L.item + idx);
-    T acc = cta_row_dot<T>(M, vals, xg, w.x, w.y, w.z);
+    T acc = cta_row_dot<T, EARLY>(M, vals, xg, w.x, w.y, w.z);
     if (w.w >= 0) {  // block-uniform
         double tot, unused;
         if (!segment_finish(L, idx, w.w, static_cast<double>(acc), 0.0, &tot, &unused)) return;
@@ -323,7 +348,7 @@ __device__ __forceinline__ void cta_item(const FastIter<T>& a, const DevCsr& M, 
     // the row's operands are loaded after its dot (rows here are long: the
     // load's latency is small beside the dot, and nothing stays live across it)
     if (threadIdx.x == 0) {
-        const EpiIn<T> in = epi_load<T, PRIMAL>(a.it, pv, w.x, first, fresh, hw);
+        const EpiIn<T> in = pass_operands<T, PRIMAL, EARLY>(a.it, pv, w.x, first, fresh, hw);
         epi_store<T, PRIMAL>(a.it, w.x, acc, in, tau, sigma, hw, a.tz);
     }
 }
@@ -333,9 +358,10 @@ __device__ __forceinline__ void cta_item(const FastIter<T>& a, const DevCsr& M, 
 // a persistent grid (the resident CTAs) claims items one by one from L.fetch,
 // so no wave of CTAs ends half empty; the warp path is compiled out, so more
 // CTAs fit per SM.
-template <class T, bool PRIMAL, int MODE, bool WARPS>
+template <class T, bool PRIMAL, int MODE, bool WARPS, bool EARLY>
 __global__ void __launch_bounds__(kBlock, WARPS ? PDHG_WARPROW_MIN_CTAS : PDHG_LONG_MIN_CTAS)
     fast_iter_long(FastIter<T> a, int first, int reset, int warp_blocks) {
+    if (EARLY) pass_begin();
     DevState* st = a.st;
     iter_reset(st, reset);
     if (st->done) return;
@@ -344,11 +370,12 @@ __global__ void __launch_bounds__(kBlock, WARPS ? PDHG_WARPROW_MIN_CTAS : PDHG_L
     const T tau = static_cast<T>(st->tau), sigma = static_cast<T>(st->sigma);
     const Hw<T> hw = halpern_weight_warp<T>(a.it, st, a.hk);
     const RowItems& L = MODE == 0 ? M.items_long : M.items_huge;
+    if (EARLY) pass_wait();
     if (!WARPS) {
         for (;;) {
             const int idx = cta_fetch(L.fetch);
             if (idx >= L.n_item) break;
-            cta_item<T, PRIMAL>(a, M, L, idx, first, fresh, tau, sigma, hw);
+            cta_item<T, PRIMAL, EARLY>(a, M, L, idx, first, fresh, tau, sigma, hw);
         }
         cta_exit(L.fetch);
         return;
@@ -362,21 +389,21 @@ __global__ void __launch_bounds__(kBlock, WARPS ? PDHG_WARPROW_MIN_CTAS : PDHG_L
         const int lane = threadIdx.x & 31;
         const PV<T> pv = pvec<T>(a.P);
         EpiIn<T> in{};
-        if (lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
-        const T acc = warp_dot<T>(M, mvals<T>(M), PRIMAL ? a.it.y : a.it.xbar, r, __ldg(M.rp + r),
+        if (lane == 0) in = pass_operands<T, PRIMAL, EARLY>(a.it, pv, r, first, fresh, hw);
+        const T acc = warp_dot<T, EARLY>(M, mvals<T>(M), PRIMAL ? a.it.y : a.it.xbar, r, __ldg(M.rp + r),
                                   __ldg(M.rp + r + 1));
         if (lane == 0) epi_store<T, PRIMAL>(a.it, r, acc, in, tau, sigma, hw, a.tz);
     } else {
         // CTA work items: rows above kLongRow (mode 0) or kHugeRow (mode 1),
         // those above the segment length in segments
-        cta_item<T, PRIMAL>(a, M, L, static_cast<int>(blockIdx.x) - warp_blocks, first, fresh,
+        cta_item<T, PRIMAL, EARLY>(a, M, L, static_cast<int>(blockIdx.x) - warp_blocks, first, fresh,
                             tau, sigma, hw);
     }
 }
 
 // One warp work item of long_mode 2 (warp-uniform): a whole row, or a segment
 // of a longer one whose last warp adds the segments in order.
-template <class T, bool PRIMAL>
+template <class T, bool PRIMAL, bool EARLY>
 __device__ __forceinline__ void warp_item(const FastIter<T>& a, const DevCsr& M, const RowItems& L,
                                           int idx, int first, bool fresh, T tau, T sigma, Hw<T> hw) {
     const T* __restrict__ vals = mvals<T>(M);
@@ -385,22 +412,23 @@ __device__ __forceinline__ void warp_item(const FastIter<T>& a, const DevCsr& M,
     const int lane = threadIdx.x & 31;
     const int4 w = __ldg(L.item + idx);
     EpiIn<T> in{};
-    if (lane == 0 && w.w < 0) in = epi_load<T, PRIMAL>(a.it, pv, w.x, first, fresh, hw);
-    T acc = warp_dot<T>(M, vals, xg, w.x, w.y, w.z);
+    if (lane == 0 && w.w < 0) in = pass_operands<T, PRIMAL, EARLY>(a.it, pv, w.x, first, fresh, hw);
+    T acc = warp_dot<T, EARLY>(M, vals, xg, w.x, w.y, w.z);
     if (w.w >= 0) {  // warp-uniform
         double tot;
         if (!warp_segment_finish(L, idx, w.w, static_cast<double>(acc), &tot)) return;
         acc = static_cast<T>(tot);
-        if (lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, w.x, first, fresh, hw);
+        if (lane == 0) in = pass_operands<T, PRIMAL, EARLY>(a.it, pv, w.x, first, fresh, hw);
     }
     if (lane == 0) epi_store<T, PRIMAL>(a.it, w.x, acc, in, tau, sigma, hw, a.tz);
 }
 
 // long_mode 2: every row above short_max as warp work items; no block barrier
 // anywhere, each warp finishes on its own.
-template <class T, bool PRIMAL>
+template <class T, bool PRIMAL, bool EARLY>
 __global__ void __launch_bounds__(kBlock, PDHG_WARPITEM_MIN_CTAS)
     fast_iter_witems(FastIter<T> a, int first, int reset) {
+    if (EARLY) pass_begin();
     DevState* st = a.st;
     iter_reset(st, reset);
     if (st->done) return;
@@ -410,7 +438,8 @@ __global__ void __launch_bounds__(kBlock, PDHG_WARPITEM_MIN_CTAS)
     const bool fresh = first && st->fresh;
     const T tau = static_cast<T>(st->tau), sigma = static_cast<T>(st->sigma);
     const Hw<T> hw = halpern_weight_warp<T>(a.it, st, a.hk);
-    warp_item<T, PRIMAL>(a, M, M.items_warp, idx, first, fresh, tau, sigma, hw);
+    if (EARLY) pass_wait();
+    warp_item<T, PRIMAL, EARLY>(a, M, M.items_warp, idx, first, fresh, tau, sigma, hw);
 }
 
 template <class T>
@@ -558,7 +587,7 @@ __global__ void __launch_bounds__(kBlock, (sizeof(T) == 4 && !WITEMS) ? PDHG_SLI
         const int idx = warp_fetch(S.fetch);
         if (idx >= nt) break;
         if (!WITEMS || idx < ns) slice_item<T, PRIMAL>(a, S, idx, first, fresh, tau, sigma, hw);
-        else warp_item<T, PRIMAL>(a, M, M.items_warp, idx - ns, first, fresh, tau, sigma, hw);
+        else warp_item<T, PRIMAL, false>(a, M, M.items_warp, idx - ns, first, fresh, tau, sigma, hw);
     }
     warp_exit(S.fetch);
 }
@@ -638,6 +667,13 @@ inline PassPlan pass_plan(const DevCsr& M, int cap_long, int cap_slice, int cap_
     return p;
 }
 
+// LPs below this many entries launch the next pass early (the EARLY kernels):
+// an iteration of the mixed 500 x 1,200 LP 6.8 -> 4.2 us, FP64 2,000 x 5,000
+// 8.5 -> 5.4, mixed 50,000 x 120,000 13.3 -> 10.3, FP64 transportation 701 x
+// 1,499 (2.1M entries) 24.9 -> 23.3; above, passes run for tens of
+// microseconds and their gathers do better non-coherent.
+constexpr int64_t kEarlyNnz = int64_t{1} << 22;
+
 // Kernels one pass over M launches besides the flag reset.
 inline int pass_launches(const DevCsr& M0) {
     const PassPlan p = pass_plan(pass_matrix(M0), 1, 1, 1);
@@ -656,14 +692,41 @@ int uniform_slot(const DevCsr& M) {
 
 template <class T, int E, int VW, bool PRIMAL>
 void launch_uniform(const FastIter<T>& a, const DevCsr& M, int cap, int first, int reset,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool early) {
     const int64_t need = (static_cast<int64_t>(M.rows) * VW + kBlock - 1) / kBlock;
     const int grid = static_cast<int>(need < cap ? need : cap);
-    fast_iter_uniform<T, E, VW, PRIMAL><<<grid, kBlock, 0, s>>>(a, first, reset);
+    if (a.early) launch_pass(fast_iter_uniform<T, E, VW, PRIMAL, true>, grid, early, s, a, first, reset);
+    else fast_iter_uniform<T, E, VW, PRIMAL, false><<<grid, kBlock, 0, s>>>(a, first, reset);
+}
+
+template <class T, bool PRIMAL, bool EARLY>
+void launch_long(const FastIter<T>& a, const PassPlan& p, int mode, int first, int reset, cudaStream_t s,
+                 bool early) {
+    auto run = [&](auto kernel, auto... warp_blocks) {
+        launch_pass(kernel, p.lng, early, s, a, first, reset, warp_blocks...);
+    };
+    if (mode == 2) run(fast_iter_witems<T, PRIMAL, EARLY>);
+    else if (p.warp == 0 && mode == 1) run(fast_iter_long<T, PRIMAL, 1, false, EARLY>, 0);
+    else if (p.warp == 0) run(fast_iter_long<T, PRIMAL, 0, false, EARLY>, 0);
+    else if (mode == 1) run(fast_iter_long<T, PRIMAL, 1, true, EARLY>, p.warp);
+    else run(fast_iter_long<T, PRIMAL, 0, true, EARLY>, p.warp);
+}
+
+template <class T, bool PRIMAL, bool EARLY>
+void launch_short(const FastIter<T>& a, int lanes, int grid, int first, int reset, cudaStream_t s, bool early) {
+    auto run = [&](auto kernel) { launch_pass(kernel, grid, early, s, a, first, reset); };
+    switch (lanes) {
+        case 1: run(fast_iter<T, 1, PRIMAL, EARLY>); break;
+        case 2: run(fast_iter<T, 2, PRIMAL, EARLY>); break;
+        case 4: run(fast_iter<T, 4, PRIMAL, EARLY>); break;
+        case 8: run(fast_iter<T, 8, PRIMAL, EARLY>); break;
+        case 16: run(fast_iter<T, 16, PRIMAL, EARLY>); break;
+        default: run(fast_iter<T, 32, PRIMAL, EARLY>); break;
+    }
 }
 
 template <class T, bool PRIMAL>
-int launch_iter(const FastIter<T>& a0, int first, cudaStream_t s, const PassFork* f) {
+int launch_iter(const FastIter<T>& a0, int first, cudaStream_t s, const PassFork* f, bool early) {
     const DevCsr& M0 = PRIMAL ? a0.AT : a0.A;
     if (M0.rows == 0) {
         if (PRIMAL && first) {
@@ -685,6 +748,7 @@ int launch_iter(const FastIter<T>& a0, int first, cudaStream_t s, const PassFork
     const int reset_slc = rs && p.shrt == 0 && p.lng == 0 ? 1 : 0;
     const int kernels = (p.shrt > 0) + (p.lng > 0) + (p.slc > 0);
     const bool fork = f != nullptr && f->side[0] != nullptr && kernels > 1;
+    early = early && a.early;  // chosen for both passes (fast_early)
     cudaStream_t ls = s, ss = s;
     if (fork) {
         cudaEventRecord(f->fork, s);
@@ -693,36 +757,21 @@ int launch_iter(const FastIter<T>& a0, int first, cudaStream_t s, const PassFork
         ls = f->side[0];
         ss = f->side[1];
     }
-    if (p.lng > 0 && mode == 2) {
-        fast_iter_witems<T, PRIMAL><<<p.lng, kBlock, 0, ls>>>(a, first, reset_long);
-    } else if (p.lng > 0) {
-        const int mb = p.warp;
-        if (mb == 0) {
-            if (mode == 1) fast_iter_long<T, PRIMAL, 1, false><<<p.lng, kBlock, 0, ls>>>(a, first, reset_long, 0);
-            else fast_iter_long<T, PRIMAL, 0, false><<<p.lng, kBlock, 0, ls>>>(a, first, reset_long, 0);
-        } else {
-            if (mode == 1) fast_iter_long<T, PRIMAL, 1, true><<<p.lng, kBlock, 0, ls>>>(a, first, reset_long, mb);
-            else fast_iter_long<T, PRIMAL, 0, true><<<p.lng, kBlock, 0, ls>>>(a, first, reset_long, mb);
-        }
+    if (p.lng > 0) {
+        if (a.early) launch_long<T, PRIMAL, true>(a, p, mode, first, reset_long, ls, early);
+        else launch_long<T, PRIMAL, false>(a, p, mode, first, reset_long, ls, early);
     }
     if (p.slc > 0 && mode == 2)
         fast_iter_slices<T, PRIMAL, true><<<p.slc, kBlock, 0, ss>>>(a, first, reset_slc);
     else if (p.slc > 0)
         fast_iter_slices<T, PRIMAL, false><<<p.slc, kBlock, 0, ss>>>(a, first, reset_slc);
     const int us = p.shrt > 0 ? uniform_slot<T>(M) : -1;
-    if (us == 0) launch_uniform<T, 2, 1, PRIMAL>(a, M, g_cap_uni[0][pi], first, reset_short, s);
-    else if (us == 1) launch_uniform<T, 4, 1, PRIMAL>(a, M, g_cap_uni[1][pi], first, reset_short, s);
-    else if (us == 2) launch_uniform<T, 4, 2, PRIMAL>(a, M, g_cap_uni[2][pi], first, reset_short, s);
+    if (us == 0) launch_uniform<T, 2, 1, PRIMAL>(a, M, g_cap_uni[0][pi], first, reset_short, s, early);
+    else if (us == 1) launch_uniform<T, 4, 1, PRIMAL>(a, M, g_cap_uni[1][pi], first, reset_short, s, early);
+    else if (us == 2) launch_uniform<T, 4, 2, PRIMAL>(a, M, g_cap_uni[2][pi], first, reset_short, s, early);
     else if (p.shrt > 0) {
-        const int sb = p.shrt;
-        switch (iter_lanes(M)) {
-            case 1: fast_iter<T, 1, PRIMAL><<<sb, kBlock, 0, s>>>(a, first, reset_short); break;
-            case 2: fast_iter<T, 2, PRIMAL><<<sb, kBlock, 0, s>>>(a, first, reset_short); break;
-            case 4: fast_iter<T, 4, PRIMAL><<<sb, kBlock, 0, s>>>(a, first, reset_short); break;
-            case 8: fast_iter<T, 8, PRIMAL><<<sb, kBlock, 0, s>>>(a, first, reset_short); break;
-            case 16: fast_iter<T, 16, PRIMAL><<<sb, kBlock, 0, s>>>(a, first, reset_short); break;
-            default: fast_iter<T, 32, PRIMAL><<<sb, kBlock, 0, s>>>(a, first, reset_short); break;
-        }
+        if (a.early) launch_short<T, PRIMAL, true>(a, iter_lanes(M), p.shrt, first, reset_short, s, early);
+        else launch_short<T, PRIMAL, false>(a, iter_lanes(M), p.shrt, first, reset_short, s, early);
     }
     if (fork) {
         cudaEventRecord(f->join[0], f->side[0]);
@@ -1525,16 +1574,16 @@ int init_fast_kernels(int device) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0)
         return 1;
-    const int l32 = resident_per_sm(fast_iter_long<float, false, 0, false>);
-    const int l64 = resident_per_sm(fast_iter_long<double, false, 0, false>);
+    const int l32 = resident_per_sm(fast_iter_long<float, false, 0, false, false>);
+    const int l64 = resident_per_sm(fast_iter_long<double, false, 0, false, false>);
     const int s32 = resident_per_sm(fast_iter_slices<float, false, false>);
     const int s64 = resident_per_sm(fast_iter_slices<double, false, false>);
-    const int u[3][2] = {{resident_per_sm(fast_iter_uniform<float, 2, 1, true>),
-                          resident_per_sm(fast_iter_uniform<double, 2, 1, true>)},
-                         {resident_per_sm(fast_iter_uniform<float, 4, 1, true>),
-                          resident_per_sm(fast_iter_uniform<double, 4, 1, true>)},
-                         {resident_per_sm(fast_iter_uniform<float, 4, 2, true>),
-                          resident_per_sm(fast_iter_uniform<double, 4, 2, true>)}};
+    const int u[3][2] = {{resident_per_sm(fast_iter_uniform<float, 2, 1, true, false>),
+                          resident_per_sm(fast_iter_uniform<double, 2, 1, true, false>)},
+                         {resident_per_sm(fast_iter_uniform<float, 4, 1, true, false>),
+                          resident_per_sm(fast_iter_uniform<double, 4, 1, true, false>)},
+                         {resident_per_sm(fast_iter_uniform<float, 4, 2, true, false>),
+                          resident_per_sm(fast_iter_uniform<double, 4, 2, true, false>)}};
     for (int q = 0; q < 3; ++q)
         for (int t = 0; t < 2; ++t) {
             if (u[q][t] <= 0) return 1;
@@ -1559,16 +1608,21 @@ int init_fast_kernels(int device) {
 }
 
 template <class T>
-int launch_fast_primal(const FastIter<T>& a, int first, cudaStream_t s, const PassFork* f) {
-    return launch_iter<T, true>(a, first, s, f);
+int launch_fast_primal(const FastIter<T>& a, int first, cudaStream_t s, const PassFork* f, bool early) {
+    return launch_iter<T, true>(a, first, s, f, early);
 }
 template <class T>
-int launch_fast_dual(const FastIter<T>& a, int first, cudaStream_t s, const PassFork* f) {
-    return launch_iter<T, false>(a, first, s, f);
+int launch_fast_dual(const FastIter<T>& a, int first, cudaStream_t s, const PassFork* f, bool early) {
+    return launch_iter<T, false>(a, first, s, f, early);
 }
 template <class T>
 int fast_launches_per_iteration(const FastIter<T>& a) {
     return pass_launches(a.AT) + pass_launches(a.A);
+}
+template <class T>
+bool fast_early(const FastIter<T>& a) {
+    return a.A.nnz < kEarlyNnz && pass_launches(a.AT) == 1 && pass_launches(a.A) == 1 &&
+           !(a.A.use_slices && a.A.slices.n_item > 0) && !(a.AT.use_slices && a.AT.slices.n_item > 0);
 }
 
 // Ray test, rows' half: after a check that left a pending ray d (projected
@@ -1641,10 +1695,12 @@ int fast_check_grid(const DevCsr& A, const DevCsr& AT) {
     return check_blocks(check_view(A)) + check_blocks(check_view(AT)) + 1;
 }
 
-template int launch_fast_primal<float>(const FastIter<float>&, int, cudaStream_t, const PassFork*);
-template int launch_fast_primal<double>(const FastIter<double>&, int, cudaStream_t, const PassFork*);
-template int launch_fast_dual<float>(const FastIter<float>&, int, cudaStream_t, const PassFork*);
-template int launch_fast_dual<double>(const FastIter<double>&, int, cudaStream_t, const PassFork*);
+template int launch_fast_primal<float>(const FastIter<float>&, int, cudaStream_t, const PassFork*, bool);
+template int launch_fast_primal<double>(const FastIter<double>&, int, cudaStream_t, const PassFork*, bool);
+template int launch_fast_dual<float>(const FastIter<float>&, int, cudaStream_t, const PassFork*, bool);
+template int launch_fast_dual<double>(const FastIter<double>&, int, cudaStream_t, const PassFork*, bool);
+template bool fast_early<float>(const FastIter<float>&);
+template bool fast_early<double>(const FastIter<double>&);
 template int fast_launches_per_iteration<float>(const FastIter<float>&);
 template int fast_launches_per_iteration<double>(const FastIter<double>&);
 template void launch_fast_check<float>(const FastCheck<float>&, cudaStream_t);

@@ -97,15 +97,23 @@ __device__ __forceinline__ double ordered_sum_warp(int b, int e, Term term, doub
 // kStage doubles per warp), so only the chain of additions is exposed.
 // ordered_sum_warp evaluates a round's terms (index load, then gather) and
 // only then adds it.
-template <class G>
+// wait() runs once, before the first gather and after the first two rounds'
+// index and value loads (the passes' wait for the pass before).
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
+template <class G, class W = NoWait>
 __device__ __forceinline__ double ordered_dot_warp_pipelined(int b, int e,
                                                              const int32_t* __restrict__ ci,
                                                              const double* __restrict__ v, G g,
-                                                             double init, double* stage2) {
+                                                             double init, double* stage2, W wait = W{}) {
     constexpr int Q = kStage / 32;
     const int lane = threadIdx.x & 31;
     double acc = init;
-    if (b >= e) return acc;
+    if (b >= e) {
+        wait();
+        return acc;
+    }
     auto load_cv = [&](int k0, int (&c)[Q], double (&w)[Q]) {
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -122,6 +130,7 @@ __device__ __forceinline__ double ordered_dot_warp_pipelined(int b, int e,
         double w0[Q], t0[Q];
         load_cv(b, c0, w0);
         load_cv(b + kStage, c1, w1);
+        wait();
 #pragma unroll
         for (int q = 0; q < Q; ++q) t0[q] = b + 32 * q + lane < e ? __dmul_rn(w0[q], g(c0[q])) : 0.0;
 #pragma unroll
