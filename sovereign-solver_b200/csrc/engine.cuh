@@ -415,6 +415,8 @@ struct FinalArgs {
     int part_blocks = 0;      // CTAs that fit in part (and at most a few per SM)
 };
 void launch_final(const FinalArgs& a, cudaStream_t s);
+// launch_final's products in the throughput modes (kernels_fast.cu)
+void launch_fast_final_rows(const FinalArgs& a, cudaStream_t s);
 
 // Best point selection for the final result: the check's candidate when
 // converged, else the current iterate (pdhg.cpp:420-423). Materialises the

@@ -697,25 +697,69 @@ __global__ void __launch_bounds__(kBlock) k_fin_rowscols(FinalArgs a) {
     block_acc_max(&st->acc[ACC_FIN_DINF], dinf);
 }
 
+// acc = init; acc = acc + term(k) for k in [0, n) in this order, each sum
+// rounded, by one CTA: the threads evaluate kFinStage terms at a time into
+// shared memory, one round ahead, and thread 0 adds them. It stops at the
+// first term that is not finite and clears *finite (with stop_at_inf). What is
+// left is the chain of dependent additions: the 100,200 columns of a
+// transportation LP took one thread alone 4.4 ms, a load's latency an entry.
+constexpr int kFinStage = 4 * kBlock;
+template <class Term>
+__device__ double cta_ordered_sum(int32_t n, Term term, double init, bool stop_at_inf, bool* finite,
+                                  double (*stage)[kFinStage]) {
+    double acc = init;
+    for (int32_t o = threadIdx.x; o < kFinStage && o < n; o += kBlock) stage[0][o] = term(o);
+    __syncthreads();
+    int buf = 0, stop = 0;
+    for (int32_t k0 = 0; k0 < n && !stop; k0 += kFinStage, buf ^= 1) {
+        const int32_t k1 = k0 + kFinStage;
+        int mine = 0;
+        if (threadIdx.x >= 32) {  // the next round, while thread 0 adds this one
+            for (int32_t o = static_cast<int32_t>(threadIdx.x) - 32; o < kFinStage && k1 + o < n; o += kBlock - 32)
+                stage[buf ^ 1][o] = term(k1 + o);
+        } else if (threadIdx.x == 0) {
+            const double* st = stage[buf];
+            const int32_t cnt = n - k0 < kFinStage ? n - k0 : kFinStage;
+            int32_t o = 0;
+            for (; o + 8 <= cnt; o += 8) {
+                double t[8];
+                bool all = true;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    t[u] = st[o + u];
+                    all = all && isfinite(t[u]);
+                }
+                if (stop_at_inf && !all) break;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc = __dadd_rn(acc, t[u]);
+            }
+            for (; o < cnt; ++o) {
+                if (stop_at_inf && !isfinite(st[o])) {
+                    mine = 1;
+                    break;
+                }
+                acc = __dadd_rn(acc, st[o]);
+            }
+        }
+        stop = __syncthreads_or(mine);  // the same for every thread
+    }
+    *finite = stop == 0;
+    __syncthreads();  // the stage is free for the next sum
+    return acc;
+}
+
 // Sequential sums in the reference's order (objective: problem.cpp:13-19;
 // dual objective: columns then rows, stopping at the first infinite term).
-__global__ void k_fin_sums_exact(FinalArgs a) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(kBlock) k_fin_sums_exact(FinalArgs a) {
+    __shared__ double stage[2][kFinStage];
     DevState* st = a.st;
-    double acc = a.P.obj_const;
-    for (int j = 0; j < a.P.n; ++j) acc = __dadd_rn(acc, __dmul_rn(a.P.c_o[j], a.f.xo[j]));
-    double dual = 0.0;
-    bool fin = true;
-    for (int j = 0; j < a.P.n && fin; ++j) {
-        const double t = a.f.tcol[j];
-        if (!isfinite(t)) { fin = false; break; }
-        dual = __dadd_rn(dual, t);
-    }
-    for (int i = 0; i < a.P.m && fin; ++i) {
-        const double t = a.f.trow[i];
-        if (!isfinite(t)) { fin = false; break; }
-        dual = __dadd_rn(dual, t);
-    }
+    bool fin = true, rows_fin = true;
+    const double acc = cta_ordered_sum(
+        a.P.n, [&](int32_t j) { return __dmul_rn(a.P.c_o[j], a.f.xo[j]); }, a.P.obj_const, false, &fin, stage);
+    double dual = cta_ordered_sum(a.P.n, [&](int32_t j) { return a.f.tcol[j]; }, 0.0, true, &fin, stage);
+    if (fin) dual = cta_ordered_sum(a.P.m, [&](int32_t i) { return a.f.trow[i]; }, dual, true, &rows_fin, stage);
+    fin = fin && rows_fin;
+    if (threadIdx.x != 0) return;
     st->objective = acc;
     st->dual_objective = dual;
     st->gap_finite = fin ? 1 : 0;
@@ -994,11 +1038,12 @@ void launch_fill(double* x, int64_t n, double v, cudaStream_t s) {
 void launch_final(const FinalArgs& a, cudaStream_t s) {
     const int32_t nmax = a.P.n > a.P.m ? a.P.n : a.P.m;
     if (nmax > 0) k_fin_unscale<<<blocks_for(nmax), kBlock, 0, s>>>(a);
-    const int g = mat_blocks(a.Ao) + mat_blocks(a.ATo);
-    if (g > 0) k_fin_rowscols<<<g, kBlock, 0, s>>>(a);
     if (a.exact) {
-        k_fin_sums_exact<<<1, 32, 0, s>>>(a);
+        const int g = mat_blocks(a.Ao) + mat_blocks(a.ATo);
+        if (g > 0) k_fin_rowscols<<<g, kBlock, 0, s>>>(a);
+        k_fin_sums_exact<<<1, kBlock, 0, s>>>(a);
     } else {
+        launch_fast_final_rows(a, s);
         int gs = blocks_for(nmax > 0 ? nmax : 1);
         if (gs > a.part_blocks) gs = a.part_blocks;
         k_fin_sums_tree<<<gs > 0 ? gs : 1, kBlock, 0, s>>>(a, a.part);

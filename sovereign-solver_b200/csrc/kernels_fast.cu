@@ -1561,7 +1561,112 @@ __global__ void __launch_bounds__(kBlock) fast_restart(FastCheck<T> a) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// Final result (pdhg.cpp:428-498) in the throughput modes
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ double fin_inf_over_box(double coeff, double lo, double hi) {  // pdhg.cpp:36-40
+    if (coeff == 0.0) return 0.0;
+    if (coeff > 0.0) return fb(lo) ? coeff * lo : -INFINITY;
+    return fb(hi) ? coeff * hi : -INFINITY;
+}
+
+// The terms of one row (its activity) or column (A^T y): primal infeasibility,
+// complementary slackness, reduced cost, dual objective.
+template <bool ROWS>
+__device__ __forceinline__ void fin_terms(const FinalArgs& a, int r, double dot, double& pinf, double& dinf) {
+    const double bt = a.bound_tol;
+    const double v = ROWS ? a.f.yo[r] : a.P.c_o[r] - dot;  // multiplier or reduced cost
+    const double act = ROWS ? dot : a.f.xo[r];
+    const double lo = ROWS ? a.P.rlo_o[r] : a.P.lo_o[r], hi = ROWS ? a.P.rhi_o[r] : a.P.hi_o[r];
+    if (ROWS) pinf = smax(pinf, primal_term(act, lo, hi));
+    else a.f.rc[r] = v;
+    const bool at_lo = fb(lo) && fabs(act - lo) <= bt;
+    const bool at_hi = fb(hi) && fabs(act - hi) <= bt;
+    if (!at_lo && !at_hi) dinf = smax(dinf, fabs(v));
+    (ROWS ? a.f.trow : a.f.tcol)[r] = fin_inf_over_box(v, lo, hi);
+}
+
+// Entries k, k + step, ... below e of M times x, four of each stream in flight.
+__device__ __forceinline__ double fin_products(const DevCsr& M, const double* x, int k, int e, int step) {
+    double s0 = 0.0, s1 = 0.0;
+    for (; k < e; k += 4 * step) {
+        int c[4];
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            c[u] = k + u * step < e ? M.ci[k + u * step] : 0;
+            v[u] = k + u * step < e ? M.v64[k + u * step] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k + u * step < e) (u & 1 ? s1 : s0) += v[u] * x[c[u]];
+    }
+    return s0 + s1;
+}
+
+// Virtual block vb of one matrix, split like the check's (check_part): lane
+// groups, warp rows, CTA items with split rows. One warp per row, in row
+// order, took the badly scaled LP's longest row (344,267 entries) 7.0 ms.
+template <bool ROWS>
+__device__ void fin_part(const FinalArgs& a, const DevCsr& M, int vb, int sb, int wb, double& pinf, double& dinf) {
+    const double* x = ROWS ? a.f.xo : a.f.yo;
+    if (vb < sb) {
+        const int vw = M.vw;
+        const int lane = threadIdx.x & (vw - 1);
+        const int r = (vb * kBlock + threadIdx.x) / vw;
+        if (r >= M.rows) return;
+        const int b = M.rp[r], e = M.rp[r + 1];
+        if (e - b > M.short_max) return;
+        const double dot = group_sum(fin_products(M, x, b + lane, e, vw), vw);
+        if (lane == 0) fin_terms<ROWS>(a, r, dot, pinf, dinf);
+    } else if (vb < sb + wb) {
+        const int w = (vb - sb) * (kBlock / 32) + (threadIdx.x >> 5);
+        if (w >= M.n_warp0) return;
+        const int r = M.warp_rows0[w];
+        const int lane = threadIdx.x & 31;
+        double dot = fin_products(M, x, M.rp[r] + lane, M.rp[r + 1], 32);
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane == 0) fin_terms<ROWS>(a, r, dot, pinf, dinf);
+    } else {
+        const int idx = vb - sb - wb;
+        const int4 w = M.items_long.item[idx];
+        double dot = block_total(fin_products(M, x, w.y + threadIdx.x, w.z, kBlock)), unused;
+        if (w.w >= 0 && !segment_finish(M.items_long, idx, w.w, dot, 0.0, &dot, &unused)) return;
+        if (threadIdx.x == 0) fin_terms<ROWS>(a, w.x, dot, pinf, dinf);
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) fast_final(FinalArgs a) {
+    double pinf = 0.0, dinf = 0.0;
+    const int sbA = check_short_blocks(a.Ao), wbA = check_warp_blocks(a.Ao);
+    const int sbT = check_short_blocks(a.ATo), wbT = check_warp_blocks(a.ATo);
+    const int nA = sbA + wbA + a.Ao.items_long.n_item, nT = sbT + wbT + a.ATo.items_long.n_item;
+    for (int bid = blockIdx.x; bid < nA + nT; bid += gridDim.x) {  // the longest items first
+        const int vb = bid < nA ? nA - 1 - bid : nA + nT - 1 - bid;
+        if (bid < nA) fin_part<true>(a, a.Ao, vb, sbA, wbA, pinf, dinf);
+        else fin_part<false>(a, a.ATo, vb, sbT, wbT, pinf, dinf);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        pinf = fmax(pinf, __shfl_xor_sync(0xffffffffu, pinf, o));
+        dinf = fmax(dinf, __shfl_xor_sync(0xffffffffu, dinf, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (pinf > 0.0)
+            atomicMax(&a.st->acc[ACC_FIN_PINF], static_cast<unsigned long long>(__double_as_longlong(pinf)));
+        if (dinf > 0.0)
+            atomicMax(&a.st->acc[ACC_FIN_DINF], static_cast<unsigned long long>(__double_as_longlong(dinf)));
+    }
+}
+
 }  // namespace
+
+void launch_fast_final_rows(const FinalArgs& a, cudaStream_t s) {
+    int64_t g = 0;
+    for (const DevCsr* M : {&a.Ao, &a.ATo}) g += check_short_blocks(*M) + check_warp_blocks(*M) + M->items_long.n_item;
+    if (g > 148 * 16) g = 148 * 16;
+    if (g > 0) fast_final<<<static_cast<int>(g), kBlock, 0, s>>>(a);
+}
 
 template <class K>
 int resident_per_sm(K kernel) {
