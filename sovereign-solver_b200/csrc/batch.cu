@@ -813,18 +813,8 @@ int batch_solve(BatchCtx& c, const pdhg_options& o, pdhg_info* infos, double* x,
     }
     if (o.primal_weight_update) {
         // restart points start at the initial point
-        BCK(cudaStreamSynchronize(s));
-        if (f32) {
-            std::vector<float> hx(static_cast<size_t>(c.n)), hy(static_cast<size_t>(c.m));
-            if (c.n) BCK(cudaMemcpy(hx.data(), c.x32.p, sizeof(float) * c.n, cudaMemcpyDeviceToHost));
-            if (c.m) BCK(cudaMemcpy(hy.data(), c.y32.p, sizeof(float) * c.m, cudaMemcpyDeviceToHost));
-            std::vector<double> dx(hx.begin(), hx.end()), dy(hy.begin(), hy.end());
-            if (c.n) BCK(cudaMemcpy(c.x_last.p, dx.data(), sizeof(double) * c.n, cudaMemcpyHostToDevice));
-            if (c.m) BCK(cudaMemcpy(c.y_last.p, dy.data(), sizeof(double) * c.m, cudaMemcpyHostToDevice));
-        } else {
-            if (c.n) BCK(cudaMemcpyAsync(c.x_last.p, c.x64.p, sizeof(double) * c.n, cudaMemcpyDeviceToDevice, s));
-            if (c.m) BCK(cudaMemcpyAsync(c.y_last.p, c.y64.p, sizeof(double) * c.m, cudaMemcpyDeviceToDevice, s));
-        }
+        if (f32) launch_batch_snapshot<float>(b, batch_iterates<float>(c), c.x_last.p, c.y_last.p, s);
+        else launch_batch_snapshot<double>(b, batch_iterates<double>(c), c.x_last.p, c.y_last.p, s);
     }
     BCK(cudaStreamSynchronize(s));
     // cancellation / time limit before the first iteration (pdhg.cpp:288-293)
@@ -897,14 +887,14 @@ int batch_solve(BatchCtx& c, const pdhg_options& o, pdhg_info* infos, double* x,
     const double bt = o.tolerance > 1e-6 ? o.tolerance : 1e-6;
     if (f32) {
         launch_batch_final<float>(b, batch_iterates<float>(c), bt, c.xo.p, c.yo.p, c.rc.p, 0, s);
-        launches += 1;
+        launches += 2;
         if (any_polished) {
             launch_batch_final<double>(b, batch_iterates<double>(c), bt, c.xo.p, c.yo.p, c.rc.p, 1, s);
-            launches += 1;
+            launches += 2;
         }
     } else {
         launch_batch_final<double>(b, batch_iterates<double>(c), bt, c.xo.p, c.yo.p, c.rc.p, -1, s);
-        launches += 1;
+        launches += 2;
     }
     BCK(cudaMemcpyAsync(h.data(), c.is.p, sizeof(InstState) * c.count, cudaMemcpyDeviceToHost, s));
     BatchGlobal g2;

@@ -788,66 +788,113 @@ __global__ void batch_widen(BatchView b, Iterates<float> f, Iterates<double> d) 
     }
 }
 
+// The best point in original units (unscale_to_original, pdhg.cpp:205-214) of
+// the instances `which` names.
 template <class T>
-__global__ void __launch_bounds__(kBlock) batch_final(BatchView b, Iterates<T> it, double bt,
-                                                      double* xo, double* yo, double* rc,
-                                                      int which) {
-    const int k = blockIdx.x;
-    InstState& s = b.is[k];
-    if (which >= 0 && s.polished != which) return;  // uniform per CTA
-    const DevProblem& P = b.P;
+__global__ void __launch_bounds__(kBlock) batch_best_point(BatchView b, Iterates<T> it, double* xo, double* yo,
+                                                           int which) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
     // Halpern: after a check the sums' slots hold T(z), the reported point
-    const bool cand_avg = it.halpern ? b.g->checks > 0 : (s.converged && s.avg_better);
-    const double inv = it.halpern ? 1.0 : s.inv, sign = s.obj_sign;
-    // best point in original units (unscale_to_original, pdhg.cpp:205-214)
-    for (int j = b.col_off[k] + threadIdx.x; j < b.col_off[k + 1]; j += kBlock) {
-        const double xs = cand_avg ? avg_x(it, j, inv) : static_cast<double>(it.x[j]);
-        xo[j] = xs * P.cs[j];
-    }
-    for (int i = b.row_off[k] + threadIdx.x; i < b.row_off[k + 1]; i += kBlock) {
-        const double ys = cand_avg ? avg_y(it, i, inv) : static_cast<double>(it.y[i]);
-        yo[i] = (ys * sign) * P.rs[i];
-    }
-    __syncthreads();  // xo / yo of this instance are read below by other threads of this CTA
-    double pinf = 0.0, dinf = 0.0, obj = 0.0, dual = 0.0, inf = 0.0;
-    const int lane = threadIdx.x & 31;
-    const int groups = kBlock / 32;
-    for (int i = b.row_off[k] + static_cast<int>(threadIdx.x) / 32; i < b.row_off[k + 1]; i += groups) {
-        const double act = row_dot64(b.Ao, i, lane, 32, [xo](int j) { return xo[j]; });
-        if (lane == 0) {
-            const double lo = P.rlo_o[i], hi = P.rhi_o[i];
-            pinf = smax(pinf, primal_term(act, lo, hi));
-            const bool at_lo = fb(lo) && fabs(act - lo) <= bt;
-            const bool at_hi = fb(hi) && fabs(act - hi) <= bt;
-            if (!at_lo && !at_hi) dinf = smax(dinf, fabs(yo[i]));
-            const double tr = inf_box(yo[i], lo, hi);
-            if (isfinite(tr)) dual += tr; else inf = 1.0;
+    const bool tz = it.halpern && b.g->checks > 0;
+    if (t < b.n) {
+        const InstState& s = b.is[b.col_inst[t]];
+        if (which < 0 || s.polished == which) {
+            const bool avg = it.halpern ? tz : (s.converged && s.avg_better);
+            const double xs = avg ? avg_x(it, static_cast<int>(t), it.halpern ? 1.0 : s.inv) : static_cast<double>(it.x[t]);
+            xo[t] = xs * b.P.cs[t];
         }
     }
-    for (int j = b.col_off[k] + static_cast<int>(threadIdx.x) / 32; j < b.col_off[k + 1]; j += groups) {
-        const double aty = row_dot64(b.ATo, j, lane, 32, [yo](int i) { return yo[i]; });
-        if (lane == 0) {
-            const double r = P.c_o[j] - aty;
-            rc[j] = r;
-            const double lo = P.lo_o[j], hi = P.hi_o[j];
-            const bool at_lo = fb(lo) && fabs(xo[j] - lo) <= bt;
-            const bool at_hi = fb(hi) && fabs(xo[j] - hi) <= bt;
-            if (!at_lo && !at_hi) dinf = smax(dinf, fabs(r));
-            obj += P.c_o[j] * xo[j];
-            const double tc = inf_box(r, lo, hi);
-            if (isfinite(tc)) dual += tc; else inf = 1.0;
+    if (t < b.m) {
+        const InstState& s = b.is[b.row_inst[t]];
+        if (which < 0 || s.polished == which) {
+            const bool avg = it.halpern ? tz : (s.converged && s.avg_better);
+            const double ys = avg ? avg_y(it, static_cast<int>(t), it.halpern ? 1.0 : s.inv) : static_cast<double>(it.y[t]);
+            yo[t] = (ys * s.obj_sign) * b.P.rs[t];
         }
     }
-    const double pi = bmax(pinf), di = bmax(dinf);
-    const double ob = block_sum_det(obj), du = block_sum_det(dual), nf = block_sum_det(inf);
-    if (threadIdx.x == 0) {
-        const double acc = s.obj_const + ob;
-        s.objective = acc;
-        s.dual_objective = du;
-        s.gap = nf == 0.0 ? fabs(acc - du) / (1.0 + fabs(acc) + fabs(du)) : INFINITY;
-        s.pinf = pi;
-        s.dinf = di;
+}
+
+// The point's objective, infeasibilities and gap, an instance in the check's
+// CTA parts (rows and columns on lane groups), merged by its last part in part
+// order. One CTA per instance with a warp per row took the 256-instance batch
+// of the tests' sizes 9.9 ms, the largest instance's CTA alone.
+template <bool COLS>
+__device__ __forceinline__ void final_pass(const BatchView& b, int k, int part, int parts, double bt,
+                                           const double* xo, const double* yo, double* rc, double (&v)[5]) {
+    const DevProblem& P = b.P;
+    const DevCsr& M = COLS ? b.ATo : b.Ao;
+    const double* x = COLS ? yo : xo;
+    const int vw = M.vw;
+    const int lane = threadIdx.x & (vw - 1);
+    const int q0 = COLS ? b.col_off[k] : b.row_off[k];
+    const int q1 = COLS ? b.col_off[k + 1] : b.row_off[k + 1];
+    const int r0 = q0 + static_cast<int>(static_cast<int64_t>(q1 - q0) * part / parts);
+    const int r1 = q0 + static_cast<int>(static_cast<int64_t>(q1 - q0) * (part + 1) / parts);
+    for (int r = r0 + static_cast<int>(threadIdx.x) / vw; r < r1; r += kBlock / vw) {
+        double dot = 0.0;
+        for (int q = M.rp[r] + lane; q < M.rp[r + 1]; q += vw) dot += M.v64[q] * x[M.ci[q]];
+        dot = group_sum(dot, vw);
+        if (lane != 0) continue;
+        const double mult = COLS ? P.c_o[r] - dot : yo[r];  // reduced cost or multiplier
+        const double act = COLS ? xo[r] : dot;
+        const double lo = COLS ? P.lo_o[r] : P.rlo_o[r], hi = COLS ? P.hi_o[r] : P.rhi_o[r];
+        if (COLS) {
+            rc[r] = mult;
+            v[2] += P.c_o[r] * act;
+        } else {
+            v[0] = smax(v[0], primal_term(act, lo, hi));
+        }
+        const bool at_lo = fb(lo) && fabs(act - lo) <= bt;
+        const bool at_hi = fb(hi) && fabs(act - hi) <= bt;
+        if (!at_lo && !at_hi) v[1] = smax(v[1], fabs(mult));
+        const double t = inf_box(mult, lo, hi);
+        if (isfinite(t)) v[3] += t;
+        else v[4] = 1.0;
     }
+}
+
+__global__ void __launch_bounds__(kBlock) batch_final(BatchView b, double bt, const double* xo, const double* yo,
+                                                      double* rc, int which) {
+    const int4 item = b.chk_item[blockIdx.x];
+    const int k = item.x, part = item.y, parts = item.z;
+    InstState& s = b.is[k];
+    if (which >= 0 && s.polished != which) return;  // uniform per instance
+    double v[5] = {};  // primal and dual infeasibility, objective, dual objective, an infinite term
+    final_pass<false>(b, k, part, parts, bt, xo, yo, rc, v);
+    final_pass<true>(b, k, part, parts, bt, xo, yo, rc, v);
+    v[0] = bmax(v[0]);
+    v[1] = bmax(v[1]);
+    for (int q = 2; q < 5; ++q) v[q] = block_sum_det(v[q]);
+    if (threadIdx.x != 0) return;
+    if (parts > 1) {
+        double* mine = b.chk_part + kBatchCheckVals * static_cast<int64_t>(blockIdx.x);
+        for (int q = 0; q < 5; ++q) mine[q] = v[q];
+        __threadfence();
+        if (atomicAdd(b.chk_ticket + k, 1u) != static_cast<unsigned>(parts - 1)) return;
+        __threadfence();
+        const double* first = b.chk_part + kBatchCheckVals * (static_cast<int64_t>(blockIdx.x) - part);
+        for (int q = 0; q < 5; ++q) v[q] = 0.0;
+        for (int j = 0; j < parts; ++j)
+            for (int q = 0; q < 5; ++q) {
+                const double t = __ldcg(first + kBatchCheckVals * j + q);
+                v[q] = q < 2 ? smax(v[q], t) : v[q] + t;
+            }
+        b.chk_ticket[k] = 0u;
+    }
+    const double acc = s.obj_const + v[2];
+    s.objective = acc;
+    s.dual_objective = v[3];
+    s.gap = v[4] == 0.0 ? fabs(acc - v[3]) / (1.0 + fabs(acc) + fabs(v[3])) : INFINITY;
+    s.pinf = v[0];
+    s.dinf = v[1];
+}
+
+// The restart points of the primal weight: the current x and y.
+template <class T>
+__global__ void batch_snapshot(Iterates<T> it, double* xl, double* yl, int32_t n, int32_t m) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
+    if (t < n) xl[t] = static_cast<double>(it.x[t]);
+    if (t < m) yl[t] = static_cast<double>(it.y[t]);
 }
 
 // Relative KKT residual of a given point (x, y in original units and sense; a
@@ -1031,8 +1078,18 @@ void launch_batch_widen(const BatchView& b, const Iterates<float>& f, const Iter
 template <class T>
 void launch_batch_final(const BatchView& b, const Iterates<T>& it, double bound_tol, double* xo,
                         double* yo, double* rc, int which, cudaStream_t s) {
-    if (b.count > 0) batch_final<T><<<b.count, kBlock, 0, s>>>(b, it, bound_tol, xo, yo, rc, which);
+    const int32_t nmax = b.m > b.n ? b.m : b.n;
+    if (nmax > 0) batch_best_point<T><<<nblk(nmax), kBlock, 0, s>>>(b, it, xo, yo, which);
+    if (b.n_chk > 0) batch_final<<<b.n_chk, kBlock, 0, s>>>(b, bound_tol, xo, yo, rc, which);
 }
+
+template <class T>
+void launch_batch_snapshot(const BatchView& b, const Iterates<T>& it, double* xl, double* yl, cudaStream_t s) {
+    const int32_t nmax = b.m > b.n ? b.m : b.n;
+    if (nmax > 0) batch_snapshot<T><<<nblk(nmax), kBlock, 0, s>>>(it, xl, yl, b.n, b.m);
+}
+template void launch_batch_snapshot<float>(const BatchView&, const Iterates<float>&, double*, double*, cudaStream_t);
+template void launch_batch_snapshot<double>(const BatchView&, const Iterates<double>&, double*, double*, cudaStream_t);
 
 template void launch_batch_iter<float>(const BatchView&, const Iterates<float>&, bool, int, int, cudaStream_t);
 template void launch_batch_iter<double>(const BatchView&, const Iterates<double>&, bool, int, int, cudaStream_t);

@@ -106,6 +106,9 @@ void launch_batch_tick(const BatchView& b, long long period, long long budget_it
 // Rebuilds the active block lists when g->dirty is set (one CTA; a no-op otherwise).
 void launch_batch_compact(const BatchView& b, cudaStream_t s);
 void launch_batch_fill_inst(const int32_t* off, int32_t count, int32_t* out, cudaStream_t s);
+// xl, yl <- the iterates' x and y
+template <class T>
+void launch_batch_snapshot(const BatchView& b, const Iterates<T>& it, double* xl, double* yl, cudaStream_t s);
 void launch_batch_warm(const BatchView& b, double* x0, double* y0, cudaStream_t s);
 
 // power iteration per instance (estimate_operator_norm, pdhg.cpp:48-79)
