@@ -94,7 +94,7 @@ struct Ctx {
     DBuf<double> xa64, sa64, ya64;
     DBuf<float> xa32, sa32, ya32;
     DBuf<double> act_avg, cand_xo, cand_yo, part, bx, by, xo, yo, rc, trow, tcol;
-    DBuf<double> pw_u, pw_v, pw_w, pw_part, pw_out, x0s, y0s;
+    DBuf<double> pw_u, pw_w, pw_part, pw_st, x0s, y0s;
     DBuf<int> pw_stop;
     DBuf<double> x_last, y_last;  // restart points (primal-weight update)
     DBuf<double> ray_yp, ray_atyp, ray_y;  // infeasibility test: previous y, A^T y; dy (original)
@@ -346,48 +346,43 @@ int ensure_scaled(Ctx& c, const ScalingParams& sp) {
     return PDHG_OK;
 }
 
-// estimate_operator_norm (pdhg.cpp:48-79) with the exact kernels; the scalar
-// tail (sqrt, 1/x) runs on the host exactly as in the reference.
-// The power iteration of pdhg.cpp:50-78 with the reference's arithmetic
-// (ordered sums, pairwise norms, IEEE square roots and divisions). Its scalar
-// steps run on the device (k_pw_norm_w / _e), so the loop issues every
-// iteration without waiting on the host; a device flag stands in for the
-// loop's two early exits and turns the remaining launches into no-ops.
+// estimate_operator_norm (pdhg.cpp:48-79). FP64-exact: the reference's
+// arithmetic (ordered sums, pairwise norms, IEEE square roots and divisions);
+// `fast` sums the rows in parallel. The scalar steps run on the device, so the
+// loop issues every iteration without waiting on the host; a device flag
+// stands in for the loop's two early exits and turns the remaining launches
+// into no-ops. Four launches an iteration: with the norms' levels, the scalar
+// steps and the scalings apart it was twelve, and a small LP's estimate took
+// 1.8 ms of launches.
 int operator_norm(Ctx& c, int iterations, bool fast, double* out) {
     cudaStream_t s = c.stream;
     const int32_t n = c.lp.n, m = c.lp.m;
     CK(c.pw_u.alloc(static_cast<size_t>(n) + 1));
-    CK(c.pw_v.alloc(static_cast<size_t>(m) + 1));
     CK(c.pw_w.alloc(static_cast<size_t>(m) + 1));
-    const int64_t ps = std::max(pairwise_partial_size(n), pairwise_partial_size(m));
-    CK(c.pw_part.alloc(static_cast<size_t>(ps)));
-    CK(c.pw_out.alloc(8));  // [0..1] norms' squares, [4..6] the scalar state
-    CK(c.pw_stop.alloc(1));
+    CK(c.pw_part.alloc(static_cast<size_t>(pw_partial_size(n, m))));
+    CK(c.pw_st.alloc(PW_COUNT));
+    CK(c.pw_stop.alloc(2));  // the flag; the norm kernels' ticket
     launch_fill(c.pw_u.p, n, 1.0, s);
-    launch_fill(c.pw_v.p, m, 1.0, s);
-    launch_fill(c.pw_w.p, m, 0.0, s);
-    launch_fill(c.pw_out.p, 8, 0.0, s);
-    launch_fill(c.pw_out.p + 6, 1, 1.0, s);  // u's scale before the first iteration
-    CK(cudaMemsetAsync(c.pw_stop.p, 0, sizeof(int), s));
+    launch_fill(c.pw_w.p, m, 1.0, s);  // v before the first iteration, its scales 1
+    const double st0[PW_COUNT] = {1.0, 0.0, 1.0};
+    CK(cudaMemcpyAsync(c.pw_st.p, st0, sizeof st0, cudaMemcpyHostToDevice, s));
+    CK(cudaMemsetAsync(c.pw_stop.p, 0, 2 * sizeof(int), s));
     const DevCsr A = c.As.view(), AT = c.ATs.view();
-    double* dots = c.pw_out.p;
-    double* st = c.pw_out.p + 4;
+    double *st = c.pw_st.p, *u = c.pw_u.p, *w = c.pw_w.p;
     int* stop = c.pw_stop.p;
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(stop + 1);
     for (int it = 0; it < iterations; ++it) {
-        launch_pw_w(A, c.pw_u.p, c.pw_v.p, c.pw_w.p, s, stop, st + 2, fast);  // u scaled where gathered
-        launch_pairwise_dot(c.pw_w.p, c.pw_w.p, m, c.pw_part.p, dots, s);
-        launch_pw_norm_w(dots, st, stop, s);
-        launch_scale_by(c.pw_w.p, m, st, stop, s);
-        launch_pw_u(AT, c.pw_w.p, c.pw_u.p, s, stop);
-        launch_copy_unless(c.pw_v.p, c.pw_w.p, m, stop, s);
-        launch_pairwise_dot(c.pw_u.p, c.pw_u.p, n, c.pw_part.p, dots, s);
-        launch_pairwise_dot(c.pw_v.p, c.pw_v.p, m, c.pw_part.p, dots + 1, s);
-        launch_pw_norm_e(dots, st, stop, s);
-        launch_scale_by(c.pw_v.p, m, st + 2, stop, s);
+        const bool e = it > 0;  // the first launch follows fills and copies
+        if (fast) launch_fast_pw_w(A, u, w, st, stop, e, s);
+        else launch_pw_w(A, u, w, st, stop, e, s);
+        launch_pw_norms(w, nullptr, m, nullptr, nullptr, 0, false, c.pw_part.p, st, stop, ticket, m > 0, s);
+        if (fast) launch_fast_pw_u(AT, w, u, st, stop, m > 0, s);
+        else launch_pw_u(AT, w, u, st, stop, m > 0, s);
+        launch_pw_norms(u, nullptr, n, w, st + PW_INV_W, m, true, c.pw_part.p, st, stop, ticket, n > 0, s);
     }
     CK(cudaGetLastError());
     double estimate = 0.0;
-    CK(cudaMemcpyAsync(&estimate, st + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&estimate, st + PW_EST, sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     *out = estimate;
     return PDHG_OK;

@@ -381,23 +381,26 @@ template <class T>
 void launch_fast_restart(const FastCheck<T>& a, cudaStream_t s);
 
 // ---- setup / final (kernels_exact.cu) ------------------------------------------
-// Exact pairwise sum of x[i]*y[i] (HostBackend::pairwise_dot order) into *out.
-void launch_pairwise_dot(const double* x, const double* y, int64_t n, double* partial,
-                         double* out, cudaStream_t s);
-int64_t pairwise_partial_size(int64_t n);
-// Power-iteration pieces (estimate_operator_norm, pdhg.cpp:48-79).
-// stop: a device flag that turns the launch into a no-op (null: always run)
-// fast: the rows' products added in parallel (not the reference's order)
-void launch_pw_w(const DevCsr& A, const double* u, const double* v, double* w, cudaStream_t s,
-                 const int* stop = nullptr, const double* uscale = nullptr, bool fast = false);
-void launch_pw_u(const DevCsr& AT, const double* w, double* u, cudaStream_t s,
-                 const int* stop = nullptr);
-void launch_scale(double* x, int64_t n, double alpha, cudaStream_t s);
-// the power iteration's scalar steps on the device (k_pw_norm_w / _e)
-void launch_pw_norm_w(const double* dot, double* st, int* stop, cudaStream_t s);
-void launch_pw_norm_e(const double* dots, double* st, int* stop, cudaStream_t s);
-void launch_scale_by(double* x, int64_t n, const double* alpha, const int* stop, cudaStream_t s);
-void launch_copy_unless(double* dst, const double* src, int64_t n, const int* stop, cudaStream_t s);
+// The power iteration (estimate_operator_norm, pdhg.cpp:48-79), its scalars in
+// three doubles st[], each launch early after the one before: the two products, and the exact pairwise norms
+// (HostBackend::pairwise_dot's order) with the scalar step on them. *stop: an
+// early exit. Values times *scale where a scale is given.
+enum PwSlot { PW_INV_W = 0, PW_EST, PW_INV_EST, PW_COUNT };
+int64_t pw_partial_size(int64_t n, int64_t m);  // doubles of `part`
+// both = false: 1 / ||x|| into st[PW_INV_W]; true: the estimate from ||x||, ||y||
+void launch_pw_norms(const double* x, const double* x_scale, int64_t nx, const double* y, const double* y_scale,
+                     int64_t ny, bool both, double* part, double* st, int* stop, unsigned int* ticket,
+                     bool early, cudaStream_t s);
+void launch_pw_w(const DevCsr& A, const double* u, double* w, const double* st, const int* stop, bool early,
+                 cudaStream_t s);
+void launch_pw_u(const DevCsr& AT, const double* w, double* u, const double* st, const int* stop, bool early,
+                 cudaStream_t s);
+// ... the products with each row's sum over the check's tiers, in parallel
+// (kernels_fast.cu; not the reference's order)
+void launch_fast_pw_w(const DevCsr& A, const double* u, double* w, const double* st, const int* stop, bool early,
+                      cudaStream_t s);
+void launch_fast_pw_u(const DevCsr& AT, const double* w, double* u, const double* st, const int* stop, bool early,
+                      cudaStream_t s);
 void launch_fill(double* x, int64_t n, double v, cudaStream_t s);
 
 struct FinalArgs {

@@ -17,6 +17,7 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -437,98 +438,41 @@ __global__ void __launch_bounds__(kBlock) ex_restart(ExactCheck a) {
 // Setup: power iteration pieces and the exact pairwise norm
 // ---------------------------------------------------------------------------
 
-// w = -(A u) + v  (spmv(A, -1, u, 0, w) then axpy(1, v, w), pdhg.cpp:59-60).
-// uscale (null: 1): u is read as u * uscale, the previous iteration's scaling
-// of u by 1 / estimate (pdhg.cpp:75) applied where u is gathered -- the same
-// rounded value as the scaled vector, without a pass over u.
-// FAST (the mixed and FP64 modes, whose estimate need not be the
-// reference's bit for bit): a warp row's products are added by its lanes in
-// parallel (four strided partial sums per lane, then a shuffle tree) instead
-// of in the row's order, which takes a long row from a chain of dependent
-// additions to a streaming pass.
-template <bool FAST>
-__global__ void __launch_bounds__(kBlock) k_pw_w(DevCsr A, const double* u, const double* v,
-                                                 double* w, const int* stop, const double* uscale) {
-    if (stop != nullptr && *stop) return;
+// The power iteration keeps w and u as computed and their scale factors in
+// st (PW_*): w / ||w|| (which becomes v) and u, v times 1 / estimate are formed
+// where they are read, each factor's product rounded, so every value is the one
+// the scaled vectors would hold (pdhg.cpp:58-75). Four launches an iteration:
+// the two products, and a norm kernel after each whose last CTA takes the
+// scalar step. *stop turns the launches after an early exit into no-ops.
+
+// w <- -(A u) + v (pdhg.cpp:59-60), v being the last iteration's w.
+__global__ void __launch_bounds__(kBlock) k_pw_w(DevCsr A, const double* u, double* w, const double* st,
+                                                 const int* stop) {
+    pass_begin();
     const RowTask t = row_task(A, blockIdx.x);
     if (t.row < 0) return;
-    const double us = uscale != nullptr ? *uscale : 1.0;
+    pass_wait();
+    if (*stop) return;
+    const double us = st[PW_INV_EST];
     const auto g = [u, us](int j) { return __dmul_rn(u[j], us); };
-    double sum;
-    if (FAST && t.warp) {
-        const int lane = threadIdx.x & 31;
-        const int b = A.rp[t.row], e = A.rp[t.row + 1];
-        double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
-        int k = b + lane;
-        for (; k + 96 < e; k += 128) {
-            p0 += A.v64[k] * g(A.ci[k]);
-            p1 += A.v64[k + 32] * g(A.ci[k + 32]);
-            p2 += A.v64[k + 64] * g(A.ci[k + 64]);
-            p3 += A.v64[k + 96] * g(A.ci[k + 96]);
-        }
-        for (; k < e; k += 32) p0 += A.v64[k] * g(A.ci[k]);
-        sum = (p0 + p1) + (p2 + p3);
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    } else if (t.warp) {
-        sum = ordered_dot_warp_pipelined(A.rp[t.row], A.rp[t.row + 1], A.ci, A.v64, g, 0.0,
-                                         warp_stage2());
-    } else {
-        sum = row_dot(t, A, g, 0.0);
-    }
-    if (t.lead) w[t.row] = __dadd_rn(-sum, v[t.row]);
+    const double sum = t.warp ? ordered_dot_warp_pipelined(A.rp[t.row], A.rp[t.row + 1], A.ci, A.v64, g, 0.0,
+                                                           warp_stage2())
+                              : row_dot(t, A, g, 0.0);
+    if (t.lead) w[t.row] = __dadd_rn(-sum, __dmul_rn(__dmul_rn(w[t.row], st[PW_INV_W]), us));
 }
 
 // u = A^T (-w) via spmv_transpose(A, -1, w, 0, u) (pdhg.cpp:67): u starts at
 // 0 and adds val * (-w_r) in row order.
-__global__ void __launch_bounds__(kBlock) k_pw_u(DevCsr AT, const double* w, double* u,
+__global__ void __launch_bounds__(kBlock) k_pw_u(DevCsr AT, const double* w, double* u, const double* st,
                                                  const int* stop) {
-    if (stop != nullptr && *stop) return;
+    pass_begin();
     const RowTask t = row_task(AT, blockIdx.x);
     if (t.row < 0) return;
-    const double sum = row_dot(t, AT, [w](int i) { return -w[i]; }, 0.0);
+    pass_wait();
+    if (*stop) return;
+    const double ws = st[PW_INV_W];
+    const double sum = row_dot(t, AT, [w, ws](int i) { return -__dmul_rn(w[i], ws); }, 0.0);
     if (t.lead) u[t.row] = sum;
-}
-
-// The power iteration's scalar steps on the device (pdhg.cpp:58-75, the
-// host's arithmetic: IEEE square roots and divisions, no contraction), so the
-// loop runs without a host round trip. st[0] = 1 / ||w||, st[1] = the
-// estimate, st[2] = 1 / estimate; *stop = 1 where the host loop breaks
-// (||w|| or the estimate below 1e-300), after which every step is a no-op.
-__global__ void k_pw_norm_w(const double* dot, double* st, int* stop) {
-    if (*stop) return;
-    const double wn = sqrt(dot[0]);
-    if (wn < 1e-300) {
-        *stop = 1;
-        return;
-    }
-    st[0] = 1.0 / wn;
-}
-__global__ void k_pw_norm_e(const double* dots, double* st, int* stop) {
-    if (*stop) return;
-    const double un = sqrt(dots[0]), vn = sqrt(dots[1]);
-    const double est = sqrt(__dadd_rn(__dmul_rn(un, un), __dmul_rn(vn, vn)));
-    st[1] = est;
-    if (est < 1e-300) {
-        *stop = 1;
-        return;
-    }
-    st[2] = 1.0 / est;
-}
-__global__ void k_scale_by(double* x, int64_t n, const double* alpha, const int* stop) {
-    if (*stop) return;
-    const double a = *alpha;
-    const int64_t t = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
-    if (t < n) x[t] = __dmul_rn(x[t], a);
-}
-__global__ void k_copy_unless(double* dst, const double* src, int64_t n, const int* stop) {
-    if (*stop) return;
-    const int64_t t = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
-    if (t < n) dst[t] = src[t];
-}
-
-__global__ void k_scale(double* x, int64_t n, double alpha) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
-    if (t < n) x[t] = __dmul_rn(x[t], alpha);
 }
 
 __global__ void k_fill(double* x, int64_t n, double v) {
@@ -559,44 +503,116 @@ __host__ __device__ inline void pw_node(int64_t n, int depth, int64_t idx, int64
     *size = s;
 }
 
-// The nodes of depth D-1, 32 consecutive nodes per CTA: their entries form
-// one contiguous range of at most 32 x 256 products, which all 256 threads
-// load with coalesced reads into shared memory; then thread l adds the
-// products of node l in index order (its left and right leaf sums, then
-// their sum), the recursion's sequence of additions for that node, so the
-// result is identical. (One thread per node reading its ~150 consecutive
-// entries from global memory alone made every warp-wide load touch 32 lines;
-// one warp per 32 nodes streaming the range in chunks left most lanes idle
-// while the others added.)
-constexpr int kPwNodes = 32;
+// One vector of a norm kernel: x (times *scale), n entries; nodes of depth
+// `depth`, kPwNodes per CTA.
+struct PwJob {
+    const double* x = nullptr;
+    const double* scale = nullptr;
+    int64_t n = 0;
+    int depth = 0, blocks = 0;
+};
+constexpr int kPwNodes = 32;     // a subtree of five levels
 constexpr int kPwMaxNode = 256;  // a depth D-1 node: at most two leaves of 128
-__global__ void __launch_bounds__(kBlock) k_pw_level_staged(const double* x, const double* y,
-                                                            int64_t n, int depth, double* out) {
+
+// Pairs (2t, 2t + 1) -> t, level by level, of `count` (a power of two) values
+// at `a`; `b` is scratch of the same kind. The total, valid in thread 0.
+__device__ double pw_fold(double* a, double* b, int64_t count) {
+    for (int64_t half = count / 2; half > 0; half /= 2) {
+        for (int64_t t = threadIdx.x; t < half; t += kBlock) b[t] = __dadd_rn(a[2 * t], a[2 * t + 1]);
+        __syncthreads();
+        double* tmp = a;
+        a = b;
+        b = tmp;
+    }
+    return a[0];
+}
+
+// The squared norms of one or two vectors (pairwise_dot of each with itself)
+// and the power iteration's scalar step on them. A CTA takes 32 consecutive
+// nodes of depth D-1: their entries form one contiguous range of at most
+// 32 x 256 products, which all 256 threads load with coalesced reads into
+// shared memory; thread l then adds the products of node l in index order (its
+// left and right leaf sums, then their sum), the recursion's sequence of
+// additions for that node, and the CTA folds its nodes, a whole subtree. The
+// last CTA folds the CTAs' values and takes the step: `both` = 0 the norm of w
+// (st[PW_INV_W]), 1 the estimate from the norms of u and v.
+__global__ void __launch_bounds__(kBlock) k_pw_norms(PwJob a, PwJob b, int both, double* part, double* st, int* stop,
+                                                     unsigned int* ticket) {
+    pass_begin();
     extern __shared__ double prod[];
     __shared__ int64_t off[kPwNodes + 1];
-    const int64_t nodes = int64_t{1} << depth;
-    const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kPwNodes;
+    __shared__ double node[2][kPwNodes];
+    const bool first = static_cast<int>(blockIdx.x) < a.blocks;
+    const PwJob job = first ? a : b;
+    const int64_t blk = first ? blockIdx.x : blockIdx.x - a.blocks;
+    const int64_t nodes = int64_t{1} << job.depth;
+    const int64_t t0 = blk * kPwNodes;
     const int cnt = nodes - t0 < kPwNodes ? static_cast<int>(nodes - t0) : kPwNodes;
     int64_t o = 0, sz = 0;
     if (threadIdx.x < cnt) {
-        pw_node(n, depth, t0 + threadIdx.x, &o, &sz);
+        pw_node(job.n, job.depth, t0 + threadIdx.x, &o, &sz);
         off[threadIdx.x] = o;
         if (threadIdx.x == cnt - 1) off[cnt] = o + sz;
     }
+    pass_wait();
+    if (*stop) return;  // set by the last CTA of a launch only: the same for all of this one
+    const double sc = job.scale != nullptr ? *job.scale : 1.0;
     __syncthreads();
     const int64_t r0 = off[0], len = off[cnt] - r0;
 #pragma unroll 4
-    for (int64_t i = threadIdx.x; i < len; i += kBlock) prod[i] = __dmul_rn(x[r0 + i], y[r0 + i]);
+    for (int64_t i = threadIdx.x; i < len; i += kBlock) {
+        const double v = __dmul_rn(job.x[r0 + i], sc);
+        prod[i] = __dmul_rn(v, v);
+    }
     __syncthreads();
-    if (threadIdx.x >= cnt) return;
-    const double* p = prod + (o - r0);
-    const int h = sz <= 128 ? static_cast<int>(sz) : static_cast<int>(sz / 2);
-    double accl = 0.0, accr = 0.0;
+    if (threadIdx.x < cnt) {
+        const double* p = prod + (o - r0);
+        const int h = sz <= 128 ? static_cast<int>(sz) : static_cast<int>(sz / 2);
+        double accl = 0.0, accr = 0.0;
 #pragma unroll 8
-    for (int i = 0; i < h; ++i) accl = __dadd_rn(accl, p[i]);
+        for (int i = 0; i < h; ++i) accl = __dadd_rn(accl, p[i]);
 #pragma unroll 8
-    for (int i = h; i < static_cast<int>(sz); ++i) accr = __dadd_rn(accr, p[i]);
-    out[t0 + threadIdx.x] = sz <= 128 ? accl : __dadd_rn(accl, accr);
+        for (int i = h; i < static_cast<int>(sz); ++i) accr = __dadd_rn(accr, p[i]);
+        node[0][threadIdx.x] = sz <= 128 ? accl : __dadd_rn(accl, accr);
+    }
+    __syncthreads();
+    const double sum = pw_fold(node[0], node[1], cnt);
+    if (threadIdx.x == 0) part[blockIdx.x] = sum;
+    if (!last_block(ticket)) return;
+    // the CTAs' values: folded in shared memory, more than 2,048 of them after
+    // a first level in global memory
+    double dot[2] = {0.0, 0.0};
+    for (int q = 0; q < (both ? 2 : 1); ++q) {
+        int64_t count = q == 0 ? a.blocks : b.blocks;
+        double* src = part + (q == 0 ? 0 : a.blocks);
+        if (count == 0) continue;
+        __syncthreads();
+        if (count <= 2048) {
+            for (int64_t i = threadIdx.x; i < count; i += kBlock) prod[i] = __ldcg(src + i);
+            __syncthreads();
+            dot[q] = pw_fold(prod, prod + count, count);
+        } else {
+            double* dst = part + a.blocks + b.blocks;
+            count /= 2;
+            for (int64_t t = threadIdx.x; t < count; t += kBlock)
+                dst[t] = __dadd_rn(__ldcg(src + 2 * t), __ldcg(src + 2 * t + 1));
+            __syncthreads();
+            dot[q] = pw_fold(dst, src, count);
+        }
+    }
+    if (threadIdx.x != 0) return;
+    *ticket = 0u;
+    if (!both) {
+        const double wn = sqrt(dot[0]);
+        if (wn < 1e-300) *stop = 1;
+        else st[PW_INV_W] = 1.0 / wn;
+        return;
+    }
+    const double un = sqrt(dot[0]), vn = sqrt(dot[1]);
+    const double est = sqrt(__dadd_rn(__dmul_rn(un, un), __dmul_rn(vn, vn)));
+    st[PW_EST] = est;
+    if (est < 1e-300) *stop = 1;
+    else st[PW_INV_EST] = 1.0 / est;
 }
 
 int pw_depth(int64_t n) {
@@ -610,28 +626,6 @@ int pw_depth(int64_t n) {
         ++D;
     }
     return D - 1;
-}
-
-// Uniform-barrier fold: one level per launch of a simple kernel (setup only).
-__global__ void k_pw_fold_level(const double* in, double* out, int64_t half) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
-    if (t < half) out[t] = __dadd_rn(in[2 * t], in[2 * t + 1]);
-}
-
-// Folds the remaining 2^levels (<= 1024) values in one CTA, level by level,
-// pairs (2t, 2t+1) -> t exactly as k_pw_fold_level; every thread runs the same
-// number of levels, so the barriers are uniform.
-__global__ void __launch_bounds__(512) k_pw_fold_tail(double* a, double* b, int levels,
-                                                      double* out) {
-    for (int lvl = levels; lvl > 0; --lvl) {
-        const int half = 1 << (lvl - 1);
-        for (int t = threadIdx.x; t < half; t += blockDim.x) b[t] = __dadd_rn(a[2 * t], a[2 * t + 1]);
-        __syncthreads();
-        double* tmp = a;
-        a = b;
-        b = tmp;
-    }
-    if (threadIdx.x == 0) *out = a[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -973,63 +967,54 @@ void launch_exact_restart(const ExactCheck& a, cudaStream_t s) {
     ex_restart<<<nmax > 0 ? blocks_for(nmax) : 1, kBlock, 0, s>>>(a);
 }
 
-int64_t pairwise_partial_size(int64_t n) {
-    const int d = pw_depth(n);
-    return (int64_t{1} << d) * 2 + 2;
+namespace {
+
+PwJob pw_job(const double* x, const double* scale, int64_t n) {
+    PwJob j;
+    j.x = x;
+    j.scale = scale;
+    j.n = n;
+    j.depth = pw_depth(n);
+    j.blocks = n > 0 ? static_cast<int>(((int64_t{1} << j.depth) + kPwNodes - 1) / kPwNodes) : 0;
+    return j;
 }
 
-void launch_pairwise_dot(const double* x, const double* y, int64_t n, double* partial,
-                         double* out, cudaStream_t s) {
-    if (n <= 0) {
-        launch_fill(out, 1, 0.0, s);
-        return;
-    }
-    const int d = pw_depth(n);
-    const int64_t count = int64_t{1} << d;
-    double* a = partial;
-    double* b = partial + count;
+size_t pw_smem(const PwJob& j) {
     // the CTA's range: 32 nodes of at most ceil(n / 2^d) <= 256 entries
-    const int64_t per = (n + count - 1) / count;
-    const size_t smem = sizeof(double) * static_cast<size_t>(kPwNodes * per);
-    if (smem > 48 * 1024)  // up to 64 KB: above the default dynamic limit
-        cudaFuncSetAttribute(k_pw_level_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(sizeof(double) * kPwNodes * kPwMaxNode));
-    k_pw_level_staged<<<static_cast<unsigned>((count + kPwNodes - 1) / kPwNodes), kBlock, smem, s>>>(
-        x, y, n, d, a);
-    int lvl = d;
-    for (; lvl > 10; --lvl) {  // wide levels: one launch each
-        const int64_t half = int64_t{1} << (lvl - 1);
-        k_pw_fold_level<<<grid64(half), kBlock, 0, s>>>(a, b, half);
-        double* t = a;
-        a = b;
-        b = t;
-    }
-    k_pw_fold_tail<<<1, 512, 0, s>>>(a, b, lvl, out);  // the last <= 1024 values in one CTA
+    const int64_t count = int64_t{1} << j.depth;
+    const int64_t per = j.n > 0 ? (j.n + count - 1) / count : 0;
+    return sizeof(double) * static_cast<size_t>(kPwNodes * per);
 }
 
-void launch_pw_w(const DevCsr& A, const double* u, const double* v, double* w, cudaStream_t s,
-                 const int* stop, const double* uscale, bool fast) {
-    if (A.rows == 0) return;
-    if (fast) k_pw_w<true><<<mat_blocks(A), kBlock, 0, s>>>(A, u, v, w, stop, uscale);
-    else k_pw_w<false><<<mat_blocks(A), kBlock, 0, s>>>(A, u, v, w, stop, uscale);
+}  // namespace
+
+int64_t pw_partial_size(int64_t n, int64_t m) {
+    const int64_t blocks = pw_job(nullptr, nullptr, n).blocks + pw_job(nullptr, nullptr, m).blocks;
+    return 2 * blocks + 2;  // the CTAs' values and a fold's other half
 }
-void launch_pw_u(const DevCsr& AT, const double* w, double* u, cudaStream_t s, const int* stop) {
-    if (AT.rows > 0) k_pw_u<<<mat_blocks(AT), kBlock, 0, s>>>(AT, w, u, stop);
+
+void launch_pw_norms(const double* x, const double* x_scale, int64_t nx, const double* y, const double* y_scale,
+                     int64_t ny, bool both, double* part, double* st, int* stop, unsigned int* ticket,
+                     bool early, cudaStream_t s) {
+    if (nx + ny <= 0) return;
+    const PwJob a = pw_job(x, x_scale, nx), b = both ? pw_job(y, y_scale, ny) : PwJob{};
+    // the last CTA's folds need up to 2 x 2,048 doubles
+    size_t smem = std::max(pw_smem(a), pw_smem(b));
+    smem = std::max(smem, sizeof(double) * std::min<size_t>(4096, 2 * static_cast<size_t>(std::max(a.blocks, b.blocks))));
+    if (smem > 48 * 1024)  // up to 64 KB: above the default dynamic limit
+        cudaFuncSetAttribute(k_pw_norms, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(sizeof(double) * kPwNodes * kPwMaxNode));
+    if (a.blocks + b.blocks > 0)
+        launch_pass_smem(k_pw_norms, a.blocks + b.blocks, early, s, smem, a, b, both ? 1 : 0, part, st, stop, ticket);
 }
-void launch_scale(double* x, int64_t n, double alpha, cudaStream_t s) {
-    if (n > 0) k_scale<<<grid64(n), kBlock, 0, s>>>(x, n, alpha);
+
+void launch_pw_w(const DevCsr& A, const double* u, double* w, const double* st, const int* stop, bool early,
+                 cudaStream_t s) {
+    if (A.rows > 0) launch_pass(k_pw_w, mat_blocks(A), early, s, A, u, w, st, stop);
 }
-void launch_pw_norm_w(const double* dot, double* st, int* stop, cudaStream_t s) {
-    k_pw_norm_w<<<1, 1, 0, s>>>(dot, st, stop);
-}
-void launch_pw_norm_e(const double* dots, double* st, int* stop, cudaStream_t s) {
-    k_pw_norm_e<<<1, 1, 0, s>>>(dots, st, stop);
-}
-void launch_scale_by(double* x, int64_t n, const double* alpha, const int* stop, cudaStream_t s) {
-    if (n > 0) k_scale_by<<<grid64(n), kBlock, 0, s>>>(x, n, alpha, stop);
-}
-void launch_copy_unless(double* dst, const double* src, int64_t n, const int* stop, cudaStream_t s) {
-    if (n > 0) k_copy_unless<<<grid64(n), kBlock, 0, s>>>(dst, src, n, stop);
+void launch_pw_u(const DevCsr& AT, const double* w, double* u, const double* st, const int* stop, bool early,
+                 cudaStream_t s) {
+    if (AT.rows > 0) launch_pass(k_pw_u, mat_blocks(AT), early, s, AT, w, u, st, stop);
 }
 void launch_fill(double* x, int64_t n, double v, cudaStream_t s) {
     if (n > 0) k_fill<<<grid64(n), kBlock, 0, s>>>(x, n, v);

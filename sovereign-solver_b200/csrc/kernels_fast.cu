@@ -1587,8 +1587,10 @@ __device__ __forceinline__ void fin_terms(const FinalArgs& a, int r, double dot,
     (ROWS ? a.f.trow : a.f.tcol)[r] = fin_inf_over_box(v, lo, hi);
 }
 
-// Entries k, k + step, ... below e of M times x, four of each stream in flight.
-__device__ __forceinline__ double fin_products(const DevCsr& M, const double* x, int k, int e, int step) {
+// Entries k, k + step, ... below e of M times g(column), four of each stream
+// in flight.
+template <class G>
+__device__ __forceinline__ double tier_products(const DevCsr& M, G g, int k, int e, int step) {
     double s0 = 0.0, s1 = 0.0;
     for (; k < e; k += 4 * step) {
         int c[4];
@@ -1600,17 +1602,17 @@ __device__ __forceinline__ double fin_products(const DevCsr& M, const double* x,
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (k + u * step < e) (u & 1 ? s1 : s0) += v[u] * x[c[u]];
+            if (k + u * step < e) (u & 1 ? s1 : s0) += v[u] * g(c[u]);
     }
     return s0 + s1;
 }
 
 // Virtual block vb of one matrix, split like the check's (check_part): lane
-// groups, warp rows, CTA items with split rows. One warp per row, in row
-// order, took the badly scaled LP's longest row (344,267 entries) 7.0 ms.
-template <bool ROWS>
-__device__ void fin_part(const FinalArgs& a, const DevCsr& M, int vb, int sb, int wb, double& pinf, double& dinf) {
-    const double* x = ROWS ? a.f.xo : a.f.yo;
+// groups, warp rows, CTA items with split rows; row(r, dot) on one thread per
+// row. One warp per row, in row order, took the badly scaled LP's longest row
+// (344,267 entries) 7.0 ms.
+template <class G, class R>
+__device__ __forceinline__ void tier_part(const DevCsr& M, int vb, int sb, int wb, G g, R row) {
     if (vb < sb) {
         const int vw = M.vw;
         const int lane = threadIdx.x & (vw - 1);
@@ -1618,34 +1620,63 @@ __device__ void fin_part(const FinalArgs& a, const DevCsr& M, int vb, int sb, in
         if (r >= M.rows) return;
         const int b = M.rp[r], e = M.rp[r + 1];
         if (e - b > M.short_max) return;
-        const double dot = group_sum(fin_products(M, x, b + lane, e, vw), vw);
-        if (lane == 0) fin_terms<ROWS>(a, r, dot, pinf, dinf);
+        const double dot = group_sum(tier_products(M, g, b + lane, e, vw), vw);
+        if (lane == 0) row(r, dot);
     } else if (vb < sb + wb) {
         const int w = (vb - sb) * (kBlock / 32) + (threadIdx.x >> 5);
         if (w >= M.n_warp0) return;
         const int r = M.warp_rows0[w];
         const int lane = threadIdx.x & 31;
-        double dot = fin_products(M, x, M.rp[r] + lane, M.rp[r + 1], 32);
+        double dot = tier_products(M, g, M.rp[r] + lane, M.rp[r + 1], 32);
         for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (lane == 0) fin_terms<ROWS>(a, r, dot, pinf, dinf);
+        if (lane == 0) row(r, dot);
     } else {
         const int idx = vb - sb - wb;
         const int4 w = M.items_long.item[idx];
-        double dot = block_total(fin_products(M, x, w.y + threadIdx.x, w.z, kBlock)), unused;
+        double dot = block_total(tier_products(M, g, w.y + threadIdx.x, w.z, kBlock)), unused;
         if (w.w >= 0 && !segment_finish(M.items_long, idx, w.w, dot, 0.0, &dot, &unused)) return;
-        if (threadIdx.x == 0) fin_terms<ROWS>(a, w.x, dot, pinf, dinf);
+        if (threadIdx.x == 0) row(w.x, dot);
     }
+}
+__host__ __device__ inline int tier_blocks(const DevCsr& M) {
+    return check_short_blocks(M) + check_warp_blocks(M) + M.items_long.n_item;
+}
+
+// The power iteration's products (k_pw_w, k_pw_u) over the tiers, one virtual
+// block per CTA, the longest rows' items first.
+__global__ void __launch_bounds__(kBlock) fast_pw_w(DevCsr A, const double* u, double* w, const double* st,
+                                                    const int* stop) {
+    pass_begin();
+    pass_wait();
+    if (*stop) return;
+    const double us = st[PW_INV_EST], ws = st[PW_INV_W];
+    tier_part(A, static_cast<int>(gridDim.x - 1 - blockIdx.x), check_short_blocks(A), check_warp_blocks(A),
+              [u, us](int j) { return u[j] * us; }, [&](int r, double dot) { w[r] = w[r] * ws * us - dot; });
+}
+__global__ void __launch_bounds__(kBlock) fast_pw_u(DevCsr AT, const double* w, double* u, const double* st,
+                                                    const int* stop) {
+    pass_begin();
+    pass_wait();
+    if (*stop) return;
+    const double ws = st[PW_INV_W];
+    tier_part(AT, static_cast<int>(gridDim.x - 1 - blockIdx.x), check_short_blocks(AT), check_warp_blocks(AT),
+              [w, ws](int i) { return w[i] * ws; }, [&](int r, double dot) { u[r] = -dot; });
 }
 
 __global__ void __launch_bounds__(kBlock) fast_final(FinalArgs a) {
     double pinf = 0.0, dinf = 0.0;
     const int sbA = check_short_blocks(a.Ao), wbA = check_warp_blocks(a.Ao);
     const int sbT = check_short_blocks(a.ATo), wbT = check_warp_blocks(a.ATo);
-    const int nA = sbA + wbA + a.Ao.items_long.n_item, nT = sbT + wbT + a.ATo.items_long.n_item;
+    const int nA = tier_blocks(a.Ao), nT = tier_blocks(a.ATo);
     for (int bid = blockIdx.x; bid < nA + nT; bid += gridDim.x) {  // the longest items first
         const int vb = bid < nA ? nA - 1 - bid : nA + nT - 1 - bid;
-        if (bid < nA) fin_part<true>(a, a.Ao, vb, sbA, wbA, pinf, dinf);
-        else fin_part<false>(a, a.ATo, vb, sbT, wbT, pinf, dinf);
+        const double *xo = a.f.xo, *yo = a.f.yo;
+        if (bid < nA)
+            tier_part(a.Ao, vb, sbA, wbA, [xo](int j) { return xo[j]; },
+                      [&](int r, double dot) { fin_terms<true>(a, r, dot, pinf, dinf); });
+        else
+            tier_part(a.ATo, vb, sbT, wbT, [yo](int i) { return yo[i]; },
+                      [&](int r, double dot) { fin_terms<false>(a, r, dot, pinf, dinf); });
     }
     for (int o = 16; o > 0; o >>= 1) {
         pinf = fmax(pinf, __shfl_xor_sync(0xffffffffu, pinf, o));
@@ -1662,10 +1693,18 @@ __global__ void __launch_bounds__(kBlock) fast_final(FinalArgs a) {
 }  // namespace
 
 void launch_fast_final_rows(const FinalArgs& a, cudaStream_t s) {
-    int64_t g = 0;
-    for (const DevCsr* M : {&a.Ao, &a.ATo}) g += check_short_blocks(*M) + check_warp_blocks(*M) + M->items_long.n_item;
+    int g = tier_blocks(a.Ao) + tier_blocks(a.ATo);
     if (g > 148 * 16) g = 148 * 16;
-    if (g > 0) fast_final<<<static_cast<int>(g), kBlock, 0, s>>>(a);
+    if (g > 0) fast_final<<<g, kBlock, 0, s>>>(a);
+}
+
+void launch_fast_pw_w(const DevCsr& A, const double* u, double* w, const double* st, const int* stop, bool early,
+                      cudaStream_t s) {
+    if (A.rows > 0) launch_pass(fast_pw_w, tier_blocks(A), early, s, A, u, w, st, stop);
+}
+void launch_fast_pw_u(const DevCsr& AT, const double* w, double* u, const double* st, const int* stop, bool early,
+                      cudaStream_t s) {
+    if (AT.rows > 0) launch_pass(fast_pw_u, tier_blocks(AT), early, s, AT, w, u, st, stop);
 }
 
 template <class K>

@@ -53,15 +53,17 @@ __device__ __forceinline__ V gather_ld(const V* p) {
     else return __ldg(p);
 }
 
-// Launches one pass of an iteration. early: the launch may begin while the
-// kernel before it in the stream still runs (programmatic dependent launch);
-// only after a kernel that begins with pass_begin, and with no other
+// Launches one pass (smem: dynamic shared memory). early: the launch may begin
+// while the kernel before it in the stream still runs (programmatic dependent
+// launch); only after a kernel that begins with pass_begin, and with no other
 // predecessor.
 template <class... P, class... Q>
-cudaError_t launch_pass(void (*kernel)(P...), int grid, bool early, cudaStream_t s, const Q&... args) {
+cudaError_t launch_pass_smem(void (*kernel)(P...), int grid, bool early, cudaStream_t s, size_t smem,
+                             const Q&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));
     cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -69,6 +71,10 @@ cudaError_t launch_pass(void (*kernel)(P...), int grid, bool early, cudaStream_t
     cfg.attrs = at;
     cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <class... P, class... Q>
+cudaError_t launch_pass(void (*kernel)(P...), int grid, bool early, cudaStream_t s, const Q&... args) {
+    return launch_pass_smem(kernel, grid, early, s, 0, args...);
 }
 
 }  // namespace
