@@ -67,6 +67,20 @@ struct BatchCtx {
     DBuf<double> xa64, sa64, ya64;
     DBuf<float> xa32, sa32, ya32;
 
+    // instances on clusters (batch_resident.cu): their parts, and the plan per
+    // precision and form made since the load
+    DBuf<ResParts> parts_d;
+    std::vector<ResParts> parts;
+    struct Plan {
+        bool made = false, fits = false;
+        std::vector<ResClass> classes;
+        DBuf<int32_t> list;
+        DBuf<ResFar> where;
+        size_t far_bytes = 0;
+    } plan[2][2];  // [FP32, FP64][averaged, Halpern]
+    DBuf<unsigned char> far;  // entries of instances too large for shared memory, set up by each solve
+    ResStreams side;
+
     // solve graphs, [0] FP32 and [1] FP64, with what they bake in
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     long long graph_key[2][11] = {};
@@ -81,6 +95,11 @@ struct BatchCtx {
     BatchCtx(int dev, cudaStream_t s, std::string& e) : device(dev), stream(s), err(e) {}
     ~BatchCtx() {
         drop_graphs();
+        if (side.fork != nullptr) cudaEventDestroy(side.fork);
+        for (int i = 0; i < kResClasses - 1; ++i) {
+            if (side.join[i] != nullptr) cudaEventDestroy(side.join[i]);
+            if (side.stream[i] != nullptr) cudaStreamDestroy(side.stream[i]);
+        }
         if (mail != nullptr) cudaFreeHost(mail);
     }
     void drop_graphs() {
@@ -303,7 +322,13 @@ int batch_intake(BatchCtx& c, const pdhg_options& o) {
     BCK(to_float(c.rhi32, c.rhi_s, s));
     b = c.view();
     launch_batch_norms(b, s);
+    c.parts.resize(2 * static_cast<size_t>(c.count));
+    BCK(c.parts_d.alloc(c.parts.size()));
+    launch_batch_parts(b, c.parts_d.p, s);
+    BCK(cudaMemcpyAsync(c.parts.data(), c.parts_d.p, sizeof(ResParts) * c.parts.size(), cudaMemcpyDeviceToHost, s));
     BCK(cudaStreamSynchronize(s));
+    for (auto& f : c.plan)
+        for (auto& pl : f) pl.made = false;
     c.have_opnorm = false;
     return PDHG_OK;
 }
@@ -596,6 +621,39 @@ int batch_tune(BatchCtx& c, bool autotune) {
     return PDHG_OK;
 }
 
+// Lanes (log2) per row on a cluster: the binning's, at most four. In shared
+// memory a row's entries are near, and eight lanes on a row of 18 entries cost
+// more slots than they save steps.
+int lanes_log2(int vw) { return vw >= 4 ? 2 : vw / 2; }
+
+// The plan of this precision and form, made on its first solve since the load.
+template <class T>
+int batch_plan(BatchCtx& c, BatchCtx::Plan** out) {
+    BatchCtx::Plan& pl = c.plan[std::is_same<T, float>::value ? 0 : 1][c.halpern ? 1 : 0];
+    *out = &pl;
+    if (pl.made) return PDHG_OK;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    ResPlan r;
+    pl.fits = plan_resident<T>(c.parts, lanes_log2(c.bin_vw[1]), lanes_log2(c.bin_vw[0]), c.halpern, sms, r);
+    if (pl.fits) {
+        pl.classes = r.classes;
+        pl.far_bytes = static_cast<size_t>(r.far_bytes);
+        BCK(upload(pl.list, r.list, c.stream));
+        BCK(upload(pl.where, r.where, c.stream));
+        BCK(cudaStreamSynchronize(c.stream));  // the host vectors are read by the copies above
+        if (c.side.fork == nullptr) {
+            BCK(cudaEventCreateWithFlags(&c.side.fork, cudaEventDisableTiming));
+            for (int i = 0; i < kResClasses - 1; ++i) {
+                BCK(cudaStreamCreateWithFlags(&c.side.stream[i], cudaStreamNonBlocking));
+                BCK(cudaEventCreateWithFlags(&c.side.join[i], cudaEventDisableTiming));
+            }
+        }
+    }
+    pl.made = true;
+    return PDHG_OK;
+}
+
 // Runs check periods from iteration iter0 (the global count) until every
 // instance is done or iteration `last` (absolute) is reached; returns the
 // negated stop code when the host asked the device to stop.
@@ -615,7 +673,6 @@ int batch_run(BatchCtx& c, const pdhg_options& o, std::chrono::steady_clock::tim
     p.y_last = c.y_last.p;
     p.act_avg = c.act_avg.p;
     p.allow_switch = allow_switch ? 1 : 0;
-    launch_batch_compact(c.view(), s);  // the block lists of the instances now active
     const long long span = last > iter0 ? last - iter0 : 0;
     const long long n_periods = span / p.period;
     const long long tail = span % p.period;
@@ -634,6 +691,42 @@ int batch_run(BatchCtx& c, const pdhg_options& o, std::chrono::steady_clock::tim
             stop_sent = true;
         }
     };
+    auto wait = [&]() -> int {  // the device runs to the end; the host only polls limits
+        if (o.cancel_flag == nullptr && !(o.time_limit_seconds > 0.0)) {
+            BCK(cudaStreamSynchronize(s));
+            return PDHG_OK;
+        }
+        while (true) {
+            const cudaError_t q = cudaStreamQuery(s);
+            if (q == cudaSuccess) return PDHG_OK;
+            if (q != cudaErrorNotReady) return cuda_fail(&c.err, q, "cudaStreamQuery");
+            poll();
+            std::this_thread::sleep_for(std::chrono::microseconds(200));
+        }
+    };
+    BatchCtx::Plan* plan = nullptr;
+    if (int rc = batch_plan<T>(c, &plan); rc != PDHG_OK) return rc;
+    bool resident = plan->fits;
+    if (resident && c.far.n < plan->far_bytes && c.far.alloc(plan->far_bytes) != cudaSuccess) {
+        c.far.release();
+        cudaGetLastError();  // no room for the second copy: the kernels over all instances need none
+        resident = false;
+    }
+    if (resident) {
+        const ResBuffers buf{plan->list.p, c.parts_d.p, plan->where.p, c.far.p};
+        BCK(launch_batch_resident<T>(plan->classes, buf, lanes_log2(c.bin_vw[1]), lanes_log2(c.bin_vw[0]), c.view(),
+                                     batch_iterates<T>(c), p, iter0, n_periods, tail, s, c.side));
+        *launches += static_cast<long long>(plan->classes.size());
+        if (int rc = wait(); rc != PDHG_OK) return rc;
+        BatchGlobal gh;
+        BCK(cudaMemcpy(&gh, c.g.p, sizeof gh, cudaMemcpyDeviceToHost));
+        if (!gh.done && tail > 0 && !stop_sent) {
+            gh.iter += tail;
+            BCK(cudaMemcpy(c.g.p, &gh, sizeof gh, cudaMemcpyHostToDevice));
+        }
+        return stop_sent ? -c.mail->stop_request : PDHG_OK;
+    }
+    launch_batch_compact(c.view(), s);  // the block lists of the instances now active
     if (n_periods > 0) {
         const int gi = std::is_same<T, float>::value ? 0 : 1;
         long long key[11];
@@ -655,13 +748,7 @@ int batch_run(BatchCtx& c, const pdhg_options& o, std::chrono::steady_clock::tim
         }
         BCK(cudaGraphLaunch(c.graph[gi], s));
         *launches += 1;
-        while (true) {  // the graph runs to the end on the device; the host only polls limits
-            const cudaError_t q = cudaStreamQuery(s);
-            if (q == cudaSuccess) break;
-            if (q != cudaErrorNotReady) return cuda_fail(&c.err, q, "cudaStreamQuery");
-            poll();
-            std::this_thread::sleep_for(std::chrono::microseconds(200));
-        }
+        if (int rc = wait(); rc != PDHG_OK) return rc;
     }
     BatchGlobal gh;
     BCK(cudaMemcpy(&gh, c.g.p, sizeof gh, cudaMemcpyDeviceToHost));

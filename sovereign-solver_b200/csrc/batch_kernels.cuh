@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "engine.cuh"
 
@@ -140,6 +141,58 @@ constexpr int kBatchStalled = 100;
 // FP32 iterates widened into the FP64 ones (the polish phase starts there).
 void launch_batch_widen(const BatchView& b, const Iterates<float>& f, const Iterates<double>& d,
                         cudaStream_t s);
+
+// ---- batch_resident.cu: instances that fit a cluster's shared memory --------
+// A matrix's rows in 16 consecutive parts of about equal work: the shares of a
+// cluster's CTAs. Part q is the rows [row[q], row[q + 1]) and the entries
+// [nz[q], nz[q + 1]), counted from the instance's first.
+constexpr int kResMaxCluster = 16;
+struct ResParts {
+    int32_t row[kResMaxCluster + 1] = {};
+    int32_t nz[kResMaxCluster + 1] = {};
+    int32_t longest = 0;  // entries of the longest row of at most kLongRow
+};
+// Instances that run on like clusters: `count` of the list from `first` on.
+struct ResClass {
+    int size = 1, threads = 1024;
+    int32_t first = 0, count = 0;
+    uint32_t smem = 0;
+    bool far = false;  // the entries in global memory
+};
+constexpr int kResClasses = 11;
+// Where a far instance's entries are: byte offset, and entries per CTA of its
+// columns and of its rows.
+struct ResFar {
+    int64_t base = 0;
+    uint32_t entries[2] = {0, 0};
+};
+struct ResPlan {
+    std::vector<ResClass> classes;
+    std::vector<int32_t> list;  // instances by class
+    std::vector<ResFar> where;  // of each of them
+    int64_t far_bytes = 0;
+};
+struct ResBuffers {
+    const int32_t* list = nullptr;
+    const ResParts* parts = nullptr;  // 2 per instance
+    const ResFar* where = nullptr;
+    unsigned char* far = nullptr;
+};
+// Streams and events for the classes after the first, which run side by side.
+struct ResStreams {
+    cudaStream_t stream[kResClasses - 1] = {};
+    cudaEvent_t fork = nullptr, join[kResClasses - 1] = {};
+};
+void launch_batch_parts(const BatchView& b, ResParts* parts, cudaStream_t s);  // 2 per instance
+// False where some instance fits no cluster in precision T. lgt, lga: log2 of
+// the lanes per row of A^T's and of A's rows.
+template <class T>
+bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, int sms, ResPlan& plan);
+// n_periods check periods from iteration iter0 on, then `tail` iterations.
+template <class T>
+cudaError_t launch_batch_resident(const std::vector<ResClass>& classes, const ResBuffers& buf, int lgt, int lga,
+                                  const BatchView& b, const Iterates<T>& it, const BatchParams& p, long long iter0,
+                                  long long n_periods, long long tail, cudaStream_t s, const ResStreams& side);
 
 // final result per instance (pdhg.cpp:420-498); `which`: -1 every instance,
 // 0 those not polished, 1 the polished ones.

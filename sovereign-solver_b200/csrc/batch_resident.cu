@@ -1,0 +1,428 @@
+// batch_resident.cu -- a batch whose instances fit the shared memory of a
+// cluster each: one cluster runs one instance's whole solve (resident.cuh),
+// every check period of it with the check, the decision and the restart, and
+// the next instance takes its place. No instance waits for another: an
+// instance that converges early frees its SMs, where the kernels over all
+// instances (batch_kernels.cu) launch two passes an iteration until the slowest
+// is done. Those remain for batches with an instance that does not fit.
+//
+// Bound: an iteration's two dependent passes over shared memory (per entry 8-12
+// bytes and a gather that conflicts) and two barriers; many instances: the SMs.
+// Measured per iteration, instances of one size, FP32: 60 x 150 1.3 us, 500 x
+// 1,200 3.4 us (one or 67 of them), 2,000 x 5,000 4.4 us, 5,000 x 15,000
+// (entries in global memory) 10 us. 67 FP64 instances of 500 x 1,200: a check
+// period of 40 iterations 519 -> 205 us; 256 FP32 instances of 50 to 5,000 rows
+// 2,009 -> 1,173 us. 1,024 threads at 64 registers or 512 at
+// 128 for the large classes: within 10% of each other either way.
+#include <algorithm>
+#include <vector>
+
+#include "batch_device.cuh"
+#include "batch_kernels.cuh"
+#include "resident.cuh"
+
+namespace pdhg {
+
+namespace {
+
+constexpr int K = kBatchCheckVals;
+
+// Rows of a matrix in kResMaxCluster parts of about equal work (entries plus
+// kResRowWork per row), one thread per boundary, each a multiple of four rows
+// (whole 16-byte vectors of the row vectors).
+constexpr int64_t kResRowWork = 8;
+__global__ void __launch_bounds__(kBlock) k_batch_parts(const int32_t* rp0, const int32_t* off, int which,
+                                                        ResParts* out) {
+    const int k = blockIdx.x, q = threadIdx.x;
+    const int32_t* rp = rp0 + off[k];
+    const int32_t rows = off[k + 1] - off[k];
+    ResParts& o = out[2 * k + which];
+    int longest = 0;
+    for (int i = q; i < rows; i += kBlock) {
+        const int len = rp[i + 1] - rp[i];
+        if (len <= kLongRow) longest = max(longest, len);
+    }
+    __shared__ int most;
+    if (q == 0) most = 0;
+    __syncthreads();
+    atomicMax(&most, longest);
+    __syncthreads();
+    if (q == 0) o.longest = most;
+    if (q > kResMaxCluster) return;
+    const int64_t base = rp[0];
+    const int64_t want = (rp[rows] - base + kResRowWork * rows) * q / kResMaxCluster;
+    int lo = 0, hi = rows;  // the first row whose work before it reaches `want`
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (rp[mid] - base + kResRowWork * mid < want) lo = mid + 1;
+        else hi = mid;
+    }
+    if (q < kResMaxCluster) lo &= ~3;
+    o.row[q] = lo;
+    o.nz[q] = static_cast<int32_t>(rp[lo] - base);
+}
+
+// Block maxima (values 0..7) and sums (8..15), the warps' results combined in
+// warp order: thread q < K gets value q.
+template <int NT>
+__device__ __forceinline__ double reduce_vals(const double (&v)[K], double (*red)[NT / 32]) {
+    const int lane = static_cast<int>(threadIdx.x & 31), warp = static_cast<int>(threadIdx.x >> 5);
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        double x = v[q];
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_xor_sync(0xffffffffu, x, o);
+            x = q < 8 ? fmax(x, y) : x + y;
+        }
+        if (lane == 0) red[q][warp] = x;
+    }
+    __syncthreads();
+    double x = 0.0;
+    if (threadIdx.x < K)
+        for (int w = 0; w < NT / 32; ++w)
+            x = threadIdx.x < 8 ? fmax(x, red[threadIdx.x][w]) : x + red[threadIdx.x][w];
+    __syncthreads();
+    return x;
+}
+
+// The check's products and terms (inst_pass) over the CTA's rows or columns.
+template <int NT, class T, bool COLS, bool HALPERN, bool FAR>
+__device__ __forceinline__ void check_rows(const BatchView& b, const Iterates<T>& it, const BatchParams& p,
+                                           const ResSlab<T, FAR>& S, int first, double inv, double sign, Terms& t) {
+    const DevCsr& M = COLS ? b.AT : b.A;
+    const int vw = 1 << S.lg;
+    const int lane = static_cast<int>(threadIdx.x) & (vw - 1);
+    const int r1 = first + S.r1;
+    for (int r = first + S.r0 + (static_cast<int>(threadIdx.x) >> S.lg); r < r1; r += NT >> S.lg) {
+        double ac = 0.0, aa = 0.0;
+        const int e = M.rp[r + 1];
+        for (int q = M.rp[r] + lane; q < e; q += vw) {
+            const int c = M.ci[q];
+            const double v = M.v64[q];
+            if (!HALPERN) ac += v * static_cast<double>(COLS ? it.y[c] : it.x[c]);
+            aa += v * (COLS ? avg_y<T, HALPERN>(it, c, inv) : avg_x<T, HALPERN>(it, c, inv));
+        }
+        if (!HALPERN) ac = group_sum(ac, vw);
+        aa = group_sum(aa, vw);
+        if (HALPERN) ac = aa;  // only T(z) is measured
+        if (lane == 0) {
+            if (COLS) inst_col_terms(b, it, p, sign, r, ac, aa, inv, t);
+            else inst_row_terms(b, it, p, r, ac, aa, inv, t);
+        }
+    }
+}
+
+struct ResJob {
+    const int32_t* list;    // instances, one per cluster
+    const ResParts* parts;  // per instance: of A^T's rows, of A's
+    int lgt, lga;           // log2 of the lanes per row
+    // FAR: each cluster's entries in global memory, at `far` + base, P's then
+    // D's `entries` per CTA
+    const ResFar* where;
+    unsigned char* far;
+};
+
+template <class T, int NT, bool FAR>
+__global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
+    batch_resident(BatchView b, Iterates<T> it, BatchParams p, ResJob job, long long iter0, long long n_periods,
+                   long long tail) {
+    __shared__ T weights[kResWeights];
+    __shared__ union {
+        ResBuild build;
+        double sum[2][kBlock];
+    } scratch;
+    __shared__ double red[K][NT / 32];
+    __shared__ double part[kResMaxCluster][K];  // rank 0: the CTAs' values
+    __shared__ int stop_all;
+    const ResCluster cl;
+    const int k = job.list[blockIdx.x / static_cast<unsigned>(cl.size)];
+    InstState& s = b.is[k];
+    if (s.done) return;  // the same for the cluster's CTAs, which alone run this instance
+    const int c0 = b.col_off[k], r0 = b.row_off[k];
+    const int n = b.col_off[k + 1] - c0, m = b.row_off[k + 1] - r0;
+    const ResParts &pt = job.parts[2 * k], &pa = job.parts[2 * k + 1];
+    const int per = kResMaxCluster / cl.size, p0 = cl.rank * per, p1 = p0 + per;
+    ResLp<T, FAR> L;
+    uint32_t at = L.place(n, m);
+    at = L.P.place(at, pt.row[p1] - pt.row[p0], pt.nz[p1] - pt.nz[p0], pt.longest, job.lgt, true);
+    L.D.place(at, pa.row[p1] - pa.row[p0], pa.nz[p1] - pa.nz[p0], pa.longest, job.lga, it.halpern != 0);
+    if constexpr (FAR) {
+        const ResFar w = job.where[blockIdx.x / static_cast<unsigned>(cl.size)];
+        unsigned char* mine = job.far + w.base +
+                              static_cast<int64_t>(kResFarEntry) * (w.entries[0] + w.entries[1]) * cl.rank;
+        L.P.e.place_far(mine, w.entries[0]);
+        L.D.e.place_far(mine + static_cast<int64_t>(kResFarEntry) * w.entries[0], w.entries[1]);
+    }
+    res_load_rows<NT>(L.P, b.AT, c0, r0, pt.row[p0], pt.row[p1], static_cast<uint32_t>(m), scratch.build);
+    res_load_rows<NT>(L.D, b.A, r0, c0, pa.row[p0], pa.row[p1], static_cast<uint32_t>(n), scratch.build);
+    const PV<T> pv = pvec<T>(b.P);
+    res_load_fixed<NT>(L, pv, c0, r0);
+    const bool lead = cl.rank == 0 && threadIdx.x == 0;
+    const double sign = s.obj_sign;
+    bool done = false;
+    long long periods = 0;
+    // whole check periods, then the tail: one body, so that the slabs stay in
+    // registers (as a function of its own it reads them from local memory:
+    // FP64 500 x 1,200 instances 4.8 -> 8.5 us an iteration)
+    for (bool checked = n_periods > 0; !done; checked = periods < n_periods) {
+        const long long count = checked ? p.period : tail;
+        // read ahead of the period, so that nobody waits for the host's memory
+        int stop = lead && b.mail != nullptr ? b.mail->stop_request : 0;
+        if (!checked) {
+            if (lead)
+                for (int c = 0; c < cl.size; ++c) *cg::this_cluster().map_shared_rank(&stop_all, c) = stop;
+            cl.sync();
+            if (count == 0 || stop_all != 0) break;
+        }
+        res_load_iterates<NT>(L, it, c0, r0);
+        ResStep<T> step;
+        step.tau = static_cast<T>(s.tau);
+        step.sigma = static_cast<T>(s.sigma);
+        const long long since = s.since_restart;
+        const bool fresh = s.fresh != 0;
+        cl.sync();  // every CTA has its copies before a neighbour writes into them
+        if (it.halpern) res_iterate<NT, T, true>(L, cl, step, it, since, count, fresh, weights);
+        else res_iterate<NT, T, false>(L, cl, step, it, since, count, fresh, weights);
+        res_store_iterates<NT>(L, it, c0, r0);
+        cl.sync();  // the stored vectors, seen by the whole cluster
+        if (!checked) break;
+        const long long iter = iter0 + periods * p.period;
+        ++periods;
+        // ---- check
+        const double inv = it.halpern ? 1.0 : 1.0 / static_cast<double>(s.since_restart + p.period);
+        Terms t;
+        if (it.halpern) {
+            check_rows<NT, T, false, true, FAR>(b, it, p, L.D, r0, inv, sign, t);
+            check_rows<NT, T, true, true, FAR>(b, it, p, L.P, c0, inv, sign, t);
+        } else {
+            check_rows<NT, T, false, false, FAR>(b, it, p, L.D, r0, inv, sign, t);
+            check_rows<NT, T, true, false, FAR>(b, it, p, L.P, c0, inv, sign, t);
+        }
+        __syncwarp();
+        const double v[K] = {t.cp,     t.cd,     t.ap,     t.ad,     t.ocp, t.ocd, t.oap, t.oad,
+                             t.pobj_c, t.dobj_c, t.pobj_a, t.dobj_a, t.ppc, t.ddc, t.ppa, t.dda};
+        const double mine = reduce_vals<NT>(v, red);
+        if (threadIdx.x < K) *cg::this_cluster().map_shared_rank(&part[cl.rank][threadIdx.x], 0) = mine;
+        cl.sync();
+        if (lead) {  // merged in rank order
+            double w[K];
+            for (int q = 0; q < K; ++q) {
+                w[q] = part[0][q];
+                for (int c = 1; c < cl.size; ++c) w[q] = q < 8 ? smax(w[q], part[c][q]) : w[q] + part[c][q];
+            }
+            batch_decide(b, p, s, w, it.halpern != 0, std::is_same<T, float>::value, iter, stop);
+        }
+        cl.sync();
+        // ---- restart
+        const int restart = s.restart, fold = s.fold;
+        done = s.done != 0;
+        if (restart || fold) {
+            const bool to_avg = s.restart_to_avg != 0;
+            const double ri = s.inv;
+            if (restart && p.primal_weight_update) {
+                // the weight's sums in batch_restart's order, whatever the
+                // cluster: the iterates that follow are its bits
+                if (cl.rank == 0) {
+                    double dx2 = 0.0, dy2 = 0.0;
+                    if (NT == kBlock || threadIdx.x < kBlock)
+                        for (int j = c0 + static_cast<int>(threadIdx.x); j < c0 + n; j += kBlock) {
+                            const double d = restart_move_col<T>(it, p, pv, j, to_avg, ri);
+                            dx2 += d * d;
+                        }
+                    if (NT == kBlock || (threadIdx.x >= kBlock && threadIdx.x < 2 * kBlock))
+                        for (int i = r0 + static_cast<int>(threadIdx.x % kBlock); i < r0 + m; i += kBlock) {
+                            const double d = restart_move_row<T>(it, p, i, to_avg, ri);
+                            dy2 += d * d;
+                        }
+                    // block_sum_det's tree, x's and y's sums side by side
+                    double(*sum)[kBlock] = scratch.sum;
+                    const int t = static_cast<int>(threadIdx.x);
+                    if (NT == kBlock) {
+                        sum[0][t] = dx2;
+                        sum[1][t] = dy2;
+                    } else if (t < 2 * kBlock) {
+                        sum[t / kBlock][t % kBlock] = t < kBlock ? dx2 : dy2;
+                    }
+                    __syncthreads();
+                    for (int o = kBlock / 2; o > 0; o >>= 1) {
+                        if (t < 2 * o) sum[t / o][t % o] += sum[t / o][t % o + o];
+                        __syncthreads();
+                    }
+                    if (lead) restart_weight(s, sum[0][0], sum[1][0]);
+                }
+                cl.sync();  // read before it changes
+            }
+            for (int j = c0 + L.P.r0 + static_cast<int>(threadIdx.x); j < c0 + L.P.r1; j += NT)
+                restart_col<T>(it, p, pv, j, restart, to_avg, ri);
+            for (int i = r0 + L.D.r0 + static_cast<int>(threadIdx.x); i < r0 + L.D.r1; i += NT)
+                restart_row<T>(it, p, pv, i, restart, to_avg, ri);
+        }
+        cl.sync();  // every CTA has read the flags
+        if (lead) {
+            s.restart = 0;
+            s.fold = 0;
+        }
+        cl.sync();
+    }
+    if (lead) {
+        // as the period count of the kernels over all instances: the period in
+        // which the last instance ends is not counted
+        atomicMax(&b.g->iter, iter0 + (periods - (done ? 1 : 0)) * p.period);
+        atomicMax(&b.g->checks, periods);
+    }
+}
+
+template <class T>
+cudaError_t launch_class(const ResClass& c, const BatchView& b, const Iterates<T>& it, const BatchParams& p,
+                         const ResJob& job, long long iter0, long long n_periods, long long tail, cudaStream_t s) {
+    auto run = [&](auto kernel) {
+        return res_launch(kernel, c.count, c.size, c.threads, c.smem, s, b, it, p, job, iter0, n_periods, tail);
+    };
+    if (c.far) return run(batch_resident<T, 1024, true>);
+    if (c.threads == 256) return run(batch_resident<T, 256, false>);
+    if (c.threads == 512) return run(batch_resident<T, 512, false>);
+    return run(batch_resident<T, 1024, false>);
+}
+
+// The largest cluster the device schedules at the largest shared memory.
+int g_res_cluster = 0;
+
+}  // namespace
+
+int init_resident_kernels() {
+    const int c[8] = {res_largest_cluster(batch_resident<float, 1024, false>, 1024),
+                      res_largest_cluster(batch_resident<double, 1024, false>, 1024),
+                      res_largest_cluster(batch_resident<float, 1024, true>, 1024),
+                      res_largest_cluster(batch_resident<double, 1024, true>, 1024),
+                      res_largest_cluster(batch_resident<float, 512, false>, 512),
+                      res_largest_cluster(batch_resident<double, 512, false>, 512),
+                      res_largest_cluster(batch_resident<float, 256, false>, 256),
+                      res_largest_cluster(batch_resident<double, 256, false>, 256)};
+    if (*std::min_element(c, c + 8) == 0) return 1;
+    g_res_cluster = *std::min_element(c, c + 4);
+    return 0;
+}
+
+void launch_batch_parts(const BatchView& b, ResParts* parts, cudaStream_t s) {
+    if (b.count == 0) return;
+    k_batch_parts<<<b.count, kBlock, 0, s>>>(b.AT.rp, b.col_off, 0, parts);
+    k_batch_parts<<<b.count, kBlock, 0, s>>>(b.A.rp, b.row_off, 1, parts);
+}
+
+// Classes of like CTAs, tried in the order of their CTAs; the largest instances
+// first (a class's launch ends with its last instance).
+constexpr ResClass kClasses[kResClasses] = {
+    {1, 256}, {1, 512}, {1, 1024}, {1, 1024, 0, 0, 0, true}, {2, 1024}, {2, 1024, 0, 0, 0, true},
+    {4, 1024}, {4, 1024, 0, 0, 0, true}, {8, 1024}, {8, 1024, 0, 0, 0, true}, {16, 1024, 0, 0, 0, true}};
+// ... of an instance of nnz entries. `packed`: the batch has more instances
+// than fill the GPU, so what counts is SM time: the fewest CTAs that hold the
+// instance at up to kResPacked entries each, its entries in global memory where
+// they do not fit. Otherwise each instance's own time counts: the CTAs that
+// hold its entries, at most eight (60 KB to all CTAs of a cluster: 3,500 cycles
+// for eight, 4,600 for sixteen). 256 FP32 instances of 50 x 100 to 5,000 x
+// 15,000, a check period of 40 iterations: 1,483 us at their own time's
+// clusters; packed with 8,192 / 16,384 / 32,768 / 65,536 entries a CTA 1,483 /
+// 1,244 / 1,184 / 1,218 us.
+constexpr int64_t kResPacked = 32768;
+template <class T>
+int res_class(const ResParts& pt, const ResParts& pa, int lgt, int lga, bool halpern, bool packed, ResSize* z) {
+    const int32_t nnz = pa.nz[kResMaxCluster];
+    int last = -1;
+    for (int c = 2; c < kResClasses; ++c) {
+        const ResClass& k = kClasses[c];
+        if (k.size > g_res_cluster) continue;
+        const ResSize y = k.far ? res_size<T, true>(pt, pa, k.size, lgt, lga, halpern)
+                                : res_size<T, false>(pt, pa, k.size, lgt, lga, halpern);
+        if (y.smem > kResMaxSmem) continue;
+        if (!packed && k.far && k.size < 8) continue;
+        last = c;
+        *z = y;
+        if (!packed || k.size >= 8 || nnz <= kResPacked * k.size) break;
+    }
+    if (last == 2 && nnz <= 3000 && z->smem <= kResMaxSmem / 4) return 0;   // four to an SM
+    if (last == 2 && nnz <= 12000 && z->smem <= kResMaxSmem / 2) return 1;  // two
+    return last;
+}
+
+template <class T>
+bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, int sms, ResPlan& plan) {
+    plan = ResPlan{};
+    const size_t count = parts.size() / 2;
+    if (g_res_cluster == 0) return false;
+    struct Item {
+        int32_t k, nnz, cls;
+        ResFar far;
+    };
+    std::vector<Item> items(count);
+    ResClass all[kResClasses];
+    bool packed = false;
+    for (int pass = 0; pass < 2; ++pass) {
+        std::copy(kClasses, kClasses + kResClasses, all);
+        plan.far_bytes = 0;
+        int64_t quarters = 0;  // of SMs that all instances at once would fill
+        for (size_t k = 0; k < count; ++k) {
+            const ResParts &pt = parts[2 * k], &pa = parts[2 * k + 1];
+            ResSize z;
+            const int cls = res_class<T>(pt, pa, lgt, lga, halpern, packed, &z);
+            if (cls < 0) return false;
+            items[k] = {static_cast<int32_t>(k), pa.nz[kResMaxCluster], cls, ResFar{}};
+            if (all[cls].far) {
+                // whole 16-byte vectors per CTA
+                for (int w = 0; w < 2; ++w) items[k].far.entries[w] = (z.entries[w] + 7u) / 8u * 8u;
+                items[k].far.base = plan.far_bytes;
+                plan.far_bytes += static_cast<int64_t>(kResFarEntry) *
+                                  (items[k].far.entries[0] + items[k].far.entries[1]) * all[cls].size;
+                plan.far_bytes = (plan.far_bytes + 255) / 256 * 256;
+            }
+            all[cls].count += 1;
+            all[cls].smem = std::max(all[cls].smem, z.smem);
+            quarters += cls == 0 ? 1 : cls == 1 ? 2 : 4 * all[cls].size;
+        }
+        if (packed || quarters <= 4 * static_cast<int64_t>(sms)) break;
+        packed = true;
+    }
+    std::sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
+        return a.cls != b.cls ? a.cls > b.cls : a.nnz != b.nnz ? a.nnz > b.nnz : a.k < b.k;
+    });
+    for (const Item& i : items) {
+        plan.list.push_back(i.k);
+        plan.where.push_back(i.far);
+    }
+    int32_t first = 0;
+    for (int c = kResClasses - 1; c >= 0; --c) {
+        if (all[c].count == 0) continue;
+        all[c].first = first;
+        first += all[c].count;
+        plan.classes.push_back(all[c]);
+    }
+    return true;
+}
+
+template <class T>
+cudaError_t launch_batch_resident(const std::vector<ResClass>& classes, const ResBuffers& buf, int lgt, int lga,
+                                  const BatchView& b, const Iterates<T>& it, const BatchParams& p, long long iter0,
+                                  long long n_periods, long long tail, cudaStream_t s, const ResStreams& side) {
+    cudaError_t e = cudaEventRecord(side.fork, s);
+    for (size_t c = 0; c < classes.size() && e == cudaSuccess; ++c) {
+        const cudaStream_t to = c == 0 ? s : side.stream[c - 1];
+        if (c > 0) e = cudaStreamWaitEvent(to, side.fork, 0);
+        if (e == cudaSuccess)
+            e = launch_class<T>(classes[c], b, it, p, ResJob{buf.list + classes[c].first, buf.parts, lgt, lga,
+                                       buf.where + classes[c].first, buf.far}, iter0, n_periods, tail,
+                                to);
+        if (c > 0 && e == cudaSuccess) e = cudaEventRecord(side.join[c - 1], to);
+        if (c > 0 && e == cudaSuccess) e = cudaStreamWaitEvent(s, side.join[c - 1], 0);
+    }
+    return e;
+}
+
+template bool plan_resident<float>(const std::vector<ResParts>&, int, int, bool, int, ResPlan&);
+template bool plan_resident<double>(const std::vector<ResParts>&, int, int, bool, int, ResPlan&);
+template cudaError_t launch_batch_resident<float>(const std::vector<ResClass>&, const ResBuffers&, int, int,
+                                                  const BatchView&, const Iterates<float>&, const BatchParams&,
+                                                  long long, long long, long long, cudaStream_t, const ResStreams&);
+template cudaError_t launch_batch_resident<double>(const std::vector<ResClass>&, const ResBuffers&, int, int,
+                                                   const BatchView&, const Iterates<double>&, const BatchParams&,
+                                                   long long, long long, long long, cudaStream_t, const ResStreams&);
+
+}  // namespace pdhg

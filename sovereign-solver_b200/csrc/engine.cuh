@@ -525,6 +525,8 @@ void launch_norms(int32_t m, int32_t n, const double* c_s, const double* rlo_s,
 // Inclusive prefix sum of n int32 counts into out[1..n], out[0] = 0 (CUB).
 int prefix_rows(const int32_t* cnt, int32_t n, int32_t* out, cudaStream_t s);
 
+int init_resident_kernels();  // batch_resident.cu: once per device; 0 on success
+
 // The batched engine (batch.cu), owned by a context: it uses the context's
 // stream and writes its errors into the context's error text.
 struct BatchCtx;
