@@ -5,10 +5,10 @@
 //
 // One GEMM form covers every product: C[M x N] = A[M x K] * B[N x K]^T with
 // both operands K-contiguous (row-major A and B), fused epilogue (bias, ReLU,
-// a ReLU-derivative mask, FP32 and/or BF16 outputs). Products that need a
-// transposed operand (the weight gradients dY^T H, the input gradients dY W)
-// take a transposed copy made by k_transpose (the matrices are at most
-// hidden x batch).
+// a ReLU-derivative mask or the loss's derivative; FP32, BF16 and transposed
+// BF16 outputs). The weight gradients dY^T H take their operands from the
+// transposed outputs of the GEMMs that made them, the input gradients dY W the
+// weights' transposed copies (k_transpose, when the weights change).
 //
 // Forward (batch B):  H1 = relu(X W1^T + b1), H2 = relu(H1 W2^T + b2),
 //                     Y = H2 W3^T + b3.
@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/pdhg_b200.h"
+#include "pass.cuh"
 #include "tcgen05.cuh"
 
 namespace pdhg {
@@ -35,9 +36,10 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int kGemmThreads = 128;
-constexpr int kGemmBN = 128;                 // N per CTA (TMEM columns)
+constexpr int kGemmThreads = kBlock;
 constexpr long long kSpinLimit = 1LL << 24;  // bounded mbarrier waits
+
+constexpr int kGemmSms = 148;
 
 struct GemmArgs {
     int M, N, K;
@@ -49,12 +51,26 @@ struct GemmArgs {
     int relu;
     const bf16* mask;   // M x N: output * [mask > 0], or null
     int ldm;
+    // The output is the loss's derivative 2 (v - target) scale at v = the
+    // product, or null; row r's target is row idx[r] (idx null: r) of N. Each
+    // CTA's share of the loss (v - target)^2 scale to part[its tile].
+    const float* target;
+    const int32_t* idx;
+    float scale;
+    double* part;
     float* out32;       // M x N, or null
     int ld32;
     bf16* out16;        // M x N, or null
     int ld16;
+    bf16* out16t;       // N x M: the transposed output, or null
+    int ldt;
     int* err;           // set when a bounded wait gives up
-    int vec;            // 1: every row of bias / mask / outputs starts 16-byte aligned
+    int vec;            // 1: every row of bias / mask / target / outputs starts 16-byte aligned
+};
+// One launch over the tiles of up to two products, the second's after tiles0.
+struct GemmPair {
+    GemmArgs g[2];
+    int tiles0;
 };
 
 // 16-byte asynchronous global -> shared copy (cp.async, no register staging);
@@ -64,95 +80,127 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src
                  "l"(gmem), "r"(src_bytes)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
-// C = A B^T on one 128 x kGemmBN tile: the K loop stages a 128 x 64 slice of
-// A and a kGemmBN x 64 slice of B in shared memory (core-matrix layout, see
-// tcgen05.cuh) with asynchronous 16-byte copies, all of a slice in flight at
-// once, one thread issues the four 16-deep MMAs into the TMEM accumulator and
-// commits them to an mbarrier that every thread waits on before the slices
-// are overwritten. The epilogue reads the accumulator with tcgen05.ld, one
-// TMEM lane (= output row) per thread.
-__global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(GemmArgs g) {
-    __shared__ __align__(1024) bf16 sA[tc::kTileM * tc::kTileK];
-    __shared__ __align__(1024) bf16 sB[kGemmBN * tc::kTileK];
-    __shared__ __align__(8) uint64_t bar;
+// Rows [r0, r0 + ROWS) x K-elements [k0, k0 + 64) of a matrix of `rows` x K
+// into a staged tile, zeros outside.
+template <int ROWS>
+__device__ __forceinline__ void stage_rows(bf16* dst, const bf16* src, int ld, int r0, int rows, int k0, int K) {
+#pragma unroll
+    for (int c = threadIdx.x; c < ROWS * (tc::kTileK / 8); c += kGemmThreads) {
+        const int row = c >> 3, kc = (c & 7) * 8;
+        const int gr = r0 + row, gk = k0 + kc;
+        const bool in = gr < rows && gk < K;
+        cp_async16(dst + tc::tile_offset(row, kc), in ? src + static_cast<size_t>(gr) * ld + gk : src, in ? 16 : 0);
+    }
+}
+
+// C = A B^T on one 128 x BN tile: the K loop keeps STAGES slices of A (128 x
+// 64) and B (BN x 64) in shared memory (core-matrix layout, see tcgen05.cuh)
+// or on their way there in 16-byte asynchronous copies; one thread issues each
+// slice's four 16-deep MMAs into the TMEM accumulator and commits them to the
+// slice's mbarrier, which is waited on before the slice is overwritten. The
+// epilogue reads the accumulator with tcgen05.ld, one TMEM lane (= output row)
+// per thread, 32 columns at a time; the second four warps take every other 32.
+//
+// Bound: the latency of one CTA's chain (slice, MMAs, epilogue); a product of
+// the network (256 x 512 x 512) is 0.1 us of the tensor cores. So all of its
+// slices are in flight at once, and the tiles are as narrow as keeps the grid
+// within the SMs (gemm). One slice at a time on 128-column tiles, with the
+// transposes, the loss and the column sums in launches of their own, the
+// gradients of 256 rows through 64 -> 512 -> 512 -> 512 took 536 us with their
+// copies, 25 launches; 294 us in 8, as programmatic dependents, the same bits.
+template <int BN, int STAGES>
+__global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(const __grid_constant__ GemmPair pair) {
+    extern __shared__ __align__(1024) unsigned char dyn[];
+    __shared__ __align__(8) uint64_t bar[STAGES];
     __shared__ uint32_t tmem_base;
+    __shared__ double loss_part[kGemmThreads / 32];
+    constexpr int kA = tc::kTileM * tc::kTileK, kB = BN * tc::kTileK;
+    bf16* const slices = reinterpret_cast<bf16*>(dyn);  // A's and B's of stage 0, of stage 1, ...
+    pass_begin();
+    const bool second = static_cast<int>(blockIdx.x) >= pair.tiles0;
+    const GemmArgs& g = pair.g[second ? 1 : 0];
+    const int tile = static_cast<int>(blockIdx.x) - (second ? pair.tiles0 : 0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * tc::kTileM, n0 = blockIdx.y * kGemmBN;
+    const int tiles_m = (g.M + tc::kTileM - 1) / tc::kTileM;
+    const int m0 = tile % tiles_m * tc::kTileM, n0 = tile / tiles_m * BN;
+    const int rounds = (g.K + tc::kTileK - 1) / tc::kTileK;
     if (warp == 0) {
-        tc::tmem_alloc(&tmem_base, kGemmBN);
+        tc::tmem_alloc(&tmem_base, BN);
         tc::tmem_relinquish();
     }
     if (tid == 0) {
-        tc::mbar_init(&bar, 1);
+        for (int i = 0; i < STAGES; ++i) tc::mbar_init(&bar[i], 1);
         tc::fence_mbar_init();
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const uint32_t idesc = tc::instr_desc_bf16(kGemmBN);
-    const uint32_t a_base = tc::smem_u32(sA), b_base = tc::smem_u32(sB);
-    int round = 0;
-    bool aborted = false;
-    for (int k0 = 0; k0 < g.K; k0 += tc::kTileK, ++round) {
-#pragma unroll
-        for (int c = tid; c < tc::kTileM * (tc::kTileK / 8); c += kGemmThreads) {
-            const int row = c >> 3, kc = (c & 7) * 8;
-            const int gr = m0 + row, gk = k0 + kc;
-            const bool in = gr < g.M && gk < g.K;
-            cp_async16(sA + tc::tile_offset(row, kc),
-                       in ? g.A + static_cast<size_t>(gr) * g.lda + gk : g.A, in ? 16 : 0);
+    constexpr uint32_t idesc = tc::instr_desc_bf16(BN);
+    const uint32_t base = tc::smem_u32(slices);
+    auto stage = [&](int r) {
+        if (r < rounds) {
+            bf16* at = slices + (r % STAGES) * (kA + kB);
+            stage_rows<tc::kTileM>(at, g.A, g.lda, m0, g.M, r * tc::kTileK, g.K);
+            stage_rows<BN>(at + kA, g.B, g.ldb, n0, g.N, r * tc::kTileK, g.K);
         }
-#pragma unroll
-        for (int c = tid; c < kGemmBN * (tc::kTileK / 8); c += kGemmThreads) {
-            const int row = c >> 3, kc = (c & 7) * 8;
-            const int gr = n0 + row, gk = k0 + kc;
-            const bool in = gr < g.N && gk < g.K;
-            cp_async16(sB + tc::tile_offset(row, kc),
-                       in ? g.B + static_cast<size_t>(gr) * g.ldb + gk : g.B, in ? 16 : 0);
-        }
-        cp_async_wait_all();
-        tc::fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fence_after_sync();
-#pragma unroll
-            for (int s = 0; s < tc::kTileK / 16; ++s) {
-                const uint64_t ad = tc::smem_desc(a_base + s * 2 * tc::kChunkBytes);
-                const uint64_t bd = tc::smem_desc(b_base + s * 2 * tc::kChunkBytes);
-                tc::mma_bf16(tmem, ad, bd, idesc, (k0 > 0 || s > 0) ? 1u : 0u);
-            }
-            tc::mma_commit(&bar);
-        }
+        cp_async_commit();
+    };
+    auto wait = [&](int r) {  // for round r's MMAs, bounded; the same answer for the CTA
         long long spins = 0;
         bool timed_out = false;
-        while (!tc::mbar_try_wait(&bar, static_cast<uint32_t>(round & 1))) {
+        while (!tc::mbar_try_wait(&bar[r % STAGES], static_cast<uint32_t>((r / STAGES) & 1)))
             if (++spins > kSpinLimit) {
                 timed_out = true;
                 break;
             }
+        return __syncthreads_or(timed_out) == 0;
+    };
+    pass_wait();  // the operands are the kernel before's
+    for (int r = 0; r < STAGES - 1; ++r) stage(r);
+    bool ok = true;
+    int issued = 0;
+    for (int r = 0; r < rounds; ++r) {
+        const int next = r + STAGES - 1;
+        if (next >= STAGES && next < rounds) ok = wait(next - STAGES);
+        if (!ok) break;
+        stage(next);
+        cp_async_wait<STAGES - 1>();  // round r's copies have landed
+        tc::fence_proxy_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc::fence_after_sync();
+            const uint32_t a = base + static_cast<uint32_t>(r % STAGES) * 2u * (kA + kB), b = a + 2u * kA;
+#pragma unroll
+            for (int s = 0; s < tc::kTileK / 16; ++s)
+                tc::mma_bf16(tmem, tc::smem_desc(a + s * 2 * tc::kChunkBytes),
+                             tc::smem_desc(b + s * 2 * tc::kChunkBytes), idesc, (r > 0 || s > 0) ? 1u : 0u);
+            tc::mma_commit(&bar[r % STAGES]);
         }
-        if (__syncthreads_or(timed_out)) {
-            aborted = true;
-            break;
-        }
+        ++issued;
     }
+    if (ok) ok = wait(rounds - 1);  // the commits arrive in order
     tc::fence_after_sync();
-    if (aborted) {
-        if (tid == 0) atomicExch(g.err, 1);
-        // give the MMAs in flight one more bounded chance to finish
-        long long spins = 0;
-        while (!tc::mbar_try_wait(&bar, static_cast<uint32_t>(round & 1)) && ++spins < kSpinLimit) {
-        }
+    double loss = 0.0;
+    if (!ok) {
+        if (tid == 0) *reinterpret_cast<volatile int*>(g.err) = 1;
+        cp_async_wait<0>();
+        if (issued > 0) wait(issued - 1);  // one more bounded chance for the MMAs in flight
     } else {
-        const int row = m0 + warp * 32 + lane;
-        for (int cb = 0; cb < kGemmBN; cb += 32) {
+        const int row = m0 + (warp & 3) * 32 + lane;
+        for (int cb = (warp >> 2) * 32; cb < BN; cb += kGemmThreads / 128 * 32) {
             float v[32];
-            tc::tmem_load32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + cb, v);
+            tc::tmem_load32(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + cb, v);
             if (row >= g.M) continue;
             const int c0 = n0 + cb;
+            const float* trow = nullptr;
+            if (g.target != nullptr) trow = g.target + static_cast<size_t>(g.idx != nullptr ? g.idx[row] : row) * g.N;
             if (g.vec && c0 + 32 <= g.N) {
                 // a thread's 32 columns are contiguous in its row: 16-byte
                 // loads of bias and mask, all issued before they are used,
@@ -161,7 +209,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(GemmArgs g) {
                     const float4* b4 = reinterpret_cast<const float4*>(g.bias + c0);
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        const float4 b = __ldg(b4 + q);
+                        const float4 b = b4[q];
                         v[4 * q] += b.x;
                         v[4 * q + 1] += b.y;
                         v[4 * q + 2] += b.z;
@@ -175,13 +223,27 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(GemmArgs g) {
                     const uint4* m4 = reinterpret_cast<const uint4*>(g.mask + static_cast<size_t>(row) * g.ldm + c0);
                     uint4 mk[4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) mk[q] = __ldg(m4 + q);
+                    for (int q = 0; q < 4; ++q) mk[q] = m4[q];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const bf16* mb = reinterpret_cast<const bf16*>(&mk[q]);
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
                             if (!(__bfloat162float(mb[j]) > 0.f)) v[8 * q + j] = 0.f;
+                    }
+                }
+                if (trow != nullptr) {
+                    const float4* t4 = reinterpret_cast<const float4*>(trow + c0);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 t = t4[q];
+                        const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const float d = v[4 * q + u] - tv[u];
+                            v[4 * q + u] = 2.f * d * g.scale;
+                            loss += static_cast<double>(d) * d * g.scale;
+                        }
                     }
                 }
                 if (g.out32 != nullptr) {
@@ -201,6 +263,10 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(GemmArgs g) {
                         o4[q] = w;
                     }
                 }
+                if (g.out16t != nullptr)  // a warp's 32 rows of a column are 64 contiguous bytes
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        g.out16t[static_cast<size_t>(c0 + j) * g.ldt + row] = __float2bfloat16_rn(v[j]);
                 continue;
             }
 #pragma unroll
@@ -213,15 +279,32 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(GemmArgs g) {
                 if (g.mask != nullptr &&
                     !(__bfloat162float(g.mask[static_cast<size_t>(row) * g.ldm + col]) > 0.f))
                     x = 0.f;
+                if (trow != nullptr) {
+                    const float d = x - trow[col];
+                    x = 2.f * d * g.scale;
+                    loss += static_cast<double>(d) * d * g.scale;
+                }
                 if (g.out32 != nullptr) g.out32[static_cast<size_t>(row) * g.ld32 + col] = x;
                 if (g.out16 != nullptr)
                     g.out16[static_cast<size_t>(row) * g.ld16 + col] = __float2bfloat16_rn(x);
+                if (g.out16t != nullptr)
+                    g.out16t[static_cast<size_t>(col) * g.ldt + row] = __float2bfloat16_rn(x);
             }
         }
     }
+    if (g.target != nullptr) {  // the same for the CTA
+        __syncwarp();
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if (lane == 0) loss_part[warp] = loss;
+    }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, kGemmBN);
+    if (g.target != nullptr && tid == 0) {
+        double s = 0.0;
+        for (int w = 0; w < kGemmThreads / 32; ++w) s += loss_part[w];
+        g.part[tile] = s;
+    }
+    if (warp == 0) tc::tmem_dealloc(tmem, BN);
 }
 
 // out[c * ldo + r] = in[r * ldi + c] for an R x C BF16 matrix (32 x 32 tiles).
@@ -244,53 +327,75 @@ __global__ void k_to_bf16(const float* in, bf16* out, int64_t n) {
     if (t < n) out[t] = __float2bfloat16_rn(in[t]);
 }
 
-// Rows idx[0..B) of src (S x d, FP32) -> dst32 / dst16 (B x d).
-__global__ void k_gather_rows(const float* src, int d, const int32_t* idx, int B, float* dst32,
-                              bf16* dst16) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (t >= static_cast<int64_t>(B) * d) return;
-    const int b = static_cast<int>(t / d), j = static_cast<int>(t % d);
-    const float v = src[static_cast<int64_t>(idx[b]) * d + j];
-    if (dst32 != nullptr) dst32[t] = v;
-    if (dst16 != nullptr) dst16[t] = __float2bfloat16_rn(v);
+// Rows idx[0..B) (idx null: 0..B) of src (S x d, FP32) in BF16: dst (B x d)
+// and, unless null, its transposed copy (d x B). 32 x 32 tiles.
+__global__ void k_gather_rows(const float* src, int d, const int32_t* idx, int B, bf16* dst, bf16* dst_t) {
+    __shared__ bf16 t[32][33];
+    pass_begin();
+    pass_wait();
+    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+    const int c = c0 + threadIdx.x;
+    for (int i = threadIdx.y; i < 32; i += 8) {
+        const int r = r0 + i;
+        if (r >= B || c >= d) continue;
+        const bf16 v = __float2bfloat16_rn(src[static_cast<int64_t>(idx != nullptr ? idx[r] : r) * d + c]);
+        dst[static_cast<size_t>(r) * d + c] = v;
+        t[i][threadIdx.x] = v;
+    }
+    if (dst_t == nullptr) return;
+    __syncthreads();
+    const int r = r0 + threadIdx.x;
+    for (int i = threadIdx.y; i < 32; i += 8)
+        if (r < B && c0 + i < d) dst_t[static_cast<size_t>(c0 + i) * B + r] = t[threadIdx.x][i];
 }
 
-// dY = 2 (Y - T) / (B n), FP32 and BF16; per-block partial losses.
-__global__ void k_loss_grad(const float* Y, const float* T, int64_t count, float scale,
-                            float* dY32, bf16* dY16, double* part) {
-    __shared__ double sh[256];
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    double l = 0.0;
-    if (t < count) {
-        const float d = Y[t] - T[t];
-        const float gv = 2.f * d * scale;
-        dY32[t] = gv;
-        dY16[t] = __float2bfloat16_rn(gv);
-        l = static_cast<double>(d) * d * scale;
+// db[j] = sum_b dZ[b, j] for up to three dZ (B x N), and the loss from its
+// parts, in one launch: CTA c takes 32 columns of one matrix, staged 256 rows
+// at a time so that the loads are all in flight; each column is then one
+// thread's sum in row order. The last CTA adds the loss's parts in order.
+// (One thread per column, each row's load waiting for the one before: 20 us
+// for 256 rows; staged 3 us.)
+struct ColSums {
+    const float* dz[3];
+    float* db[3];
+    int N[3], first[4];  // first[i]: matrix i's first CTA; first[3]: the loss's
+    int B;
+    const double* part;
+    int n_part;
+    double* loss;
+};
+constexpr int kColRows = 256;
+__global__ void __launch_bounds__(256) k_colsums(const __grid_constant__ ColSums a) {
+    __shared__ float st[kColRows][33];
+    pass_begin();
+    pass_wait();
+    const int b = static_cast<int>(blockIdx.x), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (b == a.first[3]) {
+        if (warp != 0) return;
+        double s = 0.0;
+        for (int i = 0; i < a.n_part; i += 32) {
+            const double v = i + lane < a.n_part ? a.part[i + lane] : 0.0;
+            for (int q = 0; q < 32; ++q) s += __shfl_sync(0xffffffffu, v, q);
+        }
+        if (lane == 0) *a.loss = s;
+        return;
     }
-    sh[threadIdx.x] = l;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+    const int k = b >= a.first[2] ? 2 : b >= a.first[1] ? 1 : 0;
+    const int N = a.N[k], j = (b - a.first[k]) * 32 + lane;
+    const float* __restrict__ dz = a.dz[k];
+    float s = 0.f;
+    for (int r0 = 0; r0 < a.B; r0 += kColRows) {
+        const int rows = min(kColRows, a.B - r0);
+#pragma unroll 8
+        for (int r = warp; r < rows; r += 8)
+            if (j < N) st[r][lane] = __ldcg(dz + static_cast<size_t>(r0 + r) * N + j);
+        __syncthreads();
+        if (warp == 0)
+#pragma unroll 16
+            for (int r = 0; r < rows; ++r) s += st[r][lane];
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-__global__ void k_sum_parts(const double* part, int n, double* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
-}
-
-// db[j] = sum_b dZ[b, j] (fixed order per column).
-__global__ void k_colsum(const float* dZ, int B, int N, float* db) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    float s = 0.f;
-    for (int b = 0; b < B; ++b) s += dZ[static_cast<size_t>(b) * N + j];
-    db[j] = s;
+    if (warp == 0 && j < N) a.db[k][j] = s;
 }
 
 // Adam (bias-corrected) on FP32 master weights; refreshes the BF16 copy.
@@ -310,24 +415,66 @@ __global__ void k_adam(float* w, const float* g, float* m, float* v, bf16* w16, 
 
 inline int blocks(int64_t n, int t) { return static_cast<int>((n + t - 1) / t); }
 
-// Host checks of the GEMM's layout contract, then the launch.
-int gemm(const GemmArgs& g, cudaStream_t s) {
-    if (g.M < 1 || g.N < 1 || g.K < 8 || g.K % 8 != 0 || g.lda % 8 != 0 || g.ldb % 8 != 0 ||
-        (reinterpret_cast<uintptr_t>(g.A) & 15u) || (reinterpret_cast<uintptr_t>(g.B) & 15u))
-        return PDHG_ERR_INVALID_ARGUMENT;
-    const dim3 grid((g.M + tc::kTileM - 1) / tc::kTileM, (g.N + kGemmBN - 1) / kGemmBN);
-    GemmArgs a = g;
-    auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    a.vec = al16(g.bias) && (g.mask == nullptr || (al16(g.mask) && g.ldm % 8 == 0)) &&
-            (g.out32 == nullptr || (al16(g.out32) && g.ld32 % 4 == 0)) &&
-            (g.out16 == nullptr || (al16(g.out16) && g.ld16 % 8 == 0)) ? 1 : 0;
-    k_gemm_tn<<<grid, kGemmThreads, 0, s>>>(a);
-    return cudaGetLastError() == cudaSuccess ? PDHG_OK : PDHG_ERR_BACKEND;
+template <int BN>
+constexpr int kStageBytes = 2 * (tc::kTileM + BN) * tc::kTileK;
+
+// Once per device (the caller's current one), before its first GEMM.
+cudaError_t init_gemm() {
+    constexpr auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_gemm_tn<32, 8>, smem, 8 * kStageBytes<32>);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tn<64, 8>, smem, 8 * kStageBytes<64>);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_tn<128, 6>, smem, 6 * kStageBytes<128>);
+    return e;
+}
+
+template <int BN, int STAGES>
+cudaError_t run_gemm(const GemmPair& p, int tiles, int rounds, bool early, cudaStream_t s) {
+    return launch_pass_smem(k_gemm_tn<BN, STAGES>, tiles, early, s, std::min(rounds, STAGES) * kStageBytes<BN>, p);
+}
+
+// Host checks of the GEMM's layout contract, then one launch of one or two
+// products (h null: one; early: see launch_pass). The tiles are 32 columns wide while that gives no more
+// CTAs than the GPU has SMs, then 64, then 128: a wider tile reads A less often,
+// a narrower one leaves fewer SMs idle (256 x 512 x 512: 8 CTAs of 128 columns,
+// 32 of 32).
+int gemm(const GemmArgs& g, const GemmArgs* h, bool early, cudaStream_t s) {
+    GemmPair p{};
+    int rounds = 0, tiles[3] = {};
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    for (int i = 0; i < (h != nullptr ? 2 : 1); ++i) {
+        GemmArgs& a = p.g[i] = i == 0 ? g : *h;
+        if (a.M < 1 || a.N < 1 || a.K < 8 || a.K % 8 != 0 || a.lda % 8 != 0 || a.ldb % 8 != 0 || !al16(a.A) ||
+            !al16(a.B))
+            return PDHG_ERR_INVALID_ARGUMENT;
+        a.vec = al16(a.bias) && (a.mask == nullptr || (al16(a.mask) && a.ldm % 8 == 0)) &&
+                (a.target == nullptr || (al16(a.target) && a.N % 4 == 0)) &&
+                (a.out32 == nullptr || (al16(a.out32) && a.ld32 % 4 == 0)) &&
+                (a.out16 == nullptr || (al16(a.out16) && a.ld16 % 8 == 0)) ? 1 : 0;
+        rounds = std::max(rounds, (a.K + tc::kTileK - 1) / tc::kTileK);
+        for (int w = 0; w < 3; ++w) {
+            const int t = ((a.M + tc::kTileM - 1) / tc::kTileM) * ((a.N + (32 << w) - 1) / (32 << w));
+            tiles[w] += t;
+        }
+    }
+    const int w = tiles[0] <= kGemmSms ? 0 : tiles[1] <= kGemmSms ? 1 : 2;
+    p.tiles0 = ((g.M + tc::kTileM - 1) / tc::kTileM) * ((g.N + (32 << w) - 1) / (32 << w));
+    const cudaError_t e = w == 0   ? run_gemm<32, 8>(p, tiles[0], rounds, early, s)
+                          : w == 1 ? run_gemm<64, 8>(p, tiles[1], rounds, early, s)
+                                   : run_gemm<128, 6>(p, tiles[2], rounds, early, s);
+    return e == cudaSuccess ? PDHG_OK : PDHG_ERR_BACKEND;
 }
 
 void transpose(const bf16* in, int ldi, bf16* out, int ldo, int R, int C, cudaStream_t s) {
     const dim3 grid((C + 31) / 32, (R + 31) / 32);
     k_transpose<<<grid, dim3(32, 8), 0, s>>>(in, ldi, out, ldo, R, C);
+}
+
+// CTAs of forward()'s last product (gemm's rule), each with its part of the loss.
+int loss_parts(int B, int n_out) {
+    const int tm = (B + tc::kTileM - 1) / tc::kTileM;
+    for (int w = 0; w < 2; ++w)
+        if (tm * blocks(n_out, 32 << w) <= kGemmSms) return tm * blocks(n_out, 32 << w);
+    return tm * blocks(n_out, 128);
 }
 
 template <class T>
@@ -361,16 +508,20 @@ struct Mlp {
     Dev<bf16> w16, w2t, w3t;  // BF16 weights, transposed W2 and W3 (for dX products)
     long long adam_t = 0;
     // activations (max_batch rows)
-    Dev<bf16> x16, xt, h1, h1t, h2, h2t, dy16, dyt, dz2_16, dz2t, dz1_16, dz1t;
-    Dev<float> t32, y32, dy32, dz2_32, dz1_32;
+    Dev<bf16> x16, xt, h1, h1t, h2, h2t, dy16, dyt, dz2_16, dz2t, dz1t;
+    Dev<float> x32, t32, y32, dy32, dz2_32, dz1_32;
     Dev<double> part;
-    Dev<int32_t> idx;
-    Dev<int> errflag;
+    // in pinned memory, written by the kernels
+    struct Status {
+        double loss;
+        int err;
+    }* status = nullptr;
     // training set on the device
     Dev<float> xs, ts;
 
     ~Mlp() {
         if (stream != nullptr) cudaStreamDestroy(stream);
+        if (status != nullptr) cudaFreeHost(status);
     }
     float* W(int i) { return w.p + off[2 * i]; }
     float* Bv(int i) { return w.p + off[2 * i + 1]; }
@@ -392,10 +543,8 @@ namespace {
     } while (0)
 
 int check_err(Mlp& h) {
-    int e = 0;
-    MCK(cudaMemcpyAsync(&e, h.errflag.p, sizeof e, cudaMemcpyDeviceToHost, h.stream));
     MCK(cudaStreamSynchronize(h.stream));
-    if (e != 0) {
+    if (h.status->err != 0) {
         h.err = "tensor-core GEMM: an MMA did not complete within its wait limit";
         return PDHG_ERR_BACKEND;
     }
@@ -422,96 +571,109 @@ void refresh_weights(Mlp& h) {
     transpose(h.W16(2), h.hidden, h.w3t.p, h.n_out, h.n_out, h.hidden, h.stream);
 }
 
-int forward(Mlp& h, int B) {
+// Y of the batch in x16, or, for a gradient (t: the targets, row r's at row
+// idx[r]), its loss's derivative and, transposed too, the layers' outputs.
+int forward(Mlp& h, int B, const float* t, const int32_t* idx) {
     int rc;
-    GemmArgs g = args(B, h.hidden, h.n_in, h.x16.p, h.n_in, h.W16(0), h.n_in, h.errflag.p);
+    GemmArgs g = args(B, h.hidden, h.n_in, h.x16.p, h.n_in, h.W16(0), h.n_in, &h.status->err);
     g.bias = h.Bv(0);
     g.relu = 1;
     g.out16 = h.h1.p;
     g.ld16 = h.hidden;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    g = args(B, h.hidden, h.hidden, h.h1.p, h.hidden, h.W16(1), h.hidden, h.errflag.p);
+    g.out16t = t != nullptr ? h.h1t.p : nullptr;
+    g.ldt = B;
+    if ((rc = gemm(g, nullptr, true, h.stream)) != PDHG_OK) return rc;
+    g = args(B, h.hidden, h.hidden, h.h1.p, h.hidden, h.W16(1), h.hidden, &h.status->err);
     g.bias = h.Bv(1);
     g.relu = 1;
     g.out16 = h.h2.p;
     g.ld16 = h.hidden;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    g = args(B, h.n_out, h.hidden, h.h2.p, h.hidden, h.W16(2), h.hidden, h.errflag.p);
+    g.out16t = t != nullptr ? h.h2t.p : nullptr;
+    g.ldt = B;
+    if ((rc = gemm(g, nullptr, true, h.stream)) != PDHG_OK) return rc;
+    g = args(B, h.n_out, h.hidden, h.h2.p, h.hidden, h.W16(2), h.hidden, &h.status->err);
     g.bias = h.Bv(2);
-    g.out32 = h.y32.p;
     g.ld32 = h.n_out;
-    return gemm(g, h.stream);
+    if (t == nullptr) {
+        g.out32 = h.y32.p;
+    } else {
+        g.target = t;
+        g.idx = idx;
+        g.scale = 1.f / static_cast<float>(static_cast<int64_t>(B) * h.n_out);
+        g.part = h.part.p;
+        g.out32 = h.dy32.p;
+        g.out16 = h.dy16.p;
+        g.ld16 = h.n_out;
+        g.out16t = h.dyt.p;
+        g.ldt = B;
+    }
+    return gemm(g, nullptr, true, h.stream);
 }
 
-// Gradients into h.g for the batch already in x16 / t32; loss -> part[0] sum.
-int backward(Mlp& h, int B) {
+// Gradients into h.g after forward() with targets; the batch's loss to *loss.
+int backward(Mlp& h, int B, double* loss) {
     int rc;
-    const int64_t cnt = static_cast<int64_t>(B) * h.n_out;
-    const int lb = blocks(cnt, 256);
-    k_loss_grad<<<lb, 256, 0, h.stream>>>(h.y32.p, h.t32.p, cnt,
-                                          1.f / static_cast<float>(cnt), h.dy32.p, h.dy16.p,
-                                          h.part.p + 1);
-    k_sum_parts<<<1, 32, 0, h.stream>>>(h.part.p + 1, lb, h.part.p);
-    // layer 3
-    transpose(h.dy16.p, h.n_out, h.dyt.p, B, B, h.n_out, h.stream);
-    transpose(h.h2.p, h.hidden, h.h2t.p, B, B, h.hidden, h.stream);
-    GemmArgs g = args(h.n_out, h.hidden, B, h.dyt.p, B, h.h2t.p, B, h.errflag.p);
+    int* err = &h.status->err;
+    // layer 3's weights and layer 2's input
+    GemmArgs g = args(h.n_out, h.hidden, B, h.dyt.p, B, h.h2t.p, B, err);
     g.out32 = h.gW(2);
     g.ld32 = h.hidden;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    k_colsum<<<blocks(h.n_out, 128), 128, 0, h.stream>>>(h.dy32.p, B, h.n_out, h.gB(2));
-    g = args(B, h.hidden, h.n_out, h.dy16.p, h.n_out, h.w3t.p, h.n_out, h.errflag.p);
-    g.mask = h.h2.p;
-    g.ldm = h.hidden;
-    g.out32 = h.dz2_32.p;
-    g.ld32 = h.hidden;
-    g.out16 = h.dz2_16.p;
-    g.ld16 = h.hidden;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    // layer 2
-    transpose(h.dz2_16.p, h.hidden, h.dz2t.p, B, B, h.hidden, h.stream);
-    transpose(h.h1.p, h.hidden, h.h1t.p, B, B, h.hidden, h.stream);
-    g = args(h.hidden, h.hidden, B, h.dz2t.p, B, h.h1t.p, B, h.errflag.p);
+    GemmArgs d = args(B, h.hidden, h.n_out, h.dy16.p, h.n_out, h.w3t.p, h.n_out, err);
+    d.mask = h.h2.p;
+    d.ldm = h.hidden;
+    d.out32 = h.dz2_32.p;
+    d.ld32 = h.hidden;
+    d.out16 = h.dz2_16.p;
+    d.ld16 = h.hidden;
+    d.out16t = h.dz2t.p;
+    d.ldt = B;
+    if ((rc = gemm(g, &d, true, h.stream)) != PDHG_OK) return rc;
+    // layer 2's weights and layer 1's input
+    g = args(h.hidden, h.hidden, B, h.dz2t.p, B, h.h1t.p, B, err);
     g.out32 = h.gW(1);
     g.ld32 = h.hidden;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    k_colsum<<<blocks(h.hidden, 128), 128, 0, h.stream>>>(h.dz2_32.p, B, h.hidden, h.gB(1));
-    g = args(B, h.hidden, h.hidden, h.dz2_16.p, h.hidden, h.w2t.p, h.hidden, h.errflag.p);
-    g.mask = h.h1.p;
-    g.ldm = h.hidden;
-    g.out32 = h.dz1_32.p;
-    g.ld32 = h.hidden;
-    g.out16 = h.dz1_16.p;
-    g.ld16 = h.hidden;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    // layer 1
-    transpose(h.dz1_16.p, h.hidden, h.dz1t.p, B, B, h.hidden, h.stream);
-    transpose(h.x16.p, h.n_in, h.xt.p, B, B, h.n_in, h.stream);
-    g = args(h.hidden, h.n_in, B, h.dz1t.p, B, h.xt.p, B, h.errflag.p);
+    d = args(B, h.hidden, h.hidden, h.dz2_16.p, h.hidden, h.w2t.p, h.hidden, err);
+    d.mask = h.h1.p;
+    d.ldm = h.hidden;
+    d.out32 = h.dz1_32.p;
+    d.ld32 = h.hidden;
+    d.out16t = h.dz1t.p;
+    d.ldt = B;
+    if ((rc = gemm(g, &d, true, h.stream)) != PDHG_OK) return rc;
+    // layer 1's weights
+    g = args(h.hidden, h.n_in, B, h.dz1t.p, B, h.xt.p, B, err);
     g.out32 = h.gW(0);
     g.ld32 = h.n_in;
-    if ((rc = gemm(g, h.stream)) != PDHG_OK) return rc;
-    k_colsum<<<blocks(h.hidden, 128), 128, 0, h.stream>>>(h.dz1_32.p, B, h.hidden, h.gB(0));
+    if ((rc = gemm(g, nullptr, true, h.stream)) != PDHG_OK) return rc;
+    ColSums c{};
+    const float* dz[3] = {h.dy32.p, h.dz2_32.p, h.dz1_32.p};
+    const int n[3] = {h.n_out, h.hidden, h.hidden};
+    for (int i = 0; i < 3; ++i) {
+        c.dz[i] = dz[i];
+        c.db[i] = h.gB(2 - i);
+        c.N[i] = n[i];
+        c.first[i + 1] = c.first[i] + blocks(n[i], 32);
+    }
+    c.B = B;
+    c.part = h.part.p;
+    c.n_part = loss_parts(B, h.n_out);
+    c.loss = loss;
+    return launch_pass(k_colsums, c.first[3] + 1, true, h.stream, c) == cudaSuccess ? PDHG_OK : PDHG_ERR_BACKEND;
+}
+
+// The batch's inputs (rows idx, null: in order) in BF16, transposed too for a gradient.
+int set_batch(Mlp& h, int B, const float* x, const int32_t* idx, bool gradient) {
+    k_gather_rows<<<dim3(blocks(h.n_in, 32), blocks(B, 32)), dim3(32, 8), 0, h.stream>>>(
+        x, h.n_in, idx, B, h.x16.p, gradient ? h.xt.p : nullptr);
+    MCK(cudaGetLastError());
     return PDHG_OK;
 }
 
 int upload_batch(Mlp& h, int B, const float* x, const float* t) {
-    std::vector<int32_t> id(static_cast<size_t>(B));
-    for (int i = 0; i < B; ++i) id[i] = i;
-    Dev<float> xs, ts;
-    MCK(xs.alloc(static_cast<size_t>(B) * h.n_in));
-    MCK(cudaMemcpyAsync(xs.p, x, sizeof(float) * B * h.n_in, cudaMemcpyHostToDevice, h.stream));
-    MCK(cudaMemcpyAsync(h.idx.p, id.data(), sizeof(int32_t) * B, cudaMemcpyHostToDevice, h.stream));
-    k_gather_rows<<<blocks(static_cast<int64_t>(B) * h.n_in, 256), 256, 0, h.stream>>>(
-        xs.p, h.n_in, h.idx.p, B, nullptr, h.x16.p);
-    if (t != nullptr) {
-        MCK(ts.alloc(static_cast<size_t>(B) * h.n_out));
-        MCK(cudaMemcpyAsync(ts.p, t, sizeof(float) * B * h.n_out, cudaMemcpyHostToDevice, h.stream));
-        k_gather_rows<<<blocks(static_cast<int64_t>(B) * h.n_out, 256), 256, 0, h.stream>>>(
-            ts.p, h.n_out, h.idx.p, B, h.t32.p, nullptr);
-    }
-    MCK(cudaStreamSynchronize(h.stream));  // xs / ts are freed on return
-    return PDHG_OK;
+    MCK(cudaMemcpyAsync(h.x32.p, x, sizeof(float) * B * h.n_in, cudaMemcpyHostToDevice, h.stream));
+    if (t != nullptr)
+        MCK(cudaMemcpyAsync(h.t32.p, t, sizeof(float) * B * h.n_out, cudaMemcpyHostToDevice, h.stream));
+    return set_batch(h, B, h.x32.p, nullptr, t != nullptr);
 }
 
 bool batch_ok(const Mlp& h, int B) { return B >= 8 && B % 8 == 0 && B <= h.max_batch; }
@@ -544,6 +706,7 @@ int pdhg_mlp_create(int device, int n_in, int hidden, int n_out, int max_batch, 
     h.n_out = n_out;
     h.max_batch = max_batch;
     MCK(cudaSetDevice(device));
+    MCK(init_gemm());
     MCK(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     const int64_t sizes[6] = {static_cast<int64_t>(hidden) * n_in, hidden,
                               static_cast<int64_t>(hidden) * hidden, hidden,
@@ -564,6 +727,7 @@ int pdhg_mlp_create(int device, int n_in, int hidden, int n_out, int max_batch, 
     MCK(h.w2t.alloc(H * H));
     MCK(h.w3t.alloc(H * n_out));
     MCK(h.x16.alloc(B * n_in));
+    MCK(h.x32.alloc(B * n_in));
     MCK(h.xt.alloc(B * n_in));
     MCK(h.h1.alloc(B * H));
     MCK(h.h1t.alloc(B * H));
@@ -573,20 +737,19 @@ int pdhg_mlp_create(int device, int n_in, int hidden, int n_out, int max_batch, 
     MCK(h.dyt.alloc(B * n_out));
     MCK(h.dz2_16.alloc(B * H));
     MCK(h.dz2t.alloc(B * H));
-    MCK(h.dz1_16.alloc(B * H));
     MCK(h.dz1t.alloc(B * H));
     MCK(h.t32.alloc(B * n_out));
     MCK(h.y32.alloc(B * n_out));
     MCK(h.dy32.alloc(B * n_out));
     MCK(h.dz2_32.alloc(B * H));
     MCK(h.dz1_32.alloc(B * H));
-    MCK(h.part.alloc(B * n_out / 256 + 4));
-    MCK(h.idx.alloc(B));
-    MCK(h.errflag.alloc(1));
+    // a batch of fewer rows has narrower tiles, up to kGemmSms of them
+    MCK(h.part.alloc(std::max<size_t>(loss_parts(max_batch, n_out), kGemmSms)));
+    MCK(cudaHostAlloc(reinterpret_cast<void**>(&h.status), sizeof(Mlp::Status), cudaHostAllocDefault));
+    *h.status = Mlp::Status{};
     MCK(cudaMemsetAsync(h.w.p, 0, sizeof(float) * o, h.stream));
     MCK(cudaMemsetAsync(h.m.p, 0, sizeof(float) * o, h.stream));
     MCK(cudaMemsetAsync(h.v.p, 0, sizeof(float) * o, h.stream));
-    MCK(cudaMemsetAsync(h.errflag.p, 0, sizeof(int), h.stream));
     MCK(cudaStreamSynchronize(h.stream));
     *out = p.release();
     return PDHG_OK;
@@ -654,7 +817,7 @@ int pdhg_mlp_forward(pdhg_mlp* p, int batch, const float* x, float* y) {
     MCK(cudaSetDevice(h.device));
     int rc = upload_batch(h, batch, x, nullptr);
     if (rc != PDHG_OK) return rc;
-    if ((rc = forward(h, batch)) != PDHG_OK) return rc;
+    if ((rc = forward(h, batch, nullptr, nullptr)) != PDHG_OK) return rc;
     MCK(cudaMemcpyAsync(y, h.y32.p, sizeof(float) * batch * h.n_out, cudaMemcpyDeviceToHost,
                         h.stream));
     return check_err(h);
@@ -670,18 +833,12 @@ int pdhg_mlp_gradients(pdhg_mlp* p, int batch, const float* x, const float* t, f
     MCK(cudaSetDevice(h.device));
     int rc = upload_batch(h, batch, x, t);
     if (rc != PDHG_OK) return rc;
-    if ((rc = forward(h, batch)) != PDHG_OK) return rc;
-    if ((rc = backward(h, batch)) != PDHG_OK) return rc;
-    int64_t dst = 0;
-    for (int i = 0; i < 6; ++i) {
-        MCK(cudaMemcpyAsync(grads + dst, h.g.p + h.off[i], sizeof(float) * h.cnt[i],
-                            cudaMemcpyDeviceToHost, h.stream));
-        dst += h.cnt[i];
-    }
-    double l = 0.0;
-    MCK(cudaMemcpyAsync(&l, h.part.p, sizeof l, cudaMemcpyDeviceToHost, h.stream));
+    if ((rc = forward(h, batch, h.t32.p, nullptr)) != PDHG_OK) return rc;
+    if ((rc = backward(h, batch, &h.status->loss)) != PDHG_OK) return rc;
+    // every section is a multiple of 8 entries (the dimensions are): one block
+    MCK(cudaMemcpyAsync(grads, h.g.p, sizeof(float) * h.total, cudaMemcpyDeviceToHost, h.stream));
     rc = check_err(h);
-    if (loss != nullptr) *loss = static_cast<float>(l);
+    if (loss != nullptr) *loss = static_cast<float>(h.status->loss);
     return rc;
 }
 
@@ -746,15 +903,10 @@ int pdhg_mlp_train(pdhg_mlp* p, int64_t samples, const float* x, const float* t,
                             cudaMemcpyHostToDevice, h.stream));
         for (int sI = 0; sI < steps; ++sI) {
             const int32_t* idx = perm_d.p + static_cast<int64_t>(sI) * batch;
-            k_gather_rows<<<blocks(static_cast<int64_t>(batch) * h.n_in, 256), 256, 0, h.stream>>>(
-                h.xs.p, h.n_in, idx, batch, nullptr, h.x16.p);
-            k_gather_rows<<<blocks(static_cast<int64_t>(batch) * h.n_out, 256), 256, 0, h.stream>>>(
-                h.ts.p, h.n_out, idx, batch, h.t32.p, nullptr);
-            int rc = forward(h, batch);
-            if (rc == PDHG_OK) rc = backward(h, batch);
+            int rc = set_batch(h, batch, h.xs.p, idx, true);
+            if (rc == PDHG_OK) rc = forward(h, batch, h.ts.p, idx);
+            if (rc == PDHG_OK) rc = backward(h, batch, lsum.p + sI);
             if (rc != PDHG_OK) return rc;
-            MCK(cudaMemcpyAsync(lsum.p + sI, h.part.p, sizeof(double), cudaMemcpyDeviceToDevice,
-                                h.stream));
             h.adam_t += 1;
             const float c1 = 1.f - std::pow(b1, static_cast<float>(h.adam_t));
             const float c2 = 1.f - std::pow(b2, static_cast<float>(h.adam_t));
@@ -784,6 +936,7 @@ int pdhg_gemm_bf16(int device, int m, int n, int k, const float* a, const float*
     if (m < 1 || n < 1 || k < 8 || k % 8 || a == nullptr || b == nullptr || c == nullptr)
         return PDHG_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(device) != cudaSuccess) return PDHG_ERR_UNSUPPORTED;
+    if (init_gemm() != cudaSuccess) return PDHG_ERR_BACKEND;
     Dev<float> a32, b32, c32, bias32;
     Dev<bf16> a16, b16;
     Dev<int> err;
@@ -802,7 +955,7 @@ int pdhg_gemm_bf16(int device, int m, int n, int k, const float* a, const float*
     g.relu = relu;
     g.out32 = c32.p;
     g.ld32 = n;
-    int rc = gemm(g, nullptr);
+    int rc = gemm(g, nullptr, false, nullptr);
     if (rc != PDHG_OK) return rc;
     int e = 0;
     if (cudaMemcpy(&e, err.p, sizeof e, cudaMemcpyDeviceToHost) != cudaSuccess) return PDHG_ERR_BACKEND;
