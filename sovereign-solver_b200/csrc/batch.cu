@@ -80,6 +80,7 @@ struct BatchCtx {
     } plan[2][2];  // [FP32, FP64][averaged, Halpern]
     DBuf<unsigned char> far;  // entries of instances too large for shared memory, set up by each solve
     ResStreams side;
+    Downloads downloads;
 
     // solve graphs, [0] FP32 and [1] FP64, with what they bake in
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -986,10 +987,10 @@ int batch_solve(BatchCtx& c, const pdhg_options& o, pdhg_info* infos, double* x,
     BCK(cudaMemcpyAsync(h.data(), c.is.p, sizeof(InstState) * c.count, cudaMemcpyDeviceToHost, s));
     BatchGlobal g2;
     BCK(cudaMemcpyAsync(&g2, c.g.p, sizeof g2, cudaMemcpyDeviceToHost, s));
-    if (x != nullptr && c.n) BCK(cudaMemcpyAsync(x, c.xo.p, sizeof(double) * c.n, cudaMemcpyDeviceToHost, s));
-    if (y != nullptr && c.m) BCK(cudaMemcpyAsync(y, c.yo.p, sizeof(double) * c.m, cudaMemcpyDeviceToHost, s));
-    if (rcv != nullptr && c.n) BCK(cudaMemcpyAsync(rcv, c.rc.p, sizeof(double) * c.n, cudaMemcpyDeviceToHost, s));
-    BCK(cudaStreamSynchronize(s));
+    const Downloads::Part down[3] = {{x, c.xo.p, sizeof(double) * static_cast<size_t>(c.n)},
+                                     {y, c.yo.p, sizeof(double) * static_cast<size_t>(c.m)},
+                                     {rcv, c.rc.p, sizeof(double) * static_cast<size_t>(c.n)}};
+    BCK(c.downloads.run(down, 3, c.device, s));
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     for (int32_t k = 0; k < c.count; ++k) {
         pdhg_info& inf = infos[k];

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/pdhg_b200.h"
+#include "download.cuh"
 #include "engine.cuh"
 
 namespace pdhg {

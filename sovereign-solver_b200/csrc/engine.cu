@@ -61,6 +61,7 @@ struct Ctx {
     int device = 0;
     int sm_count = 148;
     cudaStream_t stream = nullptr;
+    Downloads downloads;
     PassFork fork;  // side stream + events: short- and long-row kernels side by side
     std::string err;
     long long gen = 0;  // bumps on every load / rescale
@@ -1381,10 +1382,10 @@ int solve(Ctx& c, const pdhg_options& o, pdhg_info* info, double* x, double* y, 
     c.launches += 5;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&h, c.st.p, sizeof h, cudaMemcpyDeviceToHost, c.stream));
-    if (x != nullptr && n) CK(cudaMemcpyAsync(x, c.xo.p, sizeof(double) * n, cudaMemcpyDeviceToHost, c.stream));
-    if (y != nullptr && m) CK(cudaMemcpyAsync(y, c.yo.p, sizeof(double) * m, cudaMemcpyDeviceToHost, c.stream));
-    if (rcv != nullptr && n) CK(cudaMemcpyAsync(rcv, c.rc.p, sizeof(double) * n, cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaStreamSynchronize(c.stream));
+    const Downloads::Part down[3] = {{x, c.xo.p, sizeof(double) * static_cast<size_t>(n)},
+                                     {y, c.yo.p, sizeof(double) * static_cast<size_t>(m)},
+                                     {rcv, c.rc.p, sizeof(double) * static_cast<size_t>(n)}};
+    CK(c.downloads.run(down, 3, c.device, c.stream));
     pc.mark("solve: result, download");
     info->objective = h.objective;
     info->primal_infeasibility = h.pinf;
