@@ -125,6 +125,8 @@ struct MatDev {
     int vw = 1;
     int32_t rp_stride = 0;  // every row this long (0: not uniform)
     int64_t nnz_dense = 0;  // entries of the dense rows (columns computed)
+    DBuf<int2> runs;        // column runs of rows of two entries, if in use
+    int64_t nnz_runs = 0;   // entries whose columns they give
     DevCsr view() const {
         DevCsr d;
         d.rows = rows;
@@ -155,6 +157,7 @@ struct MatDev {
         d.no_slice_tiers = no_slice_tiers.view();
         d.rp_stride = rp_stride;
         d.dense_off = dense_off.p;
+        d.runs = runs.p;
         return d;
     }
 };
@@ -549,6 +552,34 @@ inline int build_dense_rows(MatDev& M, cudaStream_t s, std::string* err) {
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_fail(err, e, "build_dense_rows");
     M.nnz_dense = static_cast<int64_t>(h);
+    return PDHG_OK;
+}
+
+// Column runs of a matrix of two entries per row (k_col_runs); kept where at
+// least three in four descriptors are runs -- the others load the descriptor
+// and then the columns, one after the other.
+inline int build_col_runs(MatDev& M, cudaStream_t s, std::string* err) {
+    const char* knob = std::getenv("PDHG_B200_DENSE_ROWS");  // "0": load every column index
+    M.nnz_runs = 0;
+    M.runs.release();
+    if (M.rp_stride != 2 || (knob != nullptr && knob[0] == '0')) return PDHG_OK;
+    const size_t n = (static_cast<size_t>(M.rows) + 31) / 32;
+    if (M.runs.alloc(n) != cudaSuccess) {  // no room: the columns are loaded
+        M.runs.release();
+        cudaGetLastError();
+        return PDHG_OK;
+    }
+    DBuf<unsigned long long> cnt;
+    unsigned long long h = 0;
+    cudaError_t e;
+    if ((e = cnt.alloc(1)) != cudaSuccess || (e = cudaMemsetAsync(cnt.p, 0, sizeof h, s)) != cudaSuccess)
+        return cuda_fail(err, e, "build_col_runs");
+    launch_col_runs(M.ci.p, M.rows, M.runs.p, cnt.p, s);
+    if ((e = cudaMemcpyAsync(&h, cnt.p, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        return cuda_fail(err, e, "build_col_runs");
+    if (4 * h < 3 * n) M.runs.release();
+    else M.nnz_runs = std::min<int64_t>(64 * static_cast<int64_t>(h), M.nnz);
     return PDHG_OK;
 }
 

@@ -284,6 +284,8 @@ int ensure_scaled(Ctx& c, const ScalingParams& sp) {
     if (rc != PDHG_OK) return rc;
     rc = build_dense_rows(c.ATs, s, &c.err);
     if (rc != PDHG_OK) return rc;
+    rc = build_col_runs(c.ATs, s, &c.err);
+    if (rc != PDHG_OK) return rc;
     const double sign = c.lp.maximize ? -1.0 : 1.0;
     CK(c.c_s.alloc(static_cast<size_t>(n) + 1));
     CK(c.lo_s.alloc(static_cast<size_t>(n) + 1));
@@ -1489,7 +1491,7 @@ int load(Ctx& c, int32_t m, int32_t n, int64_t nnz, const int32_t* row_ptr,
 // plus T(z) once a period. What this LP's structure makes constant carries
 // no information and is not counted: the row pointer where every row has the
 // same length, the column bounds where all are equal, the column indices of
-// dense rows and (where the pass uses them) of affine row slices -- the
+// dense rows, of column runs and (where the pass uses them) of affine row slices -- the
 // kernels compute those instead of loading them.
 double iter_bytes(const Ctx& c, int prec, bool primal, bool halpern, long long period,
                   const DevCsr& D) {
@@ -1503,7 +1505,7 @@ double iter_bytes(const Ctx& c, int prec, bool primal, bool halpern, long long p
     if (prec == PDHG_PREC_FP64_EXACT) return b;  // the ordered kernels load everything
     if (D.rp_stride > 0) b -= 4.0 * (rows + 1);
     if (primal && c.col_uniform) b -= 2.0 * vb * rows;
-    b -= 4.0 * static_cast<double>(M.nnz_dense + (D.use_slices ? M.slices.nnz_affine : 0));
+    b -= 4.0 * static_cast<double>(M.nnz_dense + M.nnz_runs + (D.use_slices ? M.slices.nnz_affine : 0));
     return b;
 }
 

@@ -143,7 +143,18 @@ struct DevCsr {
     // columns), kNotDense otherwise; the long-row iteration paths then compute
     // the columns and stream the gathered vector
     const int32_t* dense_off = nullptr;
+    // rows of two entries (rp_stride 2; else null): per 32 consecutive rows a
+    // descriptor of each entry's column, from which the uniform kernels compute
+    // the columns instead of loading them (run_col)
+    const int2* runs = nullptr;
 };
+// A run descriptor: the first of the 32 rows' column, and in the top bit
+// whether the column rises by one from row to row (else it is the same in all).
+// kNoRun in .x: the rows' columns follow neither form and are loaded.
+constexpr int32_t kNoRun = -1;
+__host__ __device__ inline int32_t run_col(int32_t d, int lane) {
+    return (d & 0x7fffffff) + (d < 0 ? lane : 0);
+}
 constexpr int32_t kNotDense = static_cast<int32_t>(0x80808080u);  // a byte-wise memset value
 
 
@@ -500,6 +511,7 @@ void launch_gather_cols(const int32_t* ci, const int64_t* pos, int32_t n, int32_
 // of affine slices / dense rows to
 void launch_affine_slices(const RowSlices& S, int2* affine, unsigned long long* nnz_affine,
                           cudaStream_t s);
+void launch_col_runs(const int32_t* ci, int32_t rows, int2* runs, unsigned long long* n_run, cudaStream_t s);
 void launch_dense_rows(const int32_t* ci, const int4* ext, int32_t n_ext, int32_t* dense_off,
                        unsigned long long* nnz_dense, cudaStream_t s);
 void launch_fill_slices(const DevCsr& M, RowSlices S, int32_t* col, float* v32, double* v64,

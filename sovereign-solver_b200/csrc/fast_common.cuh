@@ -39,14 +39,14 @@ struct PV {
     T lo_u, hi_u;
 };
 template <class T>
-__device__ __forceinline__ PV<T> pvec(const DevProblem& P);
+__host__ __device__ __forceinline__ PV<T> pvec(const DevProblem& P);
 template <>
-__device__ __forceinline__ PV<float> pvec<float>(const DevProblem& P) {
+__host__ __device__ __forceinline__ PV<float> pvec<float>(const DevProblem& P) {
     return {P.c32, P.lo32, P.hi32, P.rlo32, P.rhi32, P.col_bounds_uniform,
             static_cast<float>(P.lo_u), static_cast<float>(P.hi_u)};
 }
 template <>
-__device__ __forceinline__ PV<double> pvec<double>(const DevProblem& P) {
+__host__ __device__ __forceinline__ PV<double> pvec<double>(const DevProblem& P) {
     return {P.c, P.lo, P.hi, P.rlo, P.rhi, P.col_bounds_uniform, P.lo_u, P.hi_u};
 }
 

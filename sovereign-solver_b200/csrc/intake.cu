@@ -239,6 +239,28 @@ __global__ void k_dense_rows(const int32_t* ci, const int4* ext, int32_t n_ext, 
     }
 }
 
+// Rows of two entries: per 32 consecutive rows the columns' run descriptor
+// (engine.cuh run_col) where every row's first entries sit in one column or in
+// consecutive ones and so do the second entries (the columns of a
+// transportation LP: one supply row, consecutive demand rows); every entry is
+// compared. One warp per descriptor; *n_run counts those that are runs.
+__global__ void __launch_bounds__(kBlock) k_col_runs(const int32_t* ci, int32_t rows, int2* runs,
+                                                     unsigned long long* n_run) {
+    const int64_t r = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x;
+    const int lane = static_cast<int>(threadIdx.x & 31);
+    const bool in = r < rows;
+    const int c0 = in ? ci[2 * r] : 0, c1 = in ? ci[2 * r + 1] : 0;
+    const int b0 = __shfl_sync(0xffffffffu, c0, 0), b1 = __shfl_sync(0xffffffffu, c1, 0);
+    auto same = [&](int c, int b) { return __all_sync(0xffffffffu, !in || c == b); };
+    auto rises = [&](int c, int b) { return __all_sync(0xffffffffu, !in || c - b == lane); };
+    const bool s0 = same(c0, b0), s1 = same(c1, b1), r0 = rises(c0, b0), r1 = rises(c1, b1);
+    if (lane != 0 || !in) return;
+    const bool run = (s0 || r0) && (s1 || r1);
+    const int32_t top = static_cast<int32_t>(0x80000000u);
+    runs[r >> 5] = run ? make_int2(s0 ? b0 : b0 | top, s1 ? b1 : b1 | top) : make_int2(kNoRun, kNoRun);
+    if (run) atomicAdd(n_run, 1ull);
+}
+
 // Rows with lo < length <= hi appended to `list` (grid-stride; one atomic per
 // warp that has any).
 __global__ void k_bin_range(const int32_t* rp, int32_t rows, int lo, int hi, int32_t* list,
@@ -551,6 +573,12 @@ void launch_row_extents(const int32_t* rows, int32_t n, const int32_t* rp, int4*
 void launch_gather_cols(const int32_t* ci, const int64_t* pos, int32_t n, int32_t* out,
                         cudaStream_t s) {
     if (n > 0) k_gather_cols<<<nblocks(n), kBlock, 0, s>>>(ci, pos, n, out);
+}
+
+void launch_col_runs(const int32_t* ci, int32_t rows, int2* runs, unsigned long long* n_run, cudaStream_t s) {
+    if (rows > 0)
+        k_col_runs<<<static_cast<int>((static_cast<int64_t>(rows) + kBlock - 1) / kBlock), kBlock, 0, s>>>(ci, rows, runs,
+                                                                                                         n_run);
 }
 
 void launch_dense_rows(const int32_t* ci, const int4* ext, int32_t n_ext, int32_t* dense_off,

@@ -59,6 +59,12 @@
 #ifndef PDHG_UNIFORM_MIN_CTAS_E4
 #define PDHG_UNIFORM_MIN_CTAS_E4 6
 #endif
+#ifndef PDHG_WIDE_MIN_CTAS
+#define PDHG_WIDE_MIN_CTAS 5
+#endif
+#ifndef PDHG_WIDE_MIN_CTAS_F64
+#define PDHG_WIDE_MIN_CTAS_F64 5
+#endif
 #ifndef PDHG_UNIFORM_MIN_CTAS_F64
 #define PDHG_UNIFORM_MIN_CTAS_F64 4
 #endif
@@ -269,7 +275,7 @@ constexpr int uniform_min_ctas() {
     return sizeof(T) == 8 ? PDHG_UNIFORM_MIN_CTAS_F64 : (E == 2 ? PDHG_UNIFORM_MIN_CTAS : PDHG_UNIFORM_MIN_CTAS_E4);
 }
 
-template <class T, int E, int VW, bool PRIMAL, bool EARLY>
+template <class T, int E, int VW, bool PRIMAL, bool EARLY, bool RUNS>
 __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     fast_iter_uniform(FastIter<T> a, int first, int reset) {
     constexpr int S = E * VW;
@@ -291,9 +297,18 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     EpiIn<T> in{};
     if (!EARLY && lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
     if (EARLY && lane == 0) in = epi_load_fixed<T, PRIMAL>(a.it, pv, r);
-    int c[E];
+    int c[E];  // RUNS: the row's run descriptor until its columns are needed
     T v[E];
-    load_idx<E>(M.ci + static_cast<int64_t>(r) * S + lane * E, c);
+    auto load_cols = [&](int row, int (&to)[E]) {
+        if constexpr (RUNS) {
+            const int2 d = __ldg(M.runs + (row >> 5));
+            to[0] = d.x;
+            to[1] = d.y;
+        } else {
+            load_idx<E>(M.ci + static_cast<int64_t>(row) * S + lane * E, to);
+        }
+    };
+    load_cols(r, c);
     load_vals<T, E>(vals + static_cast<int64_t>(r) * S + lane * E, v);
     if (EARLY) {
         pass_wait();
@@ -301,6 +316,14 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     }
     for (;;) {
         T g[E];
+        if constexpr (RUNS) {  // a warp's 32 rows share a descriptor
+            if (c[0] != kNoRun) {
+#pragma unroll
+                for (int q = 0; q < E; ++q) c[q] = run_col(c[q], r & 31);
+            } else {
+                load_idx<E>(M.ci + static_cast<int64_t>(r) * S, c);
+            }
+        }
 #pragma unroll
         for (int q = 0; q < E; ++q) g[q] = gather_ld<EARLY>(xg + c[q]);
         const int rn = r + groups;
@@ -310,7 +333,7 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
         T nv[E];
         if (more) {
             if (lane == 0) nin = pass_operands<T, PRIMAL, EARLY>(a.it, pv, rn, first, fresh, hw);
-            load_idx<E>(M.ci + static_cast<int64_t>(rn) * S + lane * E, nc);
+            load_cols(rn, nc);
             load_vals<T, E>(vals + static_cast<int64_t>(rn) * S + lane * E, nv);
         }
         T acc = mul_rn<T>(v[0], g[0]);
@@ -326,6 +349,162 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
             c[q] = nc[q];
             v[q] = nv[q];
         }
+    }
+}
+
+// kWide<T> consecutive values as one 16-byte vector.
+template <class T>
+constexpr int kWide = 16 / static_cast<int>(sizeof(T));
+template <class T>
+struct Wide {
+    T e[kWide<T>];
+};
+template <class T>
+struct WideVec;
+template <>
+struct WideVec<float> {
+    using type = float4;
+};
+template <>
+struct WideVec<double> {
+    using type = double2;
+};
+template <class T>
+__device__ __forceinline__ Wide<T> wide_ldcs(const T* p) {
+    using V = typename WideVec<T>::type;
+    union {
+        V v;
+        Wide<T> w;
+    } u;
+    u.v = __ldcs(reinterpret_cast<const V*>(p));
+    return u.w;
+}
+template <class T, bool EARLY>  // what the passes write
+__device__ __forceinline__ Wide<T> wide_moving(const T* p, bool stream) {
+    using V = typename WideVec<T>::type;
+    union {
+        V v;
+        Wide<T> w;
+    } u;
+    if (EARLY) u.v = coherent_ld(reinterpret_cast<const V*>(p));
+    else if (stream) u.v = __ldcs(reinterpret_cast<const V*>(p));
+    else u.v = *reinterpret_cast<const V*>(p);
+    return u.w;
+}
+template <class T, bool STREAM>
+__device__ __forceinline__ void wide_st(T* p, const Wide<T>& w) {
+    using V = typename WideVec<T>::type;
+    union {
+        V v;
+        Wide<T> w;
+    } u;
+    u.w = w;
+    if (STREAM) __stcs(reinterpret_cast<V*>(p), u.v);
+    else *reinterpret_cast<V*>(p) = u.v;
+}
+
+// The primal pass over columns of two entries given by runs: a thread takes
+// kWide<T> consecutive columns, every operand, value pair and result as 16-byte
+// vectors (UB: all columns have the same bounds). fast_iter_uniform's updates
+// and order of sums.
+//
+// Bound: HBM on a large LP. One column per thread and step keeps 20 bytes a
+// thread in flight, which at eight CTAs per SM is 6 MB on the chip, about what
+// HBM's latency times its rate asks for and only while no thread waits for its
+// gathers; a vector of columns keeps four times that. The 10M-column
+// transportation LP, FP32: fast_iter_uniform loading the columns 55.7 us, from
+// runs 52.5 us, this kernel 33.3 us (242 MB, 7.3 TB/s with what L2 still holds);
+// 1,000 x 2,200 FP64 27.3 -> 19.1 us, 400 x 1,000 FP32 (launched early) 9.6 ->
+// 8.0 us. 3 / 4 / 5 / 6 CTAs per SM: within 5%.
+template <class T, bool UB, bool EARLY>
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? PDHG_WIDE_MIN_CTAS : PDHG_WIDE_MIN_CTAS_F64)
+    fast_primal_wide(FastIter<T> a, int first, int reset) {
+    constexpr int W = kWide<T>;
+    if (EARLY) pass_begin();
+    DevState* st = a.st;
+    iter_reset(st, reset);
+    if (st->done) return;
+    const DevCsr& M = a.AT;
+    const Iterates<T>& it = a.it;
+    const T* __restrict__ vals = mvals<T>(M);
+    const PV<T> pv = pvec<T>(a.P);
+    const bool fresh = first && st->fresh;
+    const T tau = static_cast<T>(st->tau);
+    const Hw<T> hw = halpern_weight_warp<T>(it, st, a.hk);
+    const int n_wide = M.rows / W;
+    bool waited = !EARLY;
+    for (int q = blockIdx.x * kBlock + static_cast<int>(threadIdx.x); q < n_wide; q += gridDim.x * kBlock) {
+        const int r = q * W;
+        const int2 d = __ldg(M.runs + (r >> 5));
+        const Wide<T> c = wide_ldcs(pv.c + r);
+        Wide<T> lo, hi, ps, b, v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) v[u] = wide_ldcs(vals + 2 * static_cast<int64_t>(r) + u * W);
+        if (!UB) {
+            lo = wide_ldcs(pv.lo + r);
+            hi = wide_ldcs(pv.hi + r);
+        }
+        if (it.halpern) ps = wide_ldcs(it.xa + r);
+        if (!waited) {
+            pass_wait();
+            waited = true;
+        }
+        b = it.lean ? wide_moving<T, EARLY>(it.xbar + r, false) : wide_moving<T, EARLY>(it.x + r, true);
+        if (!it.halpern) {
+            T* sums;
+            if constexpr (std::is_same<T, float>::value) sums = it.psx;
+            else sums = it.xsum;
+            if (std::is_same<T, float>::value ? first != 0 : fresh) ps = Wide<T>{};
+            else ps = wide_moving<T, EARLY>(sums + r, true);
+        }
+        int c0[W], c1[W];
+        if (d.x != kNoRun) {
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                c0[i] = run_col(d.x, (r & 31) + i);
+                c1[i] = run_col(d.y, (r & 31) + i);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                const int2 k = __ldcs(reinterpret_cast<const int2*>(M.ci) + r + i);
+                c0[i] = k.x;
+                c1[i] = k.y;
+            }
+        }
+        T g0[W], g1[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            g0[i] = gather_ld<EARLY>(it.y + c0[i]);
+            g1[i] = gather_ld<EARLY>(it.y + c1[i]);
+        }
+        Wide<T> xb, xo, sum;  // x_bar, x, the sums' slot
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            const T* pair = v[2 * i / W].e + 2 * i % W;
+            const T dot = fma_rn<T>(pair[1], g1[i], mul_rn<T>(pair[0], g0[i]));
+            const T x = !it.lean ? b.e[i] : hw.wp == T(0) ? ps.e[i] : halpern_mix<T>(hw.wp, b.e[i], ps.e[i]);
+            const T xn = clampT<T>(x - tau * (c.e[i] - dot), UB ? pv.lo_u : lo.e[i], UB ? pv.hi_u : hi.e[i]);
+            xb.e[i] = T(2) * xn - x;
+            xo.e[i] = it.halpern ? halpern_mix<T>(hw.w, xb.e[i], ps.e[i]) : xn;
+            sum.e[i] = it.halpern ? xn : ps.e[i] + xn;
+        }
+        wide_st<T, false>(it.xbar + r, xb);
+        if (!it.lean || a.tz != 0) {
+            wide_st<T, true>(it.x + r, xo);
+            if constexpr (std::is_same<T, float>::value) wide_st<T, true>(it.psx + r, sum);
+            else wide_st<T, true>(it.xsum + r, sum);
+        }
+    }
+    if (!waited) pass_wait();
+    // the last columns, fewer than a vector
+    const int r = n_wide * W + static_cast<int>(threadIdx.x);
+    if (blockIdx.x == 0 && r < M.rows) {
+        const EpiIn<T> in = pass_operands<T, true, EARLY>(it, pv, r, first, fresh, hw);
+        const int2 k = __ldcs(reinterpret_cast<const int2*>(M.ci) + r);
+        const T* e = vals + 2 * static_cast<int64_t>(r);
+        const T g0 = gather_ld<EARLY>(it.y + k.x), g1 = gather_ld<EARLY>(it.y + k.y);
+        epi_store<T, true>(it, r, fma_rn<T>(e[1], g1, mul_rn<T>(e[0], g0)), in, tau, T(0), hw, a.tz);
     }
 }
 
@@ -641,6 +820,9 @@ int g_cap_uni[3][2] = {{148 * PDHG_UNIFORM_MIN_CTAS, 148 * PDHG_UNIFORM_MIN_CTAS
                        {148 * PDHG_UNIFORM_MIN_CTAS_E4, 148 * PDHG_UNIFORM_MIN_CTAS_F64},
                        {148 * PDHG_UNIFORM_MIN_CTAS_E4, 148 * PDHG_UNIFORM_MIN_CTAS_F64}};
 
+// ... and of fast_primal_wide
+int g_cap_wide[2] = {148 * PDHG_WIDE_MIN_CTAS, 148 * PDHG_WIDE_MIN_CTAS_F64};
+
 inline PassPlan pass_plan(const DevCsr& M, int cap_long, int cap_slice, int cap_slice_w) {
     PassPlan p;
     if (M.rows == 0) return p;
@@ -690,13 +872,47 @@ int uniform_slot(const DevCsr& M) {
     return M.rp_stride == 2 ? 0 : M.rp_stride == 4 ? 1 : M.rp_stride == 8 ? 2 : -1;
 }
 
+// fast_primal_wide's operands, all 16-byte aligned.
+template <class T>
+bool wide_ok(const FastIter<T>& a) {
+    if (a.AT.runs == nullptr) return false;
+    const PV<T> pv = pvec<T>(a.P);
+    const Iterates<T>& it = a.it;
+    const void* sums = std::is_same<T, float>::value ? static_cast<const void*>(it.psx) : it.xsum;
+    uintptr_t all = 0;
+    for (const void* p : {static_cast<const void*>(pv.c), static_cast<const void*>(pv.lo), static_cast<const void*>(pv.hi),
+                          static_cast<const void*>(it.x), static_cast<const void*>(it.xbar),
+                          static_cast<const void*>(it.xa), sums})
+        all |= reinterpret_cast<uintptr_t>(p);
+    return (all & 15u) == 0;
+}
+
+template <class T>
+void launch_wide(const FastIter<T>& a, int cap, int first, int reset, cudaStream_t s, bool early) {
+    const int64_t need = (static_cast<int64_t>(a.AT.rows) / kWide<T> + kBlock) / kBlock;
+    const int grid = static_cast<int>(need < cap ? need : cap);
+    auto run = [&](auto kernel) { launch_pass(kernel, grid, early, s, a, first, reset); };
+    const bool ub = pvec<T>(a.P).ub;
+    if (a.early && ub) run(fast_primal_wide<T, true, true>);
+    else if (a.early) run(fast_primal_wide<T, false, true>);
+    else if (ub) run(fast_primal_wide<T, true, false>);
+    else run(fast_primal_wide<T, false, false>);
+}
+
 template <class T, int E, int VW, bool PRIMAL>
 void launch_uniform(const FastIter<T>& a, const DevCsr& M, int cap, int first, int reset,
                     cudaStream_t s, bool early) {
     const int64_t need = (static_cast<int64_t>(M.rows) * VW + kBlock - 1) / kBlock;
     const int grid = static_cast<int>(need < cap ? need : cap);
-    if (a.early) launch_pass(fast_iter_uniform<T, E, VW, PRIMAL, true>, grid, early, s, a, first, reset);
-    else fast_iter_uniform<T, E, VW, PRIMAL, false><<<grid, kBlock, 0, s>>>(a, first, reset);
+    auto run = [&](auto runs) {
+        constexpr bool R = decltype(runs)::value;
+        if (a.early) launch_pass(fast_iter_uniform<T, E, VW, PRIMAL, true, R>, grid, early, s, a, first, reset);
+        else fast_iter_uniform<T, E, VW, PRIMAL, false, R><<<grid, kBlock, 0, s>>>(a, first, reset);
+    };
+    if constexpr (E * VW == 2) {
+        if (M.runs != nullptr) return run(std::true_type{});
+    }
+    run(std::false_type{});
 }
 
 template <class T, bool PRIMAL, bool EARLY>
@@ -766,7 +982,8 @@ int launch_iter(const FastIter<T>& a0, int first, cudaStream_t s, const PassFork
     else if (p.slc > 0)
         fast_iter_slices<T, PRIMAL, false><<<p.slc, kBlock, 0, ss>>>(a, first, reset_slc);
     const int us = p.shrt > 0 ? uniform_slot<T>(M) : -1;
-    if (us == 0) launch_uniform<T, 2, 1, PRIMAL>(a, M, g_cap_uni[0][pi], first, reset_short, s, early);
+    if (PRIMAL && us == 0 && wide_ok(a)) launch_wide(a, g_cap_wide[pi], first, reset_short, s, early);
+    else if (us == 0) launch_uniform<T, 2, 1, PRIMAL>(a, M, g_cap_uni[0][pi], first, reset_short, s, early);
     else if (us == 1) launch_uniform<T, 4, 1, PRIMAL>(a, M, g_cap_uni[1][pi], first, reset_short, s, early);
     else if (us == 2) launch_uniform<T, 4, 2, PRIMAL>(a, M, g_cap_uni[2][pi], first, reset_short, s, early);
     else if (p.shrt > 0) {
@@ -1134,8 +1351,10 @@ template <int S>
 __device__ __forceinline__ void load_col_row(const DevCsr& M, int j, int (&c)[S], double (&v)[S]) {
     const int64_t b = static_cast<int64_t>(j) * S;
     if constexpr (S == 2) {
-        const int2 q = __ldcs(reinterpret_cast<const int2*>(M.ci + b));
         const double2 w = __ldcs(reinterpret_cast<const double2*>(M.v64 + b));
+        int2 q = M.runs != nullptr ? __ldg(M.runs + (j >> 5)) : make_int2(kNoRun, 0);
+        if (q.x != kNoRun) q = make_int2(run_col(q.x, j & 31), run_col(q.y, j & 31));
+        else q = __ldcs(reinterpret_cast<const int2*>(M.ci + b));
         c[0] = q.x;
         c[1] = q.y;
         v[0] = w.x;
@@ -1722,12 +1941,18 @@ int init_fast_kernels(int device) {
     const int l64 = resident_per_sm(fast_iter_long<double, false, 0, false, false>);
     const int s32 = resident_per_sm(fast_iter_slices<float, false, false>);
     const int s64 = resident_per_sm(fast_iter_slices<double, false, false>);
-    const int u[3][2] = {{resident_per_sm(fast_iter_uniform<float, 2, 1, true, false>),
-                          resident_per_sm(fast_iter_uniform<double, 2, 1, true, false>)},
-                         {resident_per_sm(fast_iter_uniform<float, 4, 1, true, false>),
-                          resident_per_sm(fast_iter_uniform<double, 4, 1, true, false>)},
-                         {resident_per_sm(fast_iter_uniform<float, 4, 2, true, false>),
-                          resident_per_sm(fast_iter_uniform<double, 4, 2, true, false>)}};
+    const int w[2] = {resident_per_sm(fast_primal_wide<float, false, false>),
+                      resident_per_sm(fast_primal_wide<double, false, false>)};
+    const int u[3][2] = {{resident_per_sm(fast_iter_uniform<float, 2, 1, true, false, false>),
+                          resident_per_sm(fast_iter_uniform<double, 2, 1, true, false, false>)},
+                         {resident_per_sm(fast_iter_uniform<float, 4, 1, true, false, false>),
+                          resident_per_sm(fast_iter_uniform<double, 4, 1, true, false, false>)},
+                         {resident_per_sm(fast_iter_uniform<float, 4, 2, true, false, false>),
+                          resident_per_sm(fast_iter_uniform<double, 4, 2, true, false, false>)}};
+    for (int t = 0; t < 2; ++t) {
+        if (w[t] <= 0) return 1;
+        g_cap_wide[t] = w[t] * sms;
+    }
     for (int q = 0; q < 3; ++q)
         for (int t = 0; t < 2; ++t) {
             if (u[q][t] <= 0) return 1;
