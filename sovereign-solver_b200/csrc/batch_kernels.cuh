@@ -143,15 +143,6 @@ void launch_batch_widen(const BatchView& b, const Iterates<float>& f, const Iter
                         cudaStream_t s);
 
 // ---- batch_resident.cu: instances that fit a cluster's shared memory --------
-// A matrix's rows in 16 consecutive parts of about equal work: the shares of a
-// cluster's CTAs. Part q is the rows [row[q], row[q + 1]) and the entries
-// [nz[q], nz[q + 1]), counted from the instance's first.
-constexpr int kResMaxCluster = 16;
-struct ResParts {
-    int32_t row[kResMaxCluster + 1] = {};
-    int32_t nz[kResMaxCluster + 1] = {};
-    int32_t longest = 0;  // entries of the longest row of at most kLongRow
-};
 // Instances that run on like clusters: `count` of the list from `first` on.
 struct ResClass {
     int size = 1, threads = 1024;

@@ -31,12 +31,8 @@ constexpr int K = kBatchCheckVals;
 // kResRowWork per row), one thread per boundary, each a multiple of four rows
 // (whole 16-byte vectors of the row vectors).
 constexpr int64_t kResRowWork = 8;
-__global__ void __launch_bounds__(kBlock) k_batch_parts(const int32_t* rp0, const int32_t* off, int which,
-                                                        ResParts* out) {
-    const int k = blockIdx.x, q = threadIdx.x;
-    const int32_t* rp = rp0 + off[k];
-    const int32_t rows = off[k + 1] - off[k];
-    ResParts& o = out[2 * k + which];
+__device__ void row_parts(const int32_t* rp, int32_t rows, ResParts& o) {
+    const int q = threadIdx.x;
     int longest = 0;
     for (int i = q; i < rows; i += kBlock) {
         const int len = rp[i + 1] - rp[i];
@@ -60,6 +56,14 @@ __global__ void __launch_bounds__(kBlock) k_batch_parts(const int32_t* rp0, cons
     if (q < kResMaxCluster) lo &= ~3;
     o.row[q] = lo;
     o.nz[q] = static_cast<int32_t>(rp[lo] - base);
+}
+__global__ void __launch_bounds__(kBlock) k_parts(const int32_t* rp, int32_t rows, ResParts* out) {
+    row_parts(rp, rows, *out);
+}
+__global__ void __launch_bounds__(kBlock) k_batch_parts(const int32_t* rp, const int32_t* off, int which,
+                                                        ResParts* out) {
+    const int k = blockIdx.x;
+    row_parts(rp + off[k], off[k + 1] - off[k], out[2 * k + which]);
 }
 
 // Block maxima (values 0..7) and sums (8..15), the warps' results combined in
@@ -289,7 +293,7 @@ int g_res_cluster = 0;
 
 }  // namespace
 
-int init_resident_kernels() {
+void init_resident_kernels() {
     const int c[8] = {res_largest_cluster(batch_resident<float, 1024, false>, 1024),
                       res_largest_cluster(batch_resident<double, 1024, false>, 1024),
                       res_largest_cluster(batch_resident<float, 1024, true>, 1024),
@@ -298,9 +302,11 @@ int init_resident_kernels() {
                       res_largest_cluster(batch_resident<double, 512, false>, 512),
                       res_largest_cluster(batch_resident<float, 256, false>, 256),
                       res_largest_cluster(batch_resident<double, 256, false>, 256)};
-    if (*std::min_element(c, c + 8) == 0) return 1;
-    g_res_cluster = *std::min_element(c, c + 4);
-    return 0;
+    g_res_cluster = *std::min_element(c, c + 8) == 0 ? 0 : *std::min_element(c, c + 4);
+}
+
+void launch_parts(const int32_t* rp, int32_t rows, ResParts* out, cudaStream_t s) {
+    k_parts<<<1, kBlock, 0, s>>>(rp, rows, out);
 }
 
 void launch_batch_parts(const BatchView& b, ResParts* parts, cudaStream_t s) {

@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -127,6 +128,7 @@ struct MatDev {
     int64_t nnz_dense = 0;  // entries of the dense rows (columns computed)
     DBuf<int2> runs;        // column runs of rows of two entries, if in use
     int64_t nnz_runs = 0;   // entries whose columns they give
+    ResParts parts;         // of at most kResPartRows rows (else empty)
     DevCsr view() const {
         DevCsr d;
         d.rows = rows;
@@ -276,17 +278,22 @@ inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err) {
         (e = M.warp_rows1.alloc(static_cast<size_t>(M.rows) + 1)) != cudaSuccess)
         return cuda_fail(err, e, "bin_matrix");
     DBuf<unsigned long long> cnt;
-    if ((e = cnt.alloc(9)) != cudaSuccess) return cuda_fail(err, e, "bin_matrix");
+    constexpr size_t kPartWords = (sizeof(ResParts) + 7) / 8;  // the parts travel with the counters
+    if ((e = cnt.alloc(9 + kPartWords)) != cudaSuccess) return cuda_fail(err, e, "bin_matrix");
     cudaMemsetAsync(cnt.p, 0, 9 * sizeof(unsigned long long), s);
+    const bool parts = M.rows > 0 && M.rows <= kResPartRows;
+    if (parts) launch_parts(M.rp.p, M.rows, reinterpret_cast<ResParts*>(cnt.p + 9), s);
     launch_bin(M.rp.p, M.rows, kLongRow, M.long_rows.p, cnt.p, s);
     launch_bin(M.rp.p, M.rows, kWarpRow, M.wrows.p, cnt.p + 3, s);
     // rows all of one length: the short-row kernel computes their extents
     launch_uniform_rows(M.rp.p, M.rows, reinterpret_cast<unsigned*>(cnt.p + 8), s);
     int32_t rp01[2] = {0, 0};
     if (M.rows > 0) cudaMemcpyAsync(rp01, M.rp.p, sizeof rp01, cudaMemcpyDeviceToHost, s);
-    unsigned long long h[9];
-    cudaMemcpyAsync(h, cnt.p, sizeof h, cudaMemcpyDeviceToHost, s);
+    unsigned long long h[9 + kPartWords];
+    cudaMemcpyAsync(h, cnt.p, sizeof(h[0]) * (parts ? 9 + kPartWords : 9), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(err, e, "bin_matrix");
+    M.parts = ResParts{};
+    if (parts) std::memcpy(&M.parts, h + 9, sizeof M.parts);
     M.n_long = static_cast<int32_t>(h[0]);
     M.n_short = static_cast<int32_t>(h[1]);
     M.n_wrows = static_cast<int32_t>(h[3]);
@@ -300,7 +307,7 @@ inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err) {
     M.short_max = std::min(kLongRow, std::max(kWarpRow, 16 * w));
     launch_bin_range(M.rp.p, M.rows, M.short_max, kLongRow, M.warp_rows0.p, cnt.p + 6, s);
     launch_bin_range(M.rp.p, M.rows, M.short_max, kHugeRow, M.warp_rows1.p, cnt.p + 7, s);
-    cudaMemcpyAsync(h, cnt.p, sizeof h, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(h, cnt.p, 9 * sizeof(h[0]), cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(err, e, "bin_matrix");
     M.n_warp0 = static_cast<int32_t>(h[6]);
     M.n_warp1 = static_cast<int32_t>(h[7]);

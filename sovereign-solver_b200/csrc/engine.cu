@@ -484,6 +484,7 @@ struct Launcher {
     FastIter<double> fi64;
     FastCheck<float> fc32;
     FastCheck<double> fc64;
+    ExactPlan one{};  // FP64-exact: the cluster that runs a period's iterations, if one holds the LP
 
     // iteration t of a check period (t = 0 first): the Halpern weight uses t;
     // tz: a check or the final selection reads this iteration's T(z)
@@ -510,6 +511,15 @@ struct Launcher {
             c.launches += launch_fast_dual(fi64, first, s, &c.fork, one);
         }
     }
+    // iterations 0 .. count - 1 of a check period, the last one storing T(z)
+    void iterations(long long count, cudaStream_t s) {
+        if (one.size > 0) {
+            launch_exact_resident(ei, one, c.ATs.parts, c.As.parts, count, s);
+            c.launches += 1;
+            return;
+        }
+        for (long long t = 0; t < count; ++t) iteration(t, s, t == count - 1);
+    }
     void check(long long period, cudaStream_t s) {
         if (prec == PDHG_PREC_FP64_EXACT) {
             ec.period_iters = period;
@@ -531,6 +541,7 @@ struct Launcher {
     long long launches_per_period(long long period) const {
         const long long chk =
             prec == PDHG_PREC_FP64_EXACT ? 3 : 2 + (fc32.want_candidate ? 1 : 0) + fc32.infeas;
+        if (one.size > 0) return 1 + chk;
         long long per_iter = 2;
         long long clear = 0;  // the flag reset when the primal pass has no rows
         if (prec != PDHG_PREC_FP64_EXACT) {
@@ -555,6 +566,8 @@ void apply_tuning(const Ctx::Tuning& t, FastIter<T>& fi) {
 
 Launcher make_launcher(Ctx& c, int prec, const pdhg_options& o, bool want_candidate) {
     Launcher L{c, prec, {}, {}, {}, {}, {}, {}};
+    if (prec == PDHG_PREC_FP64_EXACT && c.As.n_long + c.ATs.n_long == 0)
+        L.one = plan_exact_resident(c.ATs.parts, c.As.parts, std::max(c.ATs.parts.longest, c.As.parts.longest));
     const DevProblem P = c.problem();
     const double bt = o.tolerance > 1e-6 ? o.tolerance : 1e-6;
     L.ei = ExactIter{c.As.view(), c.ATs.view(), P, iterates<double>(c), c.st.p};
@@ -618,7 +631,7 @@ int build_graph(Ctx& c, Launcher& L, long long period, const GraphSig& sig) {
     cudaGraph_t g = nullptr;
     const long long before = c.launches;
     CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-    for (long long t = 0; t < period; ++t) L.iteration(t, c.stream, t == period - 1);
+    L.iterations(period, c.stream);
     L.check(period, c.stream);
     cudaError_t e = cudaStreamEndCapture(c.stream, &g);
     c.launches = before;
@@ -841,8 +854,10 @@ int run_loop(Ctx& c, Launcher& L, const pdhg_options& o, long long budget, long 
     if (!done && tail > 0 && !stop_sent) {
         poll_stop();
         if (!stop_sent) {
-            for (long long t = 0; t < tail; ++t) {
-                L.iteration(t, c.stream, t == tail - 1, iter0 + n_periods * period >= o.trace_iters);
+            const bool trace = iter0 + n_periods * period < o.trace_iters;
+            if (!trace) L.iterations(tail, c.stream);
+            for (long long t = 0; trace && t < tail; ++t) {
+                L.iteration(t, c.stream, t == tail - 1, false);
                 const long long k = iter0 + n_periods * period + t;
                 if (k < o.trace_iters) {
                     int rc = trace_copy(c, L.prec, k, o);
@@ -1671,7 +1686,9 @@ int pdhg_create(int device, pdhg_ctx** out) {
     if (cudaSetDevice(device) != cudaSuccess) return PDHG_ERR_BACKEND;
     cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device);
     if (c.sm_count <= 0) c.sm_count = 148;
-    if (pdhg::init_fast_kernels(device) != 0 || pdhg::init_resident_kernels() != 0) return PDHG_ERR_BACKEND;
+    if (pdhg::init_fast_kernels(device) != 0) return PDHG_ERR_BACKEND;
+    pdhg::init_resident_kernels();
+    pdhg::init_exact_resident();
     if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c.fork.side[0], cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c.fork.side[1], cudaStreamNonBlocking) != cudaSuccess ||

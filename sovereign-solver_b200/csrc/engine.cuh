@@ -87,6 +87,19 @@ struct LongTiers {
     RowItems items_long, items_huge, items_warp;
 };
 
+// A matrix's rows in 16 consecutive parts of about equal work: the shares of a
+// cluster's CTAs. Part q is the rows [row[q], row[q + 1]) and the entries
+// [nz[q], nz[q + 1]), counted from the matrix's (an instance's) first.
+constexpr int kResMaxCluster = 16;
+struct ResParts {
+    int32_t row[kResMaxCluster + 1] = {};
+    int32_t nz[kResMaxCluster + 1] = {};
+    int32_t longest = 0;  // entries of the longest row of at most kLongRow
+};
+// ... of one matrix, of at most kResPartRows rows (batch_resident.cu).
+constexpr int32_t kResPartRows = 16384;
+void launch_parts(const int32_t* rp, int32_t rows, ResParts* out, cudaStream_t s);
+
 struct DevCsr {
     int32_t rows = 0, cols = 0;
     int64_t nnz = 0;
@@ -537,7 +550,20 @@ void launch_norms(int32_t m, int32_t n, const double* c_s, const double* rlo_s,
 // Inclusive prefix sum of n int32 counts into out[1..n], out[0] = 0 (CUB).
 int prefix_rows(const int32_t* cnt, int32_t n, int32_t* out, cudaStream_t s);
 
-int init_resident_kernels();  // batch_resident.cu: once per device; 0 on success
+void init_resident_kernels();  // batch_resident.cu: once per device
+
+// ---- exact_resident.cu: a small LP's iterations on one cluster ---------------
+void init_exact_resident();  // once per device
+struct ExactPlan {
+    int size = 0, threads = 0;  // CTAs of the cluster (0: the LP runs as passes)
+    uint32_t smem = 0;
+};
+// pt, pa: the parts of A^T's and of A's rows; longest: entries of the longest
+// row of either.
+ExactPlan plan_exact_resident(const ResParts& pt, const ResParts& pa, int longest);
+// Iterations 0 .. iters - 1 of a check period.
+void launch_exact_resident(const ExactIter& a, const ExactPlan& p, const ResParts& pt, const ResParts& pa,
+                           long long iters, cudaStream_t s);
 
 // The batched engine (batch.cu), owned by a context: it uses the context's
 // stream and writes its errors into the context's error text.
