@@ -80,6 +80,7 @@ struct BatchCtx {
     } plan[2][2];  // [FP32, FP64][averaged, Halpern]
     DBuf<unsigned char> far;  // entries of instances too large for shared memory, set up by each solve
     ResStreams side;
+    bool resident_ready[2] = {false, false};  // [FP32, FP64]
     Downloads downloads;
 
     // solve graphs, [0] FP32 and [1] FP64, with what they bake in
@@ -325,7 +326,8 @@ int batch_intake(BatchCtx& c, const pdhg_options& o) {
     launch_batch_norms(b, s);
     c.parts.resize(2 * static_cast<size_t>(c.count));
     BCK(c.parts_d.alloc(c.parts.size()));
-    launch_batch_parts(b, c.parts_d.p, s);
+    launch_batch_parts(b.AT.rp, b.col_off, b.count, 0, c.parts_d.p, s);
+    launch_batch_parts(b.A.rp, b.row_off, b.count, 1, c.parts_d.p, s);
     BCK(cudaMemcpyAsync(c.parts.data(), c.parts_d.p, sizeof(ResParts) * c.parts.size(), cudaMemcpyDeviceToHost, s));
     BCK(cudaStreamSynchronize(s));
     for (auto& f : c.plan)
@@ -633,6 +635,9 @@ int batch_plan(BatchCtx& c, BatchCtx::Plan** out) {
     BatchCtx::Plan& pl = c.plan[std::is_same<T, float>::value ? 0 : 1][c.halpern ? 1 : 0];
     *out = &pl;
     if (pl.made) return PDHG_OK;
+    bool& ready = c.resident_ready[std::is_same<T, float>::value ? 0 : 1];
+    if (!ready) init_resident_kernels<T>();
+    ready = true;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     ResPlan r;

@@ -174,7 +174,6 @@ struct ResStreams {
     cudaStream_t stream[kResClasses - 1] = {};
     cudaEvent_t fork = nullptr, join[kResClasses - 1] = {};
 };
-void launch_batch_parts(const BatchView& b, ResParts* parts, cudaStream_t s);  // 2 per instance
 // False where some instance fits no cluster in precision T. lgt, lga: log2 of
 // the lanes per row of A^T's and of A's rows.
 template <class T>

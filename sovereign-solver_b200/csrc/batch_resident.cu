@@ -15,6 +15,7 @@
 // 2,009 -> 1,173 us. 1,024 threads at 64 registers or 512 at
 // 128 for the large classes: within 10% of each other either way.
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "batch_device.cuh"
@@ -26,45 +27,6 @@ namespace pdhg {
 namespace {
 
 constexpr int K = kBatchCheckVals;
-
-// Rows of a matrix in kResMaxCluster parts of about equal work (entries plus
-// kResRowWork per row), one thread per boundary, each a multiple of four rows
-// (whole 16-byte vectors of the row vectors).
-constexpr int64_t kResRowWork = 8;
-__device__ void row_parts(const int32_t* rp, int32_t rows, ResParts& o) {
-    const int q = threadIdx.x;
-    int longest = 0;
-    for (int i = q; i < rows; i += kBlock) {
-        const int len = rp[i + 1] - rp[i];
-        if (len <= kLongRow) longest = max(longest, len);
-    }
-    __shared__ int most;
-    if (q == 0) most = 0;
-    __syncthreads();
-    atomicMax(&most, longest);
-    __syncthreads();
-    if (q == 0) o.longest = most;
-    if (q > kResMaxCluster) return;
-    const int64_t base = rp[0];
-    const int64_t want = (rp[rows] - base + kResRowWork * rows) * q / kResMaxCluster;
-    int lo = 0, hi = rows;  // the first row whose work before it reaches `want`
-    while (lo < hi) {
-        const int mid = (lo + hi) / 2;
-        if (rp[mid] - base + kResRowWork * mid < want) lo = mid + 1;
-        else hi = mid;
-    }
-    if (q < kResMaxCluster) lo &= ~3;
-    o.row[q] = lo;
-    o.nz[q] = static_cast<int32_t>(rp[lo] - base);
-}
-__global__ void __launch_bounds__(kBlock) k_parts(const int32_t* rp, int32_t rows, ResParts* out) {
-    row_parts(rp, rows, *out);
-}
-__global__ void __launch_bounds__(kBlock) k_batch_parts(const int32_t* rp, const int32_t* off, int which,
-                                                        ResParts* out) {
-    const int k = blockIdx.x;
-    row_parts(rp + off[k], off[k + 1] - off[k], out[2 * k + which]);
-}
 
 // Block maxima (values 0..7) and sums (8..15), the warps' results combined in
 // warp order: thread q < K gets value q.
@@ -288,32 +250,27 @@ cudaError_t launch_class(const ResClass& c, const BatchView& b, const Iterates<T
     return run(batch_resident<T, 1024, false>);
 }
 
-// The largest cluster the device schedules at the largest shared memory.
-int g_res_cluster = 0;
+// The largest cluster the device schedules at the largest shared memory, FP32
+// and FP64.
+std::atomic<int> g_res_cluster[2];
+
+template <class T>
+int res_cluster() {
+    return g_res_cluster[std::is_same<T, float>::value ? 0 : 1].load(std::memory_order_relaxed);
+}
 
 }  // namespace
 
+template <class T>
 void init_resident_kernels() {
-    const int c[8] = {res_largest_cluster(batch_resident<float, 1024, false>, 1024),
-                      res_largest_cluster(batch_resident<double, 1024, false>, 1024),
-                      res_largest_cluster(batch_resident<float, 1024, true>, 1024),
-                      res_largest_cluster(batch_resident<double, 1024, true>, 1024),
-                      res_largest_cluster(batch_resident<float, 512, false>, 512),
-                      res_largest_cluster(batch_resident<double, 512, false>, 512),
-                      res_largest_cluster(batch_resident<float, 256, false>, 256),
-                      res_largest_cluster(batch_resident<double, 256, false>, 256)};
-    g_res_cluster = *std::min_element(c, c + 8) == 0 ? 0 : *std::min_element(c, c + 4);
+    const int c[4] = {res_largest_cluster(batch_resident<T, 1024, false>, 1024),
+                      res_largest_cluster(batch_resident<T, 1024, true>, 1024),
+                      res_largest_cluster(batch_resident<T, 512, false>, 512),
+                      res_largest_cluster(batch_resident<T, 256, false>, 256)};
+    g_res_cluster[std::is_same<T, float>::value ? 0 : 1] = *std::min_element(c, c + 4) == 0 ? 0 : std::min(c[0], c[1]);
 }
-
-void launch_parts(const int32_t* rp, int32_t rows, ResParts* out, cudaStream_t s) {
-    k_parts<<<1, kBlock, 0, s>>>(rp, rows, out);
-}
-
-void launch_batch_parts(const BatchView& b, ResParts* parts, cudaStream_t s) {
-    if (b.count == 0) return;
-    k_batch_parts<<<b.count, kBlock, 0, s>>>(b.AT.rp, b.col_off, 0, parts);
-    k_batch_parts<<<b.count, kBlock, 0, s>>>(b.A.rp, b.row_off, 1, parts);
-}
+template void init_resident_kernels<float>();
+template void init_resident_kernels<double>();
 
 // Classes of like CTAs, tried in the order of their CTAs; the largest instances
 // first (a class's launch ends with its last instance).
@@ -336,7 +293,7 @@ int res_class(const ResParts& pt, const ResParts& pa, int lgt, int lga, bool hal
     int last = -1;
     for (int c = 2; c < kResClasses; ++c) {
         const ResClass& k = kClasses[c];
-        if (k.size > g_res_cluster) continue;
+        if (k.size > res_cluster<T>()) continue;
         const ResSize y = k.far ? res_size<T, true>(pt, pa, k.size, lgt, lga, halpern)
                                 : res_size<T, false>(pt, pa, k.size, lgt, lga, halpern);
         if (y.smem > kResMaxSmem) continue;
@@ -354,7 +311,7 @@ template <class T>
 bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, int sms, ResPlan& plan) {
     plan = ResPlan{};
     const size_t count = parts.size() / 2;
-    if (g_res_cluster == 0) return false;
+    if (res_cluster<T>() == 0) return false;
     struct Item {
         int32_t k, nnz, cls;
         ResFar far;

@@ -62,6 +62,7 @@ struct Ctx {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     Downloads downloads;
+    bool exact_resident_ready = false;
     PassFork fork;  // side stream + events: short- and long-row kernels side by side
     std::string err;
     long long gen = 0;  // bumps on every load / rescale
@@ -566,6 +567,10 @@ void apply_tuning(const Ctx::Tuning& t, FastIter<T>& fi) {
 
 Launcher make_launcher(Ctx& c, int prec, const pdhg_options& o, bool want_candidate) {
     Launcher L{c, prec, {}, {}, {}, {}, {}, {}};
+    if (prec == PDHG_PREC_FP64_EXACT && !c.exact_resident_ready) {
+        init_exact_resident();
+        c.exact_resident_ready = true;
+    }
     if (prec == PDHG_PREC_FP64_EXACT && c.As.n_long + c.ATs.n_long == 0)
         L.one = plan_exact_resident(c.ATs.parts, c.As.parts, std::max(c.ATs.parts.longest, c.As.parts.longest));
     const DevProblem P = c.problem();
@@ -1687,8 +1692,6 @@ int pdhg_create(int device, pdhg_ctx** out) {
     cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device);
     if (c.sm_count <= 0) c.sm_count = 148;
     if (pdhg::init_fast_kernels(device) != 0) return PDHG_ERR_BACKEND;
-    pdhg::init_resident_kernels();
-    pdhg::init_exact_resident();
     if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c.fork.side[0], cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c.fork.side[1], cudaStreamNonBlocking) != cudaSuccess ||

@@ -96,9 +96,12 @@ struct ResParts {
     int32_t nz[kResMaxCluster + 1] = {};
     int32_t longest = 0;  // entries of the longest row of at most kLongRow
 };
-// ... of one matrix, of at most kResPartRows rows (batch_resident.cu).
+// ... of one matrix, of at most kResPartRows rows (intake.cu), and of a batch's
+// matrices, whose rows are [off[k], off[k + 1]) of rp, into out[2 k + which].
 constexpr int32_t kResPartRows = 16384;
 void launch_parts(const int32_t* rp, int32_t rows, ResParts* out, cudaStream_t s);
+void launch_batch_parts(const int32_t* rp, const int32_t* off, int32_t count, int which, ResParts* out,
+                        cudaStream_t s);
 
 struct DevCsr {
     int32_t rows = 0, cols = 0;
@@ -550,10 +553,13 @@ void launch_norms(int32_t m, int32_t n, const double* c_s, const double* rlo_s,
 // Inclusive prefix sum of n int32 counts into out[1..n], out[0] = 0 (CUB).
 int prefix_rows(const int32_t* cnt, int32_t n, int32_t* out, cudaStream_t s);
 
-void init_resident_kernels();  // batch_resident.cu: once per device
+// batch_resident.cu, exact_resident.cu: before an engine's first use of the
+// kernels (the first in a process loads them onto the device: milliseconds)
+template <class T>
+void init_resident_kernels();
 
 // ---- exact_resident.cu: a small LP's iterations on one cluster ---------------
-void init_exact_resident();  // once per device
+void init_exact_resident();
 struct ExactPlan {
     int size = 0, threads = 0;  // CTAs of the cluster (0: the LP runs as passes)
     uint32_t smem = 0;

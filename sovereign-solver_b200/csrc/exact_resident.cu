@@ -13,6 +13,7 @@
 // 7.5 -> 4.9, 2,000 x 5,000 (eight CTAs) 7.4 -> 6.0, 2,500 x 6,000 (sixteen)
 // 9.4 -> 7.2: faster wherever a cluster holds the LP.
 #include <algorithm>
+#include <atomic>
 
 #include "resident.cuh"
 
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(NT) exact_resident(ExactIter a, ResParts pt, R
 }
 
 constexpr int kFewThreads = 256, kManyThreads = 1024;
-int g_exact_cluster = 0;  // the largest cluster the device schedules
+std::atomic<int> g_exact_cluster{0};  // the largest cluster the device schedules
 
 }  // namespace
 
@@ -129,11 +130,12 @@ constexpr int64_t kExactNnz = 4096;
 ExactPlan plan_exact_resident(const ResParts& pt, const ResParts& pa, int longest) {
     ExactPlan p;
     const int64_t nnz = pa.nz[kResMaxCluster];
-    if (g_exact_cluster == 0 || pt.row[kResMaxCluster] < 1 || pa.row[kResMaxCluster] < 1 || longest > kExactRow)
+    if (pt.row[kResMaxCluster] < 1 || pa.row[kResMaxCluster] < 1 || longest > kExactRow)
         return p;
-    for (int c = 1; c <= g_exact_cluster; c *= 2) {
+    const int most = g_exact_cluster;
+    for (int c = 1; c <= most; c *= 2) {
         const ResSize z = res_size<double, false>(pt, pa, c, 0, 0, false);
-        if (z.smem > kResMaxSmem || (nnz > kExactNnz * c && 2 * c <= g_exact_cluster)) continue;
+        if (z.smem > kResMaxSmem || (nnz > kExactNnz * c && 2 * c <= most)) continue;
         p.size = c;
         p.smem = z.smem;
         p.threads = c == 1 && nnz <= 3000 ? kFewThreads : kManyThreads;

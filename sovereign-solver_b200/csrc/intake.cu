@@ -261,6 +261,45 @@ __global__ void __launch_bounds__(kBlock) k_col_runs(const int32_t* ci, int32_t 
     if (run) atomicAdd(n_run, 1ull);
 }
 
+// Rows of a matrix in kResMaxCluster parts of about equal work (entries plus
+// kResRowWork per row), one thread per boundary, each a multiple of four rows
+// (whole 16-byte vectors of the row vectors).
+constexpr int64_t kResRowWork = 8;
+__device__ void row_parts(const int32_t* rp, int32_t rows, ResParts& o) {
+    const int q = threadIdx.x;
+    int longest = 0;
+    for (int i = q; i < rows; i += kBlock) {
+        const int len = rp[i + 1] - rp[i];
+        if (len <= kLongRow) longest = max(longest, len);
+    }
+    __shared__ int most;
+    if (q == 0) most = 0;
+    __syncthreads();
+    atomicMax(&most, longest);
+    __syncthreads();
+    if (q == 0) o.longest = most;
+    if (q > kResMaxCluster) return;
+    const int64_t base = rp[0];
+    const int64_t want = (rp[rows] - base + kResRowWork * rows) * q / kResMaxCluster;
+    int lo = 0, hi = rows;  // the first row whose work before it reaches `want`
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (rp[mid] - base + kResRowWork * mid < want) lo = mid + 1;
+        else hi = mid;
+    }
+    if (q < kResMaxCluster) lo &= ~3;
+    o.row[q] = lo;
+    o.nz[q] = static_cast<int32_t>(rp[lo] - base);
+}
+__global__ void __launch_bounds__(kBlock) k_parts(const int32_t* rp, int32_t rows, ResParts* out) {
+    row_parts(rp, rows, *out);
+}
+__global__ void __launch_bounds__(kBlock) k_batch_parts(const int32_t* rp, const int32_t* off, int which,
+                                                        ResParts* out) {
+    const int k = blockIdx.x;
+    row_parts(rp + off[k], off[k + 1] - off[k], out[2 * k + which]);
+}
+
 // Rows with lo < length <= hi appended to `list` (grid-stride; one atomic per
 // warp that has any).
 __global__ void k_bin_range(const int32_t* rp, int32_t rows, int lo, int hi, int32_t* list,
@@ -573,6 +612,15 @@ void launch_row_extents(const int32_t* rows, int32_t n, const int32_t* rp, int4*
 void launch_gather_cols(const int32_t* ci, const int64_t* pos, int32_t n, int32_t* out,
                         cudaStream_t s) {
     if (n > 0) k_gather_cols<<<nblocks(n), kBlock, 0, s>>>(ci, pos, n, out);
+}
+
+void launch_parts(const int32_t* rp, int32_t rows, ResParts* out, cudaStream_t s) {
+    k_parts<<<1, kBlock, 0, s>>>(rp, rows, out);
+}
+
+void launch_batch_parts(const int32_t* rp, const int32_t* off, int32_t count, int which, ResParts* out,
+                        cudaStream_t s) {
+    if (count > 0) k_batch_parts<<<count, kBlock, 0, s>>>(rp, off, which, out);
 }
 
 void launch_col_runs(const int32_t* ci, int32_t rows, int2* runs, unsigned long long* n_run, cudaStream_t s) {
