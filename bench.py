@@ -789,7 +789,8 @@ def main() -> None:
     generic = 4 * (rows + 1) + 8 * nnz + 4 * cols + 4 * touches * rows
     roofline = {"bound": "hbm", "kernel": dom["name"], "achieved": achieved,
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
-                "peak_source": peaks["source"], "traffic": traffic_from_profile(),
+                "peak_source": peaks["source"],
+                "traffic": traffic_from_profile() if dom["name"] == "primal" else None,
                 "algorithmic_bytes_per_launch": dom["bytes"],
                 "bytes_note": "this LP's: the row pointer (every column has 2 entries) and the "
                               "column bounds (all 0 <= x) carry no information and are not loaded",
