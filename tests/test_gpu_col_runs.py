@@ -1,6 +1,8 @@
 """Columns of two entries given by runs (intake.cu k_col_runs) on the wide
 primal pass (kernels_fast.cu fast_primal_wide) and in the check, against the
 passes that load every column index: the same arithmetic, so the same bits.
+(The points' bits: the check's sums over the LP take a split row's terms in the
+CTA that completes the row, so their last bits vary from run to run.)
 Sizes: fewer columns than a vector or a run, remainders of both, runs broken by
 a row's end and by shuffled columns, launched early and not (4M entries)."""
 import numpy as np
@@ -40,4 +42,4 @@ def test_runs_give_the_loaded_columns_bits(pkg, monkeypatch, m, n, boxed, shuffl
                     got.append(e.solve(opt))
             np.testing.assert_array_equal(got[0].primal, got[1].primal)
             np.testing.assert_array_equal(got[0].dual, got[1].dual)
-            assert got[0].relative_kkt == got[1].relative_kkt and got[0].restarts == got[1].restarts
+            assert got[0].restarts == got[1].restarts
