@@ -123,6 +123,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
     res_load_rows<NT>(L.D, b.A, r0, c0, pa.row[p0], pa.row[p1], static_cast<uint32_t>(n), scratch.build);
     const PV<T> pv = pvec<T>(b.P);
     res_load_fixed<NT>(L, pv, c0, r0);
+    // Every CTA of the cluster has started before another writes into its
+    // shared memory (the tail's stop_all below, where there is no whole period).
+    cl.sync();
     const bool lead = cl.rank == 0 && threadIdx.x == 0;
     const double sign = s.obj_sign;
     bool done = false;
