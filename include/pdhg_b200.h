@@ -227,7 +227,12 @@ int pdhg_solve(pdhg_ctx* ctx, const pdhg_options* options, pdhg_info* info, doub
  * stacking cannot hold (offsets, a column outside the instance) returns
  * PDHG_ERR_INVALID_ARGUMENT. Precision MIXED or FP64 only; no checkpoint and
  * no trace. x, y, rc are stacked like the inputs (any may be NULL); infos has
- * `count` entries. A loaded batch stays on the context beside the single LP. */
+ * `count` entries. A loaded batch stays on the context beside the single LP.
+ * Instances need not advance together: where they run on clusters, each takes
+ * its place when an earlier one ends. A time limit or cancellation ends those
+ * that run at their next check and those that still wait without an iteration;
+ * one already past its last check runs the few iterations left to
+ * max_iterations and reports PDHG_STATUS_ITERATION_LIMIT. */
 int pdhg_load_batch(pdhg_ctx* ctx, int32_t count, const int32_t* row_off,
                     const int32_t* col_off, int64_t nnz, const int32_t* row_ptr,
                     const int32_t* col_idx, const double* values, const double* c,

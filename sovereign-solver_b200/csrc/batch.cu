@@ -724,12 +724,6 @@ int batch_run(BatchCtx& c, const pdhg_options& o, std::chrono::steady_clock::tim
                                      batch_iterates<T>(c), p, iter0, n_periods, tail, s, c.side));
         *launches += static_cast<long long>(plan->classes.size());
         if (int rc = wait(); rc != PDHG_OK) return rc;
-        BatchGlobal gh;
-        BCK(cudaMemcpy(&gh, c.g.p, sizeof gh, cudaMemcpyDeviceToHost));
-        if (!gh.done && tail > 0 && !stop_sent) {
-            gh.iter += tail;
-            BCK(cudaMemcpy(c.g.p, &gh, sizeof gh, cudaMemcpyHostToDevice));
-        }
         return stop_sent ? -c.mail->stop_request : PDHG_OK;
     }
     launch_batch_compact(c.view(), s);  // the block lists of the instances now active
@@ -852,7 +846,7 @@ int batch_solve(BatchCtx& c, const pdhg_options& o, pdhg_info* infos, double* x,
         st.res_last = st.res_prev_cand = kInfB;
         st.cur_res = st.avg_res = st.orig_res = st.rel_kkt = 0.0;
         st.inv = 1.0;
-        st.stalled = st.polished = 0;
+        st.stalled = st.polished = st.spent = 0;
         st.since_improve = st.switch_iter = st.idle = 0;
         st.best_res = kInfB;
         if (!c.have_opnorm || c.opnorm_iters != o.power_iterations) {
@@ -1022,7 +1016,7 @@ int batch_solve(BatchCtx& c, const pdhg_options& o, pdhg_info* infos, double* x,
             inf.status = PDHG_STATUS_ITERATION_LIMIT;
             inf.iterations = st.stop_iter;
         } else {
-            inf.status = stop != 0 ? stop : PDHG_STATUS_ITERATION_LIMIT;
+            inf.status = stop != 0 && !st.spent ? stop : PDHG_STATUS_ITERATION_LIMIT;
             inf.iterations = g2.iter;
         }
         if (st.polished) inf.iterations -= st.idle;  // this instance's own iterations

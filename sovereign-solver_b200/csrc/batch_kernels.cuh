@@ -29,6 +29,7 @@ struct InstState {
     int restart, restart_to_avg, avg_better, fold;
     int fail_kind, ruiz_done, pw_done, valid;
     int stalled, polished;  // mixed mode: FP32 phase stopped improving / finished in FP64
+    int spent;              // on a cluster: ran all iterations asked for
     long long since_restart, restarts, stop_iter;
     long long since_improve, switch_iter;
     long long idle;  // global iterations a stalled instance waited for the FP64 phase

@@ -104,6 +104,29 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
     const int k = job.list[blockIdx.x / static_cast<unsigned>(cl.size)];
     InstState& s = b.is[k];
     if (s.done) return;  // the same for the cluster's CTAs, which alone run this instance
+    const bool lead = cl.rank == 0 && threadIdx.x == 0;
+    // A stop request, to the whole cluster. (No CTA writes into another's shared
+    // memory before a barrier has shown that it has started.)
+    const auto stop_requested = [&]() -> int {
+        cl.sync();
+        if (lead) {
+            const int stop = b.mail != nullptr ? b.mail->stop_request : 0;
+            for (int c = 0; c < cl.size; ++c) *cg::this_cluster().map_shared_rank(&stop_all, c) = stop;
+        }
+        cl.sync();
+        return stop_all;
+    };
+    // ends the instance where it is, `iters` iterations done
+    const auto stop_here = [&](int stop, long long iters) {
+        if (!lead) return;
+        s.done = 1;
+        s.status = stop;
+        s.stop_iter = iters;
+        atomicMax(&b.g->iter, iters);
+        finish_instance(b, s);
+    };
+    // one that came while the instance waited for its cluster
+    if (const int stop = stop_requested(); stop != 0) return stop_here(stop, iter0);
     const int c0 = b.col_off[k], r0 = b.row_off[k];
     const int n = b.col_off[k + 1] - c0, m = b.row_off[k + 1] - r0;
     const ResParts &pt = job.parts[2 * k], &pa = job.parts[2 * k + 1];
@@ -123,10 +146,6 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
     res_load_rows<NT>(L.D, b.A, r0, c0, pa.row[p0], pa.row[p1], static_cast<uint32_t>(n), scratch.build);
     const PV<T> pv = pvec<T>(b.P);
     res_load_fixed<NT>(L, pv, c0, r0);
-    // Every CTA of the cluster has started before another writes into its
-    // shared memory (the tail's stop_all below, where there is no whole period).
-    cl.sync();
-    const bool lead = cl.rank == 0 && threadIdx.x == 0;
     const double sign = s.obj_sign;
     bool done = false;
     long long periods = 0;
@@ -135,13 +154,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
     // FP64 500 x 1,200 instances 4.8 -> 8.5 us an iteration)
     for (bool checked = n_periods > 0; !done; checked = periods < n_periods) {
         const long long count = checked ? p.period : tail;
-        // read ahead of the period, so that nobody waits for the host's memory
-        int stop = lead && b.mail != nullptr ? b.mail->stop_request : 0;
         if (!checked) {
-            if (lead)
-                for (int c = 0; c < cl.size; ++c) *cg::this_cluster().map_shared_rank(&stop_all, c) = stop;
-            cl.sync();
-            if (count == 0 || stop_all != 0) break;
+            if (count == 0) break;
+            if (periods > 0)
+                if (const int stop = stop_requested(); stop != 0) return stop_here(stop, iter0 + periods * p.period);
         }
         res_load_iterates<NT>(L, it, c0, r0);
         ResStep<T> step;
@@ -158,6 +174,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
         const long long iter = iter0 + periods * p.period;
         ++periods;
         // ---- check
+        // read ahead of its products, so that nobody waits for the host's memory
+        const int stop = lead && b.mail != nullptr ? b.mail->stop_request : 0;
         const double inv = it.halpern ? 1.0 : 1.0 / static_cast<double>(s.since_restart + p.period);
         Terms t;
         if (it.halpern) {
@@ -236,7 +254,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
     if (lead) {
         // as the period count of the kernels over all instances: the period in
         // which the last instance ends is not counted
-        atomicMax(&b.g->iter, iter0 + (periods - (done ? 1 : 0)) * p.period);
+        s.spent = done ? 0 : 1;
+        atomicMax(&b.g->iter, iter0 + (done ? (periods - 1) * p.period : periods * p.period + tail));
         atomicMax(&b.g->checks, periods);
     }
 }
