@@ -122,7 +122,6 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(const __grid_constant_
     __shared__ double loss_part[kGemmThreads / 32];
     constexpr int kA = tc::kTileM * tc::kTileK, kB = BN * tc::kTileK;
     bf16* const slices = reinterpret_cast<bf16*>(dyn);  // A's and B's of stage 0, of stage 1, ...
-    pass_begin();
     const bool second = static_cast<int>(blockIdx.x) >= pair.tiles0;
     const GemmArgs& g = pair.g[second ? 1 : 0];
     const int tile = static_cast<int>(blockIdx.x) - (second ? pair.tiles0 : 0);
@@ -141,6 +140,10 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(const __grid_constant_
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    // The next launch may start only now that this CTA holds its TMEM columns:
+    // its CTAs take columns and then wait for this grid, so one of this grid's
+    // that still waited for columns beside them would never get any.
+    pass_begin();
     const uint32_t tmem = tmem_base;
     constexpr uint32_t idesc = tc::instr_desc_bf16(BN);
     const uint32_t base = tc::smem_u32(slices);
