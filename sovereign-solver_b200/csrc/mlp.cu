@@ -331,12 +331,14 @@ __global__ void k_to_bf16(const float* in, bf16* out, int64_t n) {
 }
 
 // Rows idx[0..B) (idx null: 0..B) of src (S x d, FP32) in BF16: dst (B x d)
-// and, unless null, its transposed copy (d x B). 32 x 32 tiles.
+// and, unless null, its transposed copy (d x B). 32 x 32 tiles, all along the
+// grid's x: of rows or of inputs there may be more than its y takes (65,535).
 __global__ void k_gather_rows(const float* src, int d, const int32_t* idx, int B, bf16* dst, bf16* dst_t) {
     __shared__ bf16 t[32][33];
     pass_begin();
     pass_wait();
-    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+    const int rb = (B + 31) / 32;
+    const int r0 = static_cast<int>(blockIdx.x) % rb * 32, c0 = static_cast<int>(blockIdx.x) / rb * 32;
     const int c = c0 + threadIdx.x;
     for (int i = threadIdx.y; i < 32; i += 8) {
         const int r = r0 + i;
@@ -666,7 +668,7 @@ int backward(Mlp& h, int B, double* loss) {
 
 // The batch's inputs (rows idx, null: in order) in BF16, transposed too for a gradient.
 int set_batch(Mlp& h, int B, const float* x, const int32_t* idx, bool gradient) {
-    k_gather_rows<<<dim3(blocks(h.n_in, 32), blocks(B, 32)), dim3(32, 8), 0, h.stream>>>(
+    k_gather_rows<<<blocks(B, 32) * blocks(h.n_in, 32), dim3(32, 8), 0, h.stream>>>(
         x, h.n_in, idx, B, h.x16.p, gradient ? h.xt.p : nullptr);
     MCK(cudaGetLastError());
     return PDHG_OK;
