@@ -88,18 +88,27 @@ struct ResJob {
     unsigned char* far;
 };
 
+// The kernel's static shared memory.
+template <class T, int NT>
+struct BatchShared {
+    union {
+        ResBuild build;
+        double sum[2][kBlock];
+    } scratch;
+    double red[K][NT / 32];
+    double part[kResMaxCluster][K];  // rank 0: the CTAs' values
+    T weights[kResWeights];
+    int stop_all;
+};
+
 template <class T, int NT, bool FAR>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
     batch_resident(BatchView b, Iterates<T> it, BatchParams p, ResJob job, long long iter0, long long n_periods,
                    long long tail) {
-    __shared__ T weights[kResWeights];
-    __shared__ union {
-        ResBuild build;
-        double sum[2][kBlock];
-    } scratch;
-    __shared__ double red[K][NT / 32];
-    __shared__ double part[kResMaxCluster][K];  // rank 0: the CTAs' values
-    __shared__ int stop_all;
+    __shared__ BatchShared<T, NT> sh;
+    static_assert(sizeof(sh) <= kResStaticSmem, "beside kResMaxSmem of dynamic shared memory");
+    auto& scratch = sh.scratch;
+    auto& part = sh.part;
     const ResCluster cl;
     const int k = job.list[blockIdx.x / static_cast<unsigned>(cl.size)];
     InstState& s = b.is[k];
@@ -111,10 +120,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
         cl.sync();
         if (lead) {
             const int stop = b.mail != nullptr ? b.mail->stop_request : 0;
-            for (int c = 0; c < cl.size; ++c) *cg::this_cluster().map_shared_rank(&stop_all, c) = stop;
+            for (int c = 0; c < cl.size; ++c) *cg::this_cluster().map_shared_rank(&sh.stop_all, c) = stop;
         }
         cl.sync();
-        return stop_all;
+        return sh.stop_all;
     };
     // ends the instance where it is, `iters` iterations done
     const auto stop_here = [&](int stop, long long iters) {
@@ -166,8 +175,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
         const long long since = s.since_restart;
         const bool fresh = s.fresh != 0;
         cl.sync();  // every CTA has its copies before a neighbour writes into them
-        if (it.halpern) res_iterate<NT, T, true>(L, cl, step, it, since, count, fresh, weights);
-        else res_iterate<NT, T, false>(L, cl, step, it, since, count, fresh, weights);
+        if (it.halpern) res_iterate<NT, T, true>(L, cl, step, it, since, count, fresh, sh.weights);
+        else res_iterate<NT, T, false>(L, cl, step, it, since, count, fresh, sh.weights);
         res_store_iterates<NT>(L, it, c0, r0);
         cl.sync();  // the stored vectors, seen by the whole cluster
         if (!checked) break;
@@ -188,7 +197,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
         __syncwarp();
         const double v[K] = {t.cp,     t.cd,     t.ap,     t.ad,     t.ocp, t.ocd, t.oap, t.oad,
                              t.pobj_c, t.dobj_c, t.pobj_a, t.dobj_a, t.ppc, t.ddc, t.ppa, t.dda};
-        const double mine = reduce_vals<NT>(v, red);
+        const double mine = reduce_vals<NT>(v, sh.red);
         if (threadIdx.x < K) *cg::this_cluster().map_shared_rank(&part[cl.rank][threadIdx.x], 0) = mine;
         cl.sync();
         if (lead) {  // merged in rank order

@@ -85,6 +85,7 @@ __device__ __forceinline__ void exact_pass(const ResSlab<double, false>& S, uint
 template <int NT>
 __global__ void __launch_bounds__(NT) exact_resident(ExactIter a, ResParts pt, ResParts pa, long long iters) {
     __shared__ ResBuild build;
+    static_assert(sizeof(build) <= kResStaticSmem, "beside kResMaxSmem of dynamic shared memory");
     DevState* st = a.st;
     if (st->done) return;  // written by the check kernels only: the same for every CTA
     const ResCluster cl;

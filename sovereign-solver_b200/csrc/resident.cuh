@@ -36,8 +36,12 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-// Dynamic shared memory a CTA may have; the kernels' static part is below 8 KB.
+// Dynamic shared memory a CTA may have, beside the kernels' static part (up to
+// 10.6 KB): together the 227 KB of a block. Past that no cluster could be
+// scheduled (res_largest_cluster), and every LP would take the slower kernels;
+// so each kernel asserts its part.
 constexpr uint32_t kResMaxSmem = 216 * 1024;
+constexpr uint32_t kResStaticSmem = 227 * 1024 - kResMaxSmem;
 constexpr int kResWeights = 64;    // Halpern weights tabulated at a time
 
 __host__ __device__ constexpr uint32_t res_align(uint32_t b) { return (b + 15u) / 16u * 16u; }
