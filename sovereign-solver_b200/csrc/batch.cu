@@ -67,7 +67,7 @@ struct BatchCtx {
     DBuf<double> xa64, sa64, ya64;
     DBuf<float> xa32, sa32, ya32;
 
-    // instances on clusters (batch_resident.cu): their parts, and the plan per
+    // instances on clusters (batch_resident.cuh): their parts, and the plan per
     // precision and form made since the load
     DBuf<ResParts> parts_d;
     std::vector<ResParts> parts;

@@ -1,6 +1,6 @@
 // batch_device.cuh -- an instance's check terms, decision and restart, shared
 // by the batched kernels over all instances (batch_kernels.cu) and the kernel
-// that runs an instance on one cluster (batch_resident.cu).
+// that runs an instance on one cluster (batch_resident.cuh).
 #pragma once
 
 #include <cmath>

@@ -143,7 +143,7 @@ constexpr int kBatchStalled = 100;
 void launch_batch_widen(const BatchView& b, const Iterates<float>& f, const Iterates<double>& d,
                         cudaStream_t s);
 
-// ---- batch_resident.cu: instances that fit a cluster's shared memory --------
+// ---- batch_resident.cuh: instances that fit a cluster's shared memory --------
 // Instances that run on like clusters: `count` of the list from `first` on.
 struct ResClass {
     int size = 1, threads = 1024;

@@ -1,4 +1,4 @@
-// batch_resident.cu -- a batch whose instances fit the shared memory of a
+// batch_resident.cuh -- a batch whose instances fit the shared memory of a
 // cluster each: one cluster runs one instance's whole solve (resident.cuh),
 // every check period of it with the check, the decision and the restart, and
 // the next instance takes its place. No instance waits for another: an
@@ -14,6 +14,11 @@
 // period of 40 iterations 519 -> 205 us; 256 FP32 instances of 50 to 5,000 rows
 // 2,009 -> 1,173 us. 1,024 threads at 64 registers or 512 at
 // 128 for the large classes: within 10% of each other either way.
+//
+// A translation unit per precision (batch_resident_f32.cu, _f64.cu): the first
+// kernel used of one loads all of it onto the device, 5 ms each.
+#pragma once
+
 #include <algorithm>
 #include <atomic>
 #include <vector>
@@ -281,14 +286,8 @@ cudaError_t launch_class(const ResClass& c, const BatchView& b, const Iterates<T
     return run(batch_resident<T, 1024, false>);
 }
 
-// The largest cluster the device schedules at the largest shared memory, FP32
-// and FP64.
-std::atomic<int> g_res_cluster[2];
-
-template <class T>
-int res_cluster() {
-    return g_res_cluster[std::is_same<T, float>::value ? 0 : 1].load(std::memory_order_relaxed);
-}
+// The largest cluster the device schedules at the largest shared memory.
+std::atomic<int> g_res_cluster{0};
 
 }  // namespace
 
@@ -298,10 +297,8 @@ void init_resident_kernels() {
                       res_largest_cluster(batch_resident<T, 1024, true>, 1024),
                       res_largest_cluster(batch_resident<T, 512, false>, 512),
                       res_largest_cluster(batch_resident<T, 256, false>, 256)};
-    g_res_cluster[std::is_same<T, float>::value ? 0 : 1] = *std::min_element(c, c + 4) == 0 ? 0 : std::min(c[0], c[1]);
+    g_res_cluster = *std::min_element(c, c + 4) == 0 ? 0 : std::min(c[0], c[1]);
 }
-template void init_resident_kernels<float>();
-template void init_resident_kernels<double>();
 
 // Classes of like CTAs, tried in the order of their CTAs; the largest instances
 // first (a class's launch ends with its last instance).
@@ -324,7 +321,7 @@ int res_class(const ResParts& pt, const ResParts& pa, int lgt, int lga, bool hal
     int last = -1;
     for (int c = 2; c < kResClasses; ++c) {
         const ResClass& k = kClasses[c];
-        if (k.size > res_cluster<T>()) continue;
+        if (k.size > g_res_cluster) continue;
         const ResSize y = k.far ? res_size<T, true>(pt, pa, k.size, lgt, lga, halpern)
                                 : res_size<T, false>(pt, pa, k.size, lgt, lga, halpern);
         if (y.smem > kResMaxSmem) continue;
@@ -342,7 +339,7 @@ template <class T>
 bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, int sms, ResPlan& plan) {
     plan = ResPlan{};
     const size_t count = parts.size() / 2;
-    if (res_cluster<T>() == 0) return false;
+    if (g_res_cluster == 0) return false;
     struct Item {
         int32_t k, nnz, cls;
         ResFar far;
@@ -409,14 +406,5 @@ cudaError_t launch_batch_resident(const std::vector<ResClass>& classes, const Re
     }
     return e;
 }
-
-template bool plan_resident<float>(const std::vector<ResParts>&, int, int, bool, int, ResPlan&);
-template bool plan_resident<double>(const std::vector<ResParts>&, int, int, bool, int, ResPlan&);
-template cudaError_t launch_batch_resident<float>(const std::vector<ResClass>&, const ResBuffers&, int, int,
-                                                  const BatchView&, const Iterates<float>&, const BatchParams&,
-                                                  long long, long long, long long, cudaStream_t, const ResStreams&);
-template cudaError_t launch_batch_resident<double>(const std::vector<ResClass>&, const ResBuffers&, int, int,
-                                                   const BatchView&, const Iterates<double>&, const BatchParams&,
-                                                   long long, long long, long long, cudaStream_t, const ResStreams&);
 
 }  // namespace pdhg

@@ -553,7 +553,7 @@ void launch_norms(int32_t m, int32_t n, const double* c_s, const double* rlo_s,
 // Inclusive prefix sum of n int32 counts into out[1..n], out[0] = 0 (CUB).
 int prefix_rows(const int32_t* cnt, int32_t n, int32_t* out, cudaStream_t s);
 
-// batch_resident.cu, exact_resident.cu: before an engine's first use of the
+// batch_resident.cuh, exact_resident.cu: before an engine's first use of the
 // kernels (the first in a process loads them onto the device: milliseconds)
 template <class T>
 void init_resident_kernels();

@@ -1,5 +1,5 @@
 """A stop request to a batch of more instances than run on the GPU at once
-(batch_resident.cu: an instance waits for a cluster's place): an instance that
+(batch_resident.cuh: an instance waits for a cluster's place): an instance that
 runs ends after its check period, one that still waits ends without an
 iteration, and each reports the iterations that its point has.
 

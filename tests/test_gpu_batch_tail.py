@@ -1,5 +1,5 @@
 """A batch on clusters with fewer iterations than a check period: no period and
-no check, only the tail (batch_resident.cu), against the kernels over all
+no check, only the tail (batch_resident.cuh), against the kernels over all
 instances, which a batch takes when one of its instances fits no cluster.
 
 Sizes: an instance on a cluster of two CTAs, of eight and of sixteen (the last
