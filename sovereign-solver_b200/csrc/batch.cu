@@ -648,12 +648,11 @@ int batch_plan(BatchCtx& c, BatchCtx::Plan** out) {
         BCK(upload(pl.list, r.list, c.stream));
         BCK(upload(pl.where, r.where, c.stream));
         BCK(cudaStreamSynchronize(c.stream));  // the host vectors are read by the copies above
-        if (c.side.fork == nullptr) {
-            BCK(cudaEventCreateWithFlags(&c.side.fork, cudaEventDisableTiming));
-            for (int i = 0; i < kResClasses - 1; ++i) {
-                BCK(cudaStreamCreateWithFlags(&c.side.stream[i], cudaStreamNonBlocking));
-                BCK(cudaEventCreateWithFlags(&c.side.join[i], cudaEventDisableTiming));
-            }
+        // each where it is not yet there: a solve that ran out of them may be tried again
+        if (c.side.fork == nullptr) BCK(cudaEventCreateWithFlags(&c.side.fork, cudaEventDisableTiming));
+        for (int i = 0; i < kResClasses - 1; ++i) {
+            if (c.side.stream[i] == nullptr) BCK(cudaStreamCreateWithFlags(&c.side.stream[i], cudaStreamNonBlocking));
+            if (c.side.join[i] == nullptr) BCK(cudaEventCreateWithFlags(&c.side.join[i], cudaEventDisableTiming));
         }
     }
     pl.made = true;
