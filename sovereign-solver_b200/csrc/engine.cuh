@@ -160,8 +160,9 @@ struct DevCsr {
     // the columns and stream the gathered vector
     const int32_t* dense_off = nullptr;
     // rows of two entries (rp_stride 2; else null): per 32 consecutive rows a
-    // descriptor of each entry's column, from which the uniform kernels compute
-    // the columns instead of loading them (run_col)
+    // descriptor of each entry's column, from which the primal pass
+    // (fast_primal_wide) and the check compute the columns instead of loading
+    // them (run_col)
     const int2* runs = nullptr;
 };
 // A run descriptor: the first of the 32 rows' column, and in the top bit

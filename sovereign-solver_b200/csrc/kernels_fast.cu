@@ -275,7 +275,7 @@ constexpr int uniform_min_ctas() {
     return sizeof(T) == 8 ? PDHG_UNIFORM_MIN_CTAS_F64 : (E == 2 ? PDHG_UNIFORM_MIN_CTAS : PDHG_UNIFORM_MIN_CTAS_E4);
 }
 
-template <class T, int E, int VW, bool PRIMAL, bool EARLY, bool RUNS>
+template <class T, int E, int VW, bool PRIMAL, bool EARLY>
 __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     fast_iter_uniform(FastIter<T> a, int first, int reset) {
     constexpr int S = E * VW;
@@ -297,18 +297,9 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     EpiIn<T> in{};
     if (!EARLY && lane == 0) in = epi_load<T, PRIMAL>(a.it, pv, r, first, fresh, hw);
     if (EARLY && lane == 0) in = epi_load_fixed<T, PRIMAL>(a.it, pv, r);
-    int c[E];  // RUNS: the row's run descriptor until its columns are needed
+    int c[E];
     T v[E];
-    auto load_cols = [&](int row, int (&to)[E]) {
-        if constexpr (RUNS) {
-            const int2 d = __ldg(M.runs + (row >> 5));
-            to[0] = d.x;
-            to[1] = d.y;
-        } else {
-            load_idx<E>(M.ci + static_cast<int64_t>(row) * S + lane * E, to);
-        }
-    };
-    load_cols(r, c);
+    load_idx<E>(M.ci + static_cast<int64_t>(r) * S + lane * E, c);
     load_vals<T, E>(vals + static_cast<int64_t>(r) * S + lane * E, v);
     if (EARLY) {
         pass_wait();
@@ -316,14 +307,6 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
     }
     for (;;) {
         T g[E];
-        if constexpr (RUNS) {  // a warp's 32 rows share a descriptor
-            if (c[0] != kNoRun) {
-#pragma unroll
-                for (int q = 0; q < E; ++q) c[q] = run_col(c[q], r & 31);
-            } else {
-                load_idx<E>(M.ci + static_cast<int64_t>(r) * S, c);
-            }
-        }
 #pragma unroll
         for (int q = 0; q < E; ++q) g[q] = gather_ld<EARLY>(xg + c[q]);
         const int rn = r + groups;
@@ -333,7 +316,7 @@ __global__ void __launch_bounds__(kBlock, (uniform_min_ctas<T, E, VW>()))
         T nv[E];
         if (more) {
             if (lane == 0) nin = pass_operands<T, PRIMAL, EARLY>(a.it, pv, rn, first, fresh, hw);
-            load_cols(rn, nc);
+            load_idx<E>(M.ci + static_cast<int64_t>(rn) * S + lane * E, nc);
             load_vals<T, E>(vals + static_cast<int64_t>(rn) * S + lane * E, nv);
         }
         T acc = mul_rn<T>(v[0], g[0]);
@@ -904,15 +887,8 @@ void launch_uniform(const FastIter<T>& a, const DevCsr& M, int cap, int first, i
                     cudaStream_t s, bool early) {
     const int64_t need = (static_cast<int64_t>(M.rows) * VW + kBlock - 1) / kBlock;
     const int grid = static_cast<int>(need < cap ? need : cap);
-    auto run = [&](auto runs) {
-        constexpr bool R = decltype(runs)::value;
-        if (a.early) launch_pass(fast_iter_uniform<T, E, VW, PRIMAL, true, R>, grid, early, s, a, first, reset);
-        else fast_iter_uniform<T, E, VW, PRIMAL, false, R><<<grid, kBlock, 0, s>>>(a, first, reset);
-    };
-    if constexpr (E * VW == 2) {
-        if (M.runs != nullptr) return run(std::true_type{});
-    }
-    run(std::false_type{});
+    if (a.early) launch_pass(fast_iter_uniform<T, E, VW, PRIMAL, true>, grid, early, s, a, first, reset);
+    else fast_iter_uniform<T, E, VW, PRIMAL, false><<<grid, kBlock, 0, s>>>(a, first, reset);
 }
 
 template <class T, bool PRIMAL, bool EARLY>
@@ -1943,12 +1919,12 @@ int init_fast_kernels(int device) {
     const int s64 = resident_per_sm(fast_iter_slices<double, false, false>);
     const int w[2] = {resident_per_sm(fast_primal_wide<float, false, false>),
                       resident_per_sm(fast_primal_wide<double, false, false>)};
-    const int u[3][2] = {{resident_per_sm(fast_iter_uniform<float, 2, 1, true, false, false>),
-                          resident_per_sm(fast_iter_uniform<double, 2, 1, true, false, false>)},
-                         {resident_per_sm(fast_iter_uniform<float, 4, 1, true, false, false>),
-                          resident_per_sm(fast_iter_uniform<double, 4, 1, true, false, false>)},
-                         {resident_per_sm(fast_iter_uniform<float, 4, 2, true, false, false>),
-                          resident_per_sm(fast_iter_uniform<double, 4, 2, true, false, false>)}};
+    const int u[3][2] = {{resident_per_sm(fast_iter_uniform<float, 2, 1, true, false>),
+                          resident_per_sm(fast_iter_uniform<double, 2, 1, true, false>)},
+                         {resident_per_sm(fast_iter_uniform<float, 4, 1, true, false>),
+                          resident_per_sm(fast_iter_uniform<double, 4, 1, true, false>)},
+                         {resident_per_sm(fast_iter_uniform<float, 4, 2, true, false>),
+                          resident_per_sm(fast_iter_uniform<double, 4, 2, true, false>)}};
     for (int t = 0; t < 2; ++t) {
         if (w[t] <= 0) return 1;
         g_cap_wide[t] = w[t] * sms;
