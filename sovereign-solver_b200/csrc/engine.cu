@@ -1400,6 +1400,7 @@ int solve(Ctx& c, const pdhg_options& o, pdhg_info* info, double* x, double* y, 
     fa.st = c.st.p;
     fa.part = c.part.p;
     fa.part_blocks = static_cast<int>(std::min<size_t>(c.part.n / 3, 8 * static_cast<size_t>(c.sm_count)));
+    fa.row_blocks = 16 * c.sm_count;
     launch_final(fa, c.stream);
     c.launches += 5;
     CK(cudaGetLastError());

@@ -444,6 +444,7 @@ struct FinalArgs {
     DevState* st;
     double* part = nullptr;   // 3 doubles per CTA of the fast-mode sums
     int part_blocks = 0;      // CTAs that fit in part (and at most a few per SM)
+    int row_blocks = 0;       // at most this many CTAs for the products (a few per SM)
 };
 void launch_final(const FinalArgs& a, cudaStream_t s);
 // launch_final's products in the throughput modes (kernels_fast.cu)

@@ -1889,7 +1889,7 @@ __global__ void __launch_bounds__(kBlock) fast_final(FinalArgs a) {
 
 void launch_fast_final_rows(const FinalArgs& a, cudaStream_t s) {
     int g = tier_blocks(a.Ao) + tier_blocks(a.ATo);
-    if (g > 148 * 16) g = 148 * 16;
+    if (g > a.row_blocks) g = a.row_blocks;
     if (g > 0) fast_final<<<g, kBlock, 0, s>>>(a);
 }
 

@@ -39,8 +39,6 @@ using bf16 = __nv_bfloat16;
 constexpr int kGemmThreads = kBlock;
 constexpr long long kSpinLimit = 1LL << 24;  // bounded mbarrier waits
 
-constexpr int kGemmSms = 148;
-
 struct GemmArgs {
     int M, N, K;
     const bf16* A;
@@ -442,7 +440,7 @@ cudaError_t run_gemm(const GemmPair& p, int tiles, int rounds, bool early, cudaS
 // CTAs than the GPU has SMs, then 64, then 128: a wider tile reads A less often,
 // a narrower one leaves fewer SMs idle (256 x 512 x 512: 8 CTAs of 128 columns,
 // 32 of 32).
-int gemm(const GemmArgs& g, const GemmArgs* h, bool early, cudaStream_t s) {
+int gemm(const GemmArgs& g, const GemmArgs* h, bool early, int sms, cudaStream_t s) {
     GemmPair p{};
     int rounds = 0, tiles[3] = {};
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
@@ -461,7 +459,7 @@ int gemm(const GemmArgs& g, const GemmArgs* h, bool early, cudaStream_t s) {
             tiles[w] += t;
         }
     }
-    const int w = tiles[0] <= kGemmSms ? 0 : tiles[1] <= kGemmSms ? 1 : 2;
+    const int w = tiles[0] <= sms ? 0 : tiles[1] <= sms ? 1 : 2;
     p.tiles0 = ((g.M + tc::kTileM - 1) / tc::kTileM) * ((g.N + (32 << w) - 1) / (32 << w));
     const cudaError_t e = w == 0   ? run_gemm<32, 8>(p, tiles[0], rounds, early, s)
                           : w == 1 ? run_gemm<64, 8>(p, tiles[1], rounds, early, s)
@@ -475,10 +473,10 @@ void transpose(const bf16* in, int ldi, bf16* out, int ldo, int R, int C, cudaSt
 }
 
 // CTAs of forward()'s last product (gemm's rule), each with its part of the loss.
-int loss_parts(int B, int n_out) {
+int loss_parts(int B, int n_out, int sms) {
     const int tm = (B + tc::kTileM - 1) / tc::kTileM;
     for (int w = 0; w < 2; ++w)
-        if (tm * blocks(n_out, 32 << w) <= kGemmSms) return tm * blocks(n_out, 32 << w);
+        if (tm * blocks(n_out, 32 << w) <= sms) return tm * blocks(n_out, 32 << w);
     return tm * blocks(n_out, 128);
 }
 
@@ -504,6 +502,7 @@ struct Dev {
 
 struct Mlp {
     int device = 0;
+    int sms = 0;  // the device's
     int n_in = 0, hidden = 0, n_out = 0, max_batch = 0;
     cudaStream_t stream = nullptr;
     std::string err;
@@ -587,7 +586,7 @@ int forward(Mlp& h, int B, const float* t, const int32_t* idx) {
     g.ld16 = h.hidden;
     g.out16t = t != nullptr ? h.h1t.p : nullptr;
     g.ldt = B;
-    if ((rc = gemm(g, nullptr, true, h.stream)) != PDHG_OK) return rc;
+    if ((rc = gemm(g, nullptr, true, h.sms, h.stream)) != PDHG_OK) return rc;
     g = args(B, h.hidden, h.hidden, h.h1.p, h.hidden, h.W16(1), h.hidden, &h.status->err);
     g.bias = h.Bv(1);
     g.relu = 1;
@@ -595,7 +594,7 @@ int forward(Mlp& h, int B, const float* t, const int32_t* idx) {
     g.ld16 = h.hidden;
     g.out16t = t != nullptr ? h.h2t.p : nullptr;
     g.ldt = B;
-    if ((rc = gemm(g, nullptr, true, h.stream)) != PDHG_OK) return rc;
+    if ((rc = gemm(g, nullptr, true, h.sms, h.stream)) != PDHG_OK) return rc;
     g = args(B, h.n_out, h.hidden, h.h2.p, h.hidden, h.W16(2), h.hidden, &h.status->err);
     g.bias = h.Bv(2);
     g.ld32 = h.n_out;
@@ -612,7 +611,7 @@ int forward(Mlp& h, int B, const float* t, const int32_t* idx) {
         g.out16t = h.dyt.p;
         g.ldt = B;
     }
-    return gemm(g, nullptr, true, h.stream);
+    return gemm(g, nullptr, true, h.sms, h.stream);
 }
 
 // Gradients into h.g after forward() with targets; the batch's loss to *loss.
@@ -632,7 +631,7 @@ int backward(Mlp& h, int B, double* loss) {
     d.ld16 = h.hidden;
     d.out16t = h.dz2t.p;
     d.ldt = B;
-    if ((rc = gemm(g, &d, true, h.stream)) != PDHG_OK) return rc;
+    if ((rc = gemm(g, &d, true, h.sms, h.stream)) != PDHG_OK) return rc;
     // layer 2's weights and layer 1's input
     g = args(h.hidden, h.hidden, B, h.dz2t.p, B, h.h1t.p, B, err);
     g.out32 = h.gW(1);
@@ -644,12 +643,12 @@ int backward(Mlp& h, int B, double* loss) {
     d.ld32 = h.hidden;
     d.out16t = h.dz1t.p;
     d.ldt = B;
-    if ((rc = gemm(g, &d, true, h.stream)) != PDHG_OK) return rc;
+    if ((rc = gemm(g, &d, true, h.sms, h.stream)) != PDHG_OK) return rc;
     // layer 1's weights
     g = args(h.hidden, h.n_in, B, h.dz1t.p, B, h.xt.p, B, err);
     g.out32 = h.gW(0);
     g.ld32 = h.n_in;
-    if ((rc = gemm(g, nullptr, true, h.stream)) != PDHG_OK) return rc;
+    if ((rc = gemm(g, nullptr, true, h.sms, h.stream)) != PDHG_OK) return rc;
     ColSums c{};
     const float* dz[3] = {h.dy32.p, h.dz2_32.p, h.dz1_32.p};
     const int n[3] = {h.n_out, h.hidden, h.hidden};
@@ -661,7 +660,7 @@ int backward(Mlp& h, int B, double* loss) {
     }
     c.B = B;
     c.part = h.part.p;
-    c.n_part = loss_parts(B, h.n_out);
+    c.n_part = loss_parts(B, h.n_out, h.sms);
     c.loss = loss;
     return launch_pass(k_colsums, c.first[3] + 1, true, h.stream, c) == cudaSuccess ? PDHG_OK : PDHG_ERR_BACKEND;
 }
@@ -712,6 +711,7 @@ int pdhg_mlp_create(int device, int n_in, int hidden, int n_out, int max_batch, 
     h.max_batch = max_batch;
     MCK(cudaSetDevice(device));
     MCK(init_gemm());
+    MCK(cudaDeviceGetAttribute(&h.sms, cudaDevAttrMultiProcessorCount, device));
     MCK(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
     const int64_t sizes[6] = {static_cast<int64_t>(hidden) * n_in, hidden,
                               static_cast<int64_t>(hidden) * hidden, hidden,
@@ -748,8 +748,8 @@ int pdhg_mlp_create(int device, int n_in, int hidden, int n_out, int max_batch, 
     MCK(h.dy32.alloc(B * n_out));
     MCK(h.dz2_32.alloc(B * H));
     MCK(h.dz1_32.alloc(B * H));
-    // a batch of fewer rows has narrower tiles, up to kGemmSms of them
-    MCK(h.part.alloc(std::max<size_t>(loss_parts(max_batch, n_out), kGemmSms)));
+    // a batch of fewer rows has narrower tiles, up to one per SM
+    MCK(h.part.alloc(std::max(loss_parts(max_batch, n_out, h.sms), h.sms)));
     MCK(cudaHostAlloc(reinterpret_cast<void**>(&h.status), sizeof(Mlp::Status), cudaHostAllocDefault));
     *h.status = Mlp::Status{};
     MCK(cudaMemsetAsync(h.w.p, 0, sizeof(float) * o, h.stream));
@@ -941,7 +941,10 @@ int pdhg_gemm_bf16(int device, int m, int n, int k, const float* a, const float*
     if (m < 1 || n < 1 || k < 8 || k % 8 || a == nullptr || b == nullptr || c == nullptr)
         return PDHG_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(device) != cudaSuccess) return PDHG_ERR_UNSUPPORTED;
-    if (init_gemm() != cudaSuccess) return PDHG_ERR_BACKEND;
+    int sms = 0;
+    if (init_gemm() != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        return PDHG_ERR_BACKEND;
     Dev<float> a32, b32, c32, bias32;
     Dev<bf16> a16, b16;
     Dev<int> err;
@@ -960,7 +963,7 @@ int pdhg_gemm_bf16(int device, int m, int n, int k, const float* a, const float*
     g.relu = relu;
     g.out32 = c32.p;
     g.ld32 = n;
-    int rc = gemm(g, nullptr, false, nullptr);
+    int rc = gemm(g, nullptr, false, sms, nullptr);
     if (rc != PDHG_OK) return rc;
     int e = 0;
     if (cudaMemcpy(&e, err.p, sizeof e, cudaMemcpyDeviceToHost) != cudaSuccess) return PDHG_ERR_BACKEND;
