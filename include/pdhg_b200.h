@@ -272,7 +272,10 @@ int pdhg_get_tuning(const pdhg_ctx* ctx, int precision, int* out);
  * by timing. Engine extension: on the first pdhg_solve_batch of a loaded batch
  * with >= 2^20 nonzeros (option autotune on) each pass's width is timed at the
  * binning's choice, half and twice it, and the fastest kept until the next
- * load; smaller batches and autotune = 0 keep the binning's choice. */
+ * load; smaller batches and autotune = 0 keep the binning's choice. These are
+ * the widths of the kernels over all instances. A batch whose instances run on
+ * a cluster each (all fit one in `precision`) takes the binning's width there,
+ * at most four lanes, and the timed one only where those kernels stand in. */
 int pdhg_get_batch_tuning(const pdhg_ctx* ctx, int precision, int* out);
 
 /* Per-kernel timing of the iteration kernels on the loaded problem (CUDA events

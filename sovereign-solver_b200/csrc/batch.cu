@@ -578,7 +578,8 @@ float batch_time_pass(BatchCtx& c, bool primal, cudaEvent_t e0, cudaEvent_t e1) 
 // current pick only when 5% faster. Runs on the solve's own iterates before
 // the initial point is written (the initial point resets them). Batches
 // under 2^20 nonzeros keep the binning's width (their passes are
-// launch-bound). The choice holds until the next load.
+// launch-bound). The choice holds until the next load. A batch on clusters
+// (batch_plan) does not use it, unless it has no room for its entries there.
 template <class T>
 int batch_tune(BatchCtx& c, bool autotune) {
     const int pi = std::is_same<T, float>::value ? 0 : 1;
@@ -624,9 +625,10 @@ int batch_tune(BatchCtx& c, bool autotune) {
     return PDHG_OK;
 }
 
-// Lanes (log2) per row on a cluster: the binning's, at most four. In shared
-// memory a row's entries are near, and eight lanes on a row of 18 entries cost
-// more slots than they save steps.
+// Lanes (log2) per row on a cluster: the binning's, at most four, never the
+// tuner's (its timings are of other kernels, and the points would follow timing
+// noise). In shared memory a row's entries are near, and eight lanes on a row of
+// 18 entries cost more slots than they save steps.
 int lanes_log2(int vw) { return vw >= 4 ? 2 : vw / 2; }
 
 // The plan of this precision and form, made on its first solve since the load.

@@ -10,9 +10,11 @@
 //   * row kernels (iterations, power-iteration products, Ruiz maxima): the
 //     single engine's kernels with an instance lookup per row (row_inst /
 //     col_inst) for the instance's step sizes and done flag;
-//   * instance kernels: one CTA per instance (check + decision, restart,
-//     norms, Ruiz update, final result), so every per-instance reduction and
-//     decision is made inside one CTA without atomics or tickets.
+//   * instance kernels: one CTA per instance (restart, norms, Ruiz update), or
+//     CTA parts merged by the instance's last one (check + decision, final
+//     result).
+// Instances that fit a cluster's shared memory run there instead
+// (batch_resident.cuh).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : NT == 512 ? 2 : 1)
             const double ri = s.inv;
             if (restart && p.primal_weight_update) {
                 // the weight's sums in batch_restart's order, whatever the
-                // cluster: the iterates that follow are its bits
+                // cluster, so the step sizes do not depend on its size
                 if (cl.rank == 0) {
                     double dx2 = 0.0, dy2 = 0.0;
                     if (NT == kBlock || threadIdx.x < kBlock)

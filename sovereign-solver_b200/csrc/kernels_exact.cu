@@ -485,8 +485,8 @@ __global__ void k_fill(double* x, int64_t n, double v) {
 // At depth d every node has size floor or ceil of n / 2^d, so the nodes of
 // depth D-1 (D = first depth whose sizes are all <= 128) are either leaves
 // (size <= 128) or parents of two leaves, and every node above is internal.
-// Kernel 1 evaluates depth D-1 (k_pw_level_staged); kernel 2 folds the levels
-// pairwise, left + right, exactly like the recursion.
+// k_pw_norms evaluates depth D-1 and folds the levels above pairwise, left +
+// right, exactly like the recursion.
 __host__ __device__ inline void pw_node(int64_t n, int depth, int64_t idx, int64_t* off,
                                         int64_t* size) {
     int64_t o = 0, s = n;

@@ -15,8 +15,9 @@
 // slice's lanes run the same number of steps and its entries are read without
 // bank conflicts; only the gathers conflict. Row by row (each lane reading its
 // own row's entries) a pass over 500 rows of 12 entries took 3,900 cycles of
-// one SM. A row's lanes and the order of its sum are those of the kernels over
-// all instances (batch_block, long_row_dot), so the iterates are theirs too.
+// one SM. A long row's sum has long_row_dot's order; a short one's is that of
+// the kernels over all instances only where those give it as many lanes (here
+// at most four, batch.cu lanes_log2), so the iterates differ by rounding.
 //
 // Measured on a B200, in cycles: block barrier 43, cluster barrier 470 at any
 // size, a vector of 4 KB / 16 KB / 40 KB to all CTAs with the barrier 1,140 /

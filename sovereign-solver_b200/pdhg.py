@@ -511,7 +511,8 @@ class Engine:
                 "dual_long_mode": out[3], "timed": bool(out[4])}
 
     def batch_tuning(self, precision: str = "mixed") -> dict:
-        """Lanes per row of the batched passes for the loaded batch (pdhg_get_batch_tuning)."""
+        """Lanes per row of the kernels over all instances of the loaded batch
+        (pdhg_get_batch_tuning); instances on clusters take the binning's, at most four."""
         out = (C.c_int * 3)()
         _check(lib().pdhg_get_batch_tuning(self._h, PREC[precision], out),
                "pdhg_get_batch_tuning", self._h)
