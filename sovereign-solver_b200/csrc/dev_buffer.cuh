@@ -125,6 +125,7 @@ struct MatDev {
     int32_t short_max = kLongRow, n_iter_short = 0, n_warp0 = 0, n_warp1 = 0;
     int vw = 1;
     int32_t rp_stride = 0;  // every row this long (0: not uniform)
+    int32_t longest = 0;    // entries of the longest row
     int64_t nnz_dense = 0;  // entries of the dense rows (columns computed)
     DBuf<int2> runs;        // column runs of rows of two entries, if in use
     int64_t nnz_runs = 0;   // entries whose columns they give
@@ -158,6 +159,7 @@ struct MatDev {
         d.slices = slices.view();
         d.no_slice_tiers = no_slice_tiers.view();
         d.rp_stride = rp_stride;
+        d.longest = longest;
         d.dense_off = dense_off.p;
         d.runs = runs.p;
         return d;
@@ -285,7 +287,7 @@ inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err) {
     if (parts) launch_parts(M.rp.p, M.rows, reinterpret_cast<ResParts*>(cnt.p + 9), s);
     launch_bin(M.rp.p, M.rows, kLongRow, M.long_rows.p, cnt.p, s);
     launch_bin(M.rp.p, M.rows, kWarpRow, M.wrows.p, cnt.p + 3, s);
-    // rows all of one length: the short-row kernel computes their extents
+    // rows all of one length: the short-row kernel computes their extents; the longest row
     launch_uniform_rows(M.rp.p, M.rows, reinterpret_cast<unsigned*>(cnt.p + 8), s);
     int32_t rp01[2] = {0, 0};
     if (M.rows > 0) cudaMemcpyAsync(rp01, M.rp.p, sizeof rp01, cudaMemcpyDeviceToHost, s);
@@ -297,7 +299,10 @@ inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err) {
     M.n_long = static_cast<int32_t>(h[0]);
     M.n_short = static_cast<int32_t>(h[1]);
     M.n_wrows = static_cast<int32_t>(h[3]);
-    M.rp_stride = (M.rows > 0 && h[8] == 0 && rp01[0] == 0) ? rp01[1] : 0;
+    unsigned uni[2];  // k_uniform_rows
+    std::memcpy(uni, h + 8, sizeof uni);
+    M.rp_stride = (M.rows > 0 && uni[0] == 0 && rp01[0] == 0) ? rp01[1] : 0;
+    M.longest = static_cast<int32_t>(uni[1]);
     const double mean = h[1] > 0 ? static_cast<double>(h[2]) / static_cast<double>(h[1]) : 0.0;
     int w = 1;
     while (w < 32 && 2.0 * w <= mean / 2.0 + 1e-9) w *= 2;

@@ -497,8 +497,8 @@ struct Launcher {
         // the first pass of a period follows the restart kernel in full order
         const bool p = chained && !first;
         if (prec == PDHG_PREC_FP64_EXACT) {
-            launch_exact_primal(ei, first, s, p && c.lp.m > 0);
-            launch_exact_dual(ei, first, s, c.lp.n > 0);
+            launch_exact_primal(ei, first, s, p && ei.early && c.lp.m > 0);
+            launch_exact_dual(ei, first, s, ei.early && c.lp.n > 0);
             c.launches += 2;
         } else if (prec == PDHG_PREC_MIXED) {
             const bool one = fast_early(fi32);
@@ -575,7 +575,7 @@ Launcher make_launcher(Ctx& c, int prec, const pdhg_options& o, bool want_candid
         L.one = plan_exact_resident(c.ATs.parts, c.As.parts, std::max(c.ATs.parts.longest, c.As.parts.longest));
     const DevProblem P = c.problem();
     const double bt = o.tolerance > 1e-6 ? o.tolerance : 1e-6;
-    L.ei = ExactIter{c.As.view(), c.ATs.view(), P, iterates<double>(c), c.st.p};
+    L.ei = ExactIter{c.As.view(), c.ATs.view(), P, iterates<double>(c), c.st.p, exact_early(c.As.view(), c.ATs.view()) ? 1 : 0};
     CheckScratch cs{c.act_avg.p, c.cand_xo.p, c.cand_yo.p, c.part.p, 0};
     L.ec = ExactCheck{c.As.view(), c.ATs.view(), c.Ao.view(), c.ATo.view(), P,
                       iterates<double>(c), cs, o.tolerance, bt, o.restart_sufficient_decrease,

@@ -122,6 +122,7 @@ struct DevCsr {
     // list every row runs on one thread.
     const int32_t* wrows = nullptr;
     int32_t n_wrows = 0;
+    int32_t longest = 0;  // entries of the longest row
     // The throughput kernels (iteration and check) bin once more. Rows of at
     // most short_max entries (16 lanes' worth at the binning's lanes per row,
     // within [kWarpRow, kLongRow]) run on lane groups, n_iter_short of them;
@@ -313,7 +314,10 @@ struct ExactIter {
     DevProblem P;
     Iterates<double> it;
     DevState* st;
+    int early = 0;  // the kernels that may be launched early (exact_early)
 };
+// Whether the passes of this LP are small enough for them.
+bool exact_early(const DevCsr& A, const DevCsr& AT);
 // early (here and below): the pass follows the pass before it directly
 void launch_exact_primal(const ExactIter& a, int first, cudaStream_t s, bool early = false);
 void launch_exact_dual(const ExactIter& a, int first, cudaStream_t s, bool early = false);
@@ -510,9 +514,9 @@ void launch_validate(int32_t m, int32_t n, const int32_t* rp, const int32_t* ci,
 // Rows with lo < length <= hi appended to `list`, their number added to *count.
 void launch_bin_range(const int32_t* rp, int32_t rows, int lo, int hi, int32_t* list,
                       unsigned long long* count, cudaStream_t s);
-// *flag |= 1 when the rows' lengths are not all equal / the entries of v not
-// all equal (flag zeroed by the caller).
-void launch_uniform_rows(const int32_t* rp, int32_t rows, unsigned* flag, cudaStream_t s);
+// out[0] / *flag |= 1 when the rows' lengths are not all equal / the entries of
+// v not all equal; out[1]: the longest row's length (zeroed by the caller).
+void launch_uniform_rows(const int32_t* rp, int32_t rows, unsigned* out, cudaStream_t s);
 void launch_uniform_vec(const double* v, int32_t n, unsigned* flag, cudaStream_t s);
 void launch_bin(const int32_t* rp, int32_t rows, int long_threshold, int32_t* long_rows,
                 unsigned long long* counters, cudaStream_t s);

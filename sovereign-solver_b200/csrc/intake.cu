@@ -89,14 +89,22 @@ __global__ void __launch_bounds__(kBlock) k_validate(int32_t m, int32_t n, const
 
 // Row lengths -> long-row list, number and total length of short rows
 // (grid-stride, one atomic per CTA and counter).
-// *flag |= 1 when some row's length differs from row 0's (grid-stride).
-__global__ void k_uniform_rows(const int32_t* rp, int32_t rows, unsigned* flag) {
+// out[0] |= 1 when some row's length differs from row 0's, out[1]: the longest
+// row's length (grid-stride).
+__global__ void k_uniform_rows(const int32_t* rp, int32_t rows, unsigned* out) {
     const int len0 = rp[1] - rp[0];
-    bool diff = false;
+    unsigned diff = 0, longest = 0;
     for (int64_t r = blockIdx.x * static_cast<int64_t>(kBlock) + threadIdx.x; r < rows;
-         r += static_cast<int64_t>(gridDim.x) * kBlock)
-        diff = diff || (rp[r + 1] - rp[r] != len0);
-    if (diff) atomicOr(flag, 1u);
+         r += static_cast<int64_t>(gridDim.x) * kBlock) {
+        const int len = rp[r + 1] - rp[r];
+        if (len != len0) diff = 1;
+        longest = max(longest, static_cast<unsigned>(len));
+    }
+    diff = __reduce_or_sync(0xffffffffu, diff);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) != 0) return;
+    if (diff) atomicOr(out, 1u);
+    atomicMax(out + 1, longest);
 }
 
 // *flag |= 1 when some entry differs from entry 0 (grid-stride; +-inf compare
@@ -594,9 +602,9 @@ void launch_bin(const int32_t* rp, int32_t rows, int long_threshold, int32_t* lo
     if (rows > 0) k_bin<<<g, kBlock, 0, s>>>(rp, rows, long_threshold, long_rows, counters);
 }
 
-void launch_uniform_rows(const int32_t* rp, int32_t rows, unsigned* flag, cudaStream_t s) {
+void launch_uniform_rows(const int32_t* rp, int32_t rows, unsigned* out, cudaStream_t s) {
     const int g = nblocks(rows) < kGridCap ? nblocks(rows) : kGridCap;
-    if (rows > 0) k_uniform_rows<<<g, kBlock, 0, s>>>(rp, rows, flag);
+    if (rows > 0) k_uniform_rows<<<g, kBlock, 0, s>>>(rp, rows, out);
 }
 
 void launch_uniform_vec(const double* v, int32_t n, unsigned* flag, cudaStream_t s) {

@@ -130,11 +130,25 @@ __device__ __forceinline__ double pass_row_dot(const RowTask& t, const DevCsr& M
     return ordered_dot_warp_pipelined(b, e, ci, v, g, init, warp_stage2(), wait);
 }
 
+// How a pass adds its rows (the same order and rounding):
+//   kExEarly   launched early (ExactIter::early), the loads above ahead of the wait;
+//   kExChain   a warp row's next rounds in flight while it adds one;
+//   kExRows    a warp row's round loaded, then added: fewer registers, more rows
+//              at once.
+enum ExPass { kExEarly, kExChain, kExRows };
+template <int PASS, class G>
+__device__ __forceinline__ double plain_row_dot(const RowTask& t, const DevCsr& M, G g, double init) {
+    if (PASS == kExChain && t.warp)
+        return ordered_dot_warp_pipelined(M.rp[t.row], M.rp[t.row + 1], M.ci, M.v64, g, init, warp_stage2());
+    return row_dot(t, M, g, init);
+}
+
 // K1: per column j -- grad = c - A^T y (pdhg.cpp:296-297: grad starts at c,
 // then every row adds val * (-y_r) in row order), x_new = proj(x - tau grad),
-// x_bar = 2 x_new - x, Cesaro sum.
+// x_bar = 2 x_new - x, Cesaro sum. PASS: ExPass.
+template <int PASS>
 __global__ void __launch_bounds__(kBlock) ex_primal(ExactIter a, int first) {
-    pass_begin();
+    if (PASS == kExEarly) pass_begin();
     DevState* st = a.st;
     if (first && blockIdx.x == 0 && threadIdx.x == 0) st->restart = 0;  // consumed by ex_restart
     if (st->done) return;
@@ -142,16 +156,30 @@ __global__ void __launch_bounds__(kBlock) ex_primal(ExactIter a, int first) {
     if (t.row < 0) return;
     const int j = t.row;
     const double* y = a.it.y;
-    const double tau = st->tau, lo = a.P.lo[j], hi = a.P.hi[j];
-    const bool fresh = first && st->fresh;
-    double xo = 0.0, sum = 0.0;
-    const double g = pass_row_dot(t, a.AT, [y](int i) { return -coherent_ld(y + i); }, a.P.c[j], [&]() {
-        pass_wait();
+    double tau, lo, hi, xo = 0.0, sum = 0.0, g;
+    bool fresh;
+    const auto fixed = [&]() {
+        tau = st->tau;
+        lo = a.P.lo[j];
+        hi = a.P.hi[j];
+        fresh = first && st->fresh;
+    };
+    if constexpr (PASS == kExEarly) {
+        fixed();
+        g = pass_row_dot(t, a.AT, [y](int i) { return -coherent_ld(y + i); }, a.P.c[j], [&]() {
+            pass_wait();
+            if (!t.lead) return;
+            xo = coherent_ld(a.it.x + j);
+            sum = fresh ? 0.0 : coherent_ld(a.it.xsum + j);
+        });
         if (!t.lead) return;
-        xo = coherent_ld(a.it.x + j);
-        sum = fresh ? 0.0 : coherent_ld(a.it.xsum + j);
-    });
-    if (!t.lead) return;
+    } else {
+        g = plain_row_dot<PASS>(t, a.AT, [y](int i) { return -y[i]; }, a.P.c[j]);
+        if (!t.lead) return;
+        fixed();
+        xo = a.it.x[j];
+        sum = fresh ? 0.0 : a.it.xsum[j];
+    }
     const double xn = clampd(__dadd_rn(xo, __dmul_rn(-tau, g)), lo, hi);
     a.it.xbar[j] = __dadd_rn(2.0 * xn, -xo);  // scale(2.0) then axpy(-1.0, x)
     a.it.x[j] = xn;
@@ -160,25 +188,42 @@ __global__ void __launch_bounds__(kBlock) ex_primal(ExactIter a, int first) {
 
 // K2: per row i -- s_new = proj(s - tau y), s_bar = 2 s_new - s,
 // k = -(A x_bar) + s_bar, y += sigma k (pdhg.cpp:302-318), Cesaro sum.
+template <int PASS>
 __global__ void __launch_bounds__(kBlock) ex_dual(ExactIter a, int first) {
-    pass_begin();
+    if (PASS == kExEarly) pass_begin();
     DevState* st = a.st;
     if (st->done) return;
     const RowTask t = row_task(a.A, blockIdx.x);
     if (t.row < 0) return;
     const int i = t.row;
     const double* xbar = a.it.xbar;
-    const double tau = st->tau, sigma = st->sigma, lo = a.P.rlo[i], hi = a.P.rhi[i];
-    const bool fresh = first && st->fresh;
-    double yo = 0.0, so = 0.0, ysum = 0.0;
-    const double sum = pass_row_dot(t, a.A, [xbar](int j) { return coherent_ld(xbar + j); }, 0.0, [&]() {
-        pass_wait();
+    double tau, sigma, lo, hi, yo = 0.0, so = 0.0, ysum = 0.0, sum;
+    bool fresh;
+    const auto fixed = [&]() {
+        tau = st->tau;
+        sigma = st->sigma;
+        lo = a.P.rlo[i];
+        hi = a.P.rhi[i];
+        fresh = first && st->fresh;
+    };
+    if constexpr (PASS == kExEarly) {
+        fixed();
+        sum = pass_row_dot(t, a.A, [xbar](int j) { return coherent_ld(xbar + j); }, 0.0, [&]() {
+            pass_wait();
+            if (!t.lead) return;
+            yo = coherent_ld(a.it.y + i);
+            so = coherent_ld(a.it.s + i);
+            ysum = fresh ? 0.0 : coherent_ld(a.it.ysum + i);
+        });
         if (!t.lead) return;
-        yo = coherent_ld(a.it.y + i);
-        so = coherent_ld(a.it.s + i);
-        ysum = fresh ? 0.0 : coherent_ld(a.it.ysum + i);
-    });
-    if (!t.lead) return;
+    } else {
+        sum = plain_row_dot<PASS>(t, a.A, [xbar](int j) { return xbar[j]; }, 0.0);
+        if (!t.lead) return;
+        fixed();
+        yo = a.it.y[i];
+        so = a.it.s[i];
+        ysum = fresh ? 0.0 : a.it.ysum[i];
+    }
     const double sn = clampd(__dadd_rn(so, __dmul_rn(-tau, yo)), lo, hi);
     const double sbar = __dadd_rn(2.0 * sn, -so);
     const double kb = __dadd_rn(-sum, sbar);
@@ -950,11 +995,37 @@ inline int grid64(int64_t n) { return static_cast<int>((n + kBlock - 1) / kBlock
 
 int exact_check_grid(const DevCsr& A, const DevCsr& AT) { return mat_blocks(A) + mat_blocks(AT); }
 
+// The early kernels hold a row's first entries in 64 to 80 registers, so fewer
+// rows run at once than with the 32 of kExRows: they are for passes that are
+// mostly launch and latency. Us an iteration, early / the others: 50,000 x
+// 120,000 (3,750 warps) 14.7 / 15.3, 100,000 x 250,000 (7,800) 20.7 / 23.0;
+// 200,000 x 500,000 (15,600) 46.1 / 43.9, transportation 400 x 1,000 (12,500)
+// 22.9 / 20.8, 100,000 x 250,000 with 20 entries a column (101,000) 161 / 116.
+constexpr int64_t kEarlyWarps = 8192;
+bool exact_early(const DevCsr& A, const DevCsr& AT) {
+    const auto warps = [](const DevCsr& M) { return (static_cast<int64_t>(M.rows) + 31) / 32 + M.n_wrows; };
+    return warps(A) <= kEarlyWarps && warps(AT) <= kEarlyWarps;
+}
+
+// kExChain where a pass lasts as long as its longest row's chain of additions
+// (8 cycles each) rather than as its entries take to arrive. Us an iteration
+// with every warp row that way / none: transportation 701 x 1,499 44.1 / 47.7,
+// 900 x 1,900 74.7 / 72.2, 1,500 x 3,500 212 / 181; a longest row of 344,000 of
+// 4M entries 2,770 / 5,600. By this rule, a pass at a time: 38.5, 65.0, 182,
+// 2,790.
+constexpr int64_t kChainShare = 2000;
+static ExPass ex_pass(const ExactIter& a, const DevCsr& M) {
+    if (a.early) return kExEarly;
+    return static_cast<int64_t>(M.longest) * kChainShare > M.nnz ? kExChain : kExRows;
+}
+
 void launch_exact_primal(const ExactIter& a, int first, cudaStream_t s, bool early) {
-    if (a.AT.rows > 0) launch_pass(ex_primal, mat_blocks(a.AT), early, s, a, first);
+    static void (*const pass[])(ExactIter, int) = {ex_primal<kExEarly>, ex_primal<kExChain>, ex_primal<kExRows>};
+    if (a.AT.rows > 0) launch_pass(pass[ex_pass(a, a.AT)], mat_blocks(a.AT), early, s, a, first);
 }
 void launch_exact_dual(const ExactIter& a, int first, cudaStream_t s, bool early) {
-    if (a.A.rows > 0) launch_pass(ex_dual, mat_blocks(a.A), early, s, a, first);
+    static void (*const pass[])(ExactIter, int) = {ex_dual<kExEarly>, ex_dual<kExChain>, ex_dual<kExRows>};
+    if (a.A.rows > 0) launch_pass(pass[ex_pass(a, a.A)], mat_blocks(a.A), early, s, a, first);
 }
 void launch_exact_check(const ExactCheck& a, cudaStream_t s) {
     const int g1 = mat_blocks(a.A) + mat_blocks(a.AT);
