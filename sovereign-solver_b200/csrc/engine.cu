@@ -375,14 +375,20 @@ int operator_norm(Ctx& c, int iterations, bool fast, double* out) {
     double *st = c.pw_st.p, *u = c.pw_u.p, *w = c.pw_w.p;
     int* stop = c.pw_stop.p;
     unsigned int* ticket = reinterpret_cast<unsigned int*>(stop + 1);
+    // Launched early, each of a large launch's CTAs waits on its own. An estimate,
+    // early / not: 60 x 150 0.48 / 0.69 ms, 100,000 x 250,000 (1.25M entries) 1.30
+    // / 1.42, transportation 701 x 1,499 (2.1M) 1.24 / 1.26; 200,000 x 500,000
+    // (4M) 2.29 / 2.23, transportation 2,000 x 5,000 (20M) 9.4 / 6.6.
+    const bool early = A.nnz < kEarlyNnz;
     for (int it = 0; it < iterations; ++it) {
-        const bool e = it > 0;  // the first launch follows fills and copies
+        const bool e = early && it > 0;  // the first launch follows fills and copies
+        const bool em = early && m > 0, en = early && n > 0;
         if (fast) launch_fast_pw_w(A, u, w, st, stop, e, s);
         else launch_pw_w(A, u, w, st, stop, e, s);
-        launch_pw_norms(w, nullptr, m, nullptr, nullptr, 0, false, c.pw_part.p, st, stop, ticket, m > 0, s);
-        if (fast) launch_fast_pw_u(AT, w, u, st, stop, m > 0, s);
-        else launch_pw_u(AT, w, u, st, stop, m > 0, s);
-        launch_pw_norms(u, nullptr, n, w, st + PW_INV_W, m, true, c.pw_part.p, st, stop, ticket, n > 0, s);
+        launch_pw_norms(w, nullptr, m, nullptr, nullptr, 0, false, c.pw_part.p, st, stop, ticket, em, s);
+        if (fast) launch_fast_pw_u(AT, w, u, st, stop, em, s);
+        else launch_pw_u(AT, w, u, st, stop, em, s);
+        launch_pw_norms(u, nullptr, n, w, st + PW_INV_W, m, true, c.pw_part.p, st, stop, ticket, en, s);
     }
     CK(cudaGetLastError());
     double estimate = 0.0;

@@ -369,6 +369,13 @@ int fast_launches_per_iteration(const FastIter<T>& a);
 // each, of a small or middling LP.
 template <class T>
 bool fast_early(const FastIter<T>& a);
+// LPs below this many entries launch the next pass early (the EARLY kernels):
+// an iteration of the mixed 500 x 1,200 LP 6.8 -> 4.2 us, FP64 2,000 x 5,000
+// 8.5 -> 5.4, mixed 50,000 x 120,000 13.3 -> 10.3, FP64 transportation 701 x
+// 1,499 (2.1M entries) 24.9 -> 23.3; above, passes run for tens of
+// microseconds and their gathers do better non-coherent. The power iteration's
+// launches have the same line (operator_norm).
+constexpr int64_t kEarlyNnz = int64_t{1} << 22;
 // Once per device, before the first launch and outside any stream capture:
 // records how many CTAs of the persistent iteration kernels are resident per
 // device (their grids). 0 on success.

@@ -832,13 +832,6 @@ inline PassPlan pass_plan(const DevCsr& M, int cap_long, int cap_slice, int cap_
     return p;
 }
 
-// LPs below this many entries launch the next pass early (the EARLY kernels):
-// an iteration of the mixed 500 x 1,200 LP 6.8 -> 4.2 us, FP64 2,000 x 5,000
-// 8.5 -> 5.4, mixed 50,000 x 120,000 13.3 -> 10.3, FP64 transportation 701 x
-// 1,499 (2.1M entries) 24.9 -> 23.3; above, passes run for tens of
-// microseconds and their gathers do better non-coherent.
-constexpr int64_t kEarlyNnz = int64_t{1} << 22;
-
 // Kernels one pass over M launches besides the flag reset.
 inline int pass_launches(const DevCsr& M0) {
     const PassPlan p = pass_plan(pass_matrix(M0), 1, 1, 1);
