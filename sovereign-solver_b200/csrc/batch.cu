@@ -640,10 +640,8 @@ int batch_plan(BatchCtx& c, BatchCtx::Plan** out) {
     bool& ready = c.resident_ready[std::is_same<T, float>::value ? 0 : 1];
     if (!ready) init_resident_kernels<T>();
     ready = true;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     ResPlan r;
-    pl.fits = plan_resident<T>(c.parts, lanes_log2(c.bin_vw[1]), lanes_log2(c.bin_vw[0]), c.halpern, sms, r);
+    pl.fits = plan_resident<T>(c.parts, lanes_log2(c.bin_vw[1]), lanes_log2(c.bin_vw[0]), c.halpern, r);
     if (pl.fits) {
         pl.classes = r.classes;
         pl.far_bytes = static_cast<size_t>(r.far_bytes);

@@ -180,7 +180,7 @@ struct ResStreams {
 // False where some instance fits no cluster in precision T. lgt, lga: log2 of
 // the lanes per row of A^T's and of A's rows.
 template <class T>
-bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, int sms, ResPlan& plan);
+bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, ResPlan& plan);
 // n_periods check periods from iteration iter0 on, then `tail` iterations.
 template <class T>
 cudaError_t launch_batch_resident(const std::vector<ResClass>& classes, const ResBuffers& buf, int lgt, int lga,

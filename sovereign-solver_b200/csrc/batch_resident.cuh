@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <vector>
 
 #include "batch_device.cuh"
@@ -286,37 +287,40 @@ cudaError_t launch_class(const ResClass& c, const BatchView& b, const Iterates<T
     return run(batch_resident<T, 1024, false>);
 }
 
-// The largest cluster the device schedules at the largest shared memory.
+// The largest cluster the device schedules at the largest shared memory, and how
+// many of 1, 2, ... 16 CTAs at once (on a B200 148, 74, 33, 15, 7).
 std::atomic<int> g_res_cluster{0};
+std::atomic<int> g_res_active[5];
+// Instances of class c at once.
+int res_at_once(int c, int size) {
+    int q = 0;
+    while ((1 << q) < size) ++q;
+    return g_res_active[q] * (c == 0 ? 4 : c == 1 ? 2 : 1);
+}
 
 }  // namespace
 
 template <class T>
 void init_resident_kernels() {
-    const int c[4] = {res_largest_cluster(batch_resident<T, 1024, false>, 1024),
-                      res_largest_cluster(batch_resident<T, 1024, true>, 1024),
+    int active[2][5] = {};
+    const int c[4] = {res_largest_cluster(batch_resident<T, 1024, false>, 1024, active[0]),
+                      res_largest_cluster(batch_resident<T, 1024, true>, 1024, active[1]),
                       res_largest_cluster(batch_resident<T, 512, false>, 512),
                       res_largest_cluster(batch_resident<T, 256, false>, 256)};
+    for (int q = 0; q < 5; ++q) g_res_active[q] = std::min(active[0][q], active[1][q]);
     g_res_cluster = *std::min_element(c, c + 4) == 0 ? 0 : std::min(c[0], c[1]);
 }
-
 // Classes of like CTAs, tried in the order of their CTAs; the largest instances
 // first (a class's launch ends with its last instance).
 constexpr ResClass kClasses[kResClasses] = {
     {1, 256}, {1, 512}, {1, 1024}, {1, 1024, 0, 0, 0, true}, {2, 1024}, {2, 1024, 0, 0, 0, true},
     {4, 1024}, {4, 1024, 0, 0, 0, true}, {8, 1024}, {8, 1024, 0, 0, 0, true}, {16, 1024, 0, 0, 0, true}};
-// ... of an instance of nnz entries. `packed`: the batch has more instances
-// than fill the GPU, so what counts is SM time: the fewest CTAs that hold the
-// instance at up to kResPacked entries each, its entries in global memory where
-// they do not fit. Otherwise each instance's own time counts: the CTAs that
-// hold its entries, at most eight (60 KB to all CTAs of a cluster: 3,500 cycles
-// for eight, 4,600 for sixteen). 256 FP32 instances of 50 x 100 to 5,000 x
-// 15,000, a check period of 40 iterations: 1,483 us at their own time's
-// clusters; packed with 8,192 / 16,384 / 32,768 / 65,536 entries a CTA 1,483 /
-// 1,244 / 1,184 / 1,218 us.
-constexpr int64_t kResPacked = 32768;
+// ... of an instance. per = 0: its own time counts, the CTAs that hold its
+// entries, at most eight (60 KB to all CTAs of a cluster: 3,500 cycles for
+// eight, 4,600 for sixteen). Else SM time does: the fewest CTAs that hold it at
+// up to `per` entries each, its entries in global memory where they do not fit.
 template <class T>
-int res_class(const ResParts& pt, const ResParts& pa, int lgt, int lga, bool halpern, bool packed, ResSize* z) {
+int res_class(const ResParts& pt, const ResParts& pa, int lgt, int lga, bool halpern, int64_t per, ResSize* z) {
     const int32_t nnz = pa.nz[kResMaxCluster];
     int last = -1;
     for (int c = 2; c < kResClasses; ++c) {
@@ -325,18 +329,44 @@ int res_class(const ResParts& pt, const ResParts& pa, int lgt, int lga, bool hal
         const ResSize y = k.far ? res_size<T, true>(pt, pa, k.size, lgt, lga, halpern)
                                 : res_size<T, false>(pt, pa, k.size, lgt, lga, halpern);
         if (y.smem > kResMaxSmem) continue;
-        if (!packed && k.far && k.size < 8) continue;
+        if (per == 0 && k.far && k.size < 8) continue;
         last = c;
         *z = y;
-        if (!packed || k.size >= 8 || nnz <= kResPacked * k.size) break;
+        if (per == 0 || k.size >= 8 || nnz <= per * k.size) break;
     }
     if (last == 2 && nnz <= 3000 && z->smem <= kResMaxSmem / 4) return 0;   // four to an SM
     if (last == 2 && nnz <= 12000 && z->smem <= kResMaxSmem / 2) return 1;  // two
     return last;
 }
 
+// Each instance at its own time if all of them run at once that way; else at
+// the fewest entries a CTA with which they do; else, with more instances than
+// that, at 32,768. FP32, a check period of 40 iterations of 256 instances of 50
+// x 100 to 5,000 x 15,000: 1,483 us at their own time's clusters; at 8,192 /
+// 16,384 / 32,768 / 65,536 entries a CTA 1,483 / 1,244 / 1,184 / 1,218 us. Where
+// they just do not run at once at their own time's clusters, an iteration there
+// / here: 20 FP32 instances of 3,000 x 9,000 19.5 / 11.6 us, 16 FP64 ones of
+// 1,000 x 4,000 with 20 entries a column 18.2 / 13.5, of 300 x 10,000 20.0 /
+// 12.2.
+constexpr int64_t kResPer[] = {0, 4096, 8192, 16384, 32768};
+
+// The kernels over all instances, us an iteration: 9 and what their entries and
+// rows take, and a CTA along the longest row: within 15% of what batches of 1 to
+// 64 instances of 300 x 10,000 to 10,000 x 23,000 measured, and badly scaled ones.
 template <class T>
-bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, int sms, ResPlan& plan) {
+double over_all_us(const std::vector<ResParts>& parts) {
+    constexpr bool f32 = std::is_same<T, float>::value;
+    double nnz = 0.0, rows = 0.0, longest = 0.0;
+    for (const ResParts& p : parts) {
+        nnz += 0.5 * p.nz[kResMaxCluster];
+        rows += p.row[kResMaxCluster];
+        longest = std::max(longest, static_cast<double>(p.longest_row));
+    }
+    return 9.0 + (f32 ? 9.5e-6 : 13.5e-6) * nnz + (f32 ? 12e-6 : 13e-6) * rows + 6e-3 * longest;
+}
+
+template <class T>
+bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool halpern, ResPlan& plan) {
     plan = ResPlan{};
     const size_t count = parts.size() / 2;
     if (g_res_cluster == 0) return false;
@@ -346,18 +376,27 @@ bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool ha
     };
     std::vector<Item> items(count);
     ResClass all[kResClasses];
-    bool packed = false;
-    for (int pass = 0; pass < 2; ++pass) {
+    // the longest row of more than kResLongRow entries in global memory, and what
+    // of the GPU the instances with such rows take at once
+    constexpr int kResLongRow = 2048;
+    int far_row = 0;
+    double far_fill = 0.0;
+    for (const int64_t per : kResPer) {
         std::copy(kClasses, kClasses + kResClasses, all);
         plan.far_bytes = 0;
-        int64_t quarters = 0;  // of SMs that all instances at once would fill
+        far_row = 0;
+        far_fill = 0.0;
+        double fill = 0.0;  // of the GPU, by all instances at once
         for (size_t k = 0; k < count; ++k) {
             const ResParts &pt = parts[2 * k], &pa = parts[2 * k + 1];
             ResSize z;
-            const int cls = res_class<T>(pt, pa, lgt, lga, halpern, packed, &z);
+            const int cls = res_class<T>(pt, pa, lgt, lga, halpern, per, &z);
             if (cls < 0) return false;
             items[k] = {static_cast<int32_t>(k), pa.nz[kResMaxCluster], cls, ResFar{}};
             if (all[cls].far) {
+                const int row = std::max(pt.longest_row, pa.longest_row);
+                if (row > kResLongRow) far_fill += 1.0 / res_at_once(cls, all[cls].size);
+                if (row > kResLongRow) far_row = std::max(far_row, row);
                 // whole 16-byte vectors per CTA
                 for (int w = 0; w < 2; ++w) items[k].far.entries[w] = (z.entries[w] + 7u) / 8u * 8u;
                 items[k].far.base = plan.far_bytes;
@@ -367,11 +406,24 @@ bool plan_resident(const std::vector<ResParts>& parts, int lgt, int lga, bool ha
             }
             all[cls].count += 1;
             all[cls].smem = std::max(all[cls].smem, z.smem);
-            quarters += cls == 0 ? 1 : cls == 1 ? 2 : 4 * all[cls].size;
+            fill += 1.0 / res_at_once(cls, all[cls].size);
         }
-        if (packed || quarters <= 4 * static_cast<int64_t>(sms)) break;
-        packed = true;
+        if (fill <= 1.0) break;
     }
+    // Not where the clusters alone would take longer than the kernels over all
+    // instances: several waves of sixteen CTAs (11 us an iteration each: 64 FP32
+    // instances of 10,000 x 23,000 102 us on clusters, 72 not), or a warp along a
+    // long row from global memory (FP64, badly scaled: 4,000 x 9,000 with a row of
+    // 6,000 entries 55 / 47 us, 40 of 2,000 x 5,000 with one of 3,500 56 / 47, 150
+    // of them in two waves 145 / 126; shorter rows are not what takes the time: 300
+    // of 500 x 1,200 with one of 870 49 / 72; in FP32 the clusters are as fast or
+    // faster).
+    const ResClass& wide = all[kResClasses - 1];
+    const int waves = wide.count > 0 ? (wide.count - 1) / res_at_once(kResClasses - 1, wide.size) + 1 : 0;
+    double least = waves > 1 ? 11.0 * waves : 0.0;
+    if (!std::is_same<T, float>::value && far_row > 0)
+        least = std::max(least, std::ceil(far_fill) * (3.0 + 15e-3 * far_row));
+    if (least > over_all_us<T>(parts)) return false;
     std::sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
         return a.cls != b.cls ? a.cls > b.cls : a.nnz != b.nnz ? a.nnz > b.nnz : a.k < b.k;
     });

@@ -4,7 +4,7 @@
 namespace pdhg {
 
 template void init_resident_kernels<float>();
-template bool plan_resident<float>(const std::vector<ResParts>&, int, int, bool, int, ResPlan&);
+template bool plan_resident<float>(const std::vector<ResParts>&, int, int, bool, ResPlan&);
 template cudaError_t launch_batch_resident<float>(const std::vector<ResClass>&, const ResBuffers&, int, int,
                                                 const BatchView&, const Iterates<float>&, const BatchParams&, long long,
                                                 long long, long long, cudaStream_t, const ResStreams&);

@@ -94,7 +94,8 @@ constexpr int kResMaxCluster = 16;
 struct ResParts {
     int32_t row[kResMaxCluster + 1] = {};
     int32_t nz[kResMaxCluster + 1] = {};
-    int32_t longest = 0;  // entries of the longest row of at most kLongRow
+    int32_t longest = 0;      // entries of the longest row of at most kLongRow
+    int32_t longest_row = 0;  // ... of any row
 };
 // ... of one matrix, of at most kResPartRows rows (intake.cu), and of a batch's
 // matrices, whose rows are [off[k], off[k + 1]) of rp, into out[2 k + which].

@@ -275,17 +275,22 @@ __global__ void __launch_bounds__(kBlock) k_col_runs(const int32_t* ci, int32_t 
 constexpr int64_t kResRowWork = 8;
 __device__ void row_parts(const int32_t* rp, int32_t rows, ResParts& o) {
     const int q = threadIdx.x;
-    int longest = 0;
+    int longest[2] = {0, 0};
     for (int i = q; i < rows; i += kBlock) {
         const int len = rp[i + 1] - rp[i];
-        if (len <= kLongRow) longest = max(longest, len);
+        if (len <= kLongRow) longest[0] = max(longest[0], len);
+        longest[1] = max(longest[1], len);
     }
-    __shared__ int most;
-    if (q == 0) most = 0;
+    __shared__ int most[2];
+    if (q < 2) most[q] = 0;
     __syncthreads();
-    atomicMax(&most, longest);
+    atomicMax(&most[0], longest[0]);
+    atomicMax(&most[1], longest[1]);
     __syncthreads();
-    if (q == 0) o.longest = most;
+    if (q == 0) {
+        o.longest = most[0];
+        o.longest_row = most[1];
+    }
     if (q > kResMaxCluster) return;
     const int64_t base = rp[0];
     const int64_t want = (rp[rows] - base + kResRowWork * rows) * q / kResMaxCluster;

@@ -647,14 +647,17 @@ ResSize res_size(const ResParts& pt, const ResParts& pa, int c, int lgt, int lga
 }
 
 // Lets `kernel` use kResMaxSmem and clusters up to 16; the largest size (a
-// power of two) the device schedules that way, 0 on an error.
+// power of two) the device schedules that way, 0 on an error. active: how many
+// clusters of 1, 2, ... 16 CTAs with that much run at once (an SM each, and a
+// cluster's SMs near each other: fewer than the SMs would give).
 template <class K>
-int res_largest_cluster(K kernel, int threads) {
+int res_largest_cluster(K kernel, int threads, int* active = nullptr) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(kResMaxSmem)) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
         return 0;
-    for (int c = kResMaxCluster; c > 1; c /= 2) {
+    int largest = 1;
+    for (int c = 1, q = 0; c <= kResMaxCluster; c *= 2, ++q) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(c));
         cfg.blockDim = dim3(static_cast<unsigned>(threads));
@@ -666,10 +669,11 @@ int res_largest_cluster(K kernel, int threads) {
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) return c;
-        cudaGetLastError();
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) cudaGetLastError();
+        if (active != nullptr) active[q] = n;
+        if (n > 0) largest = c;
     }
-    return 1;
+    return largest;
 }
 
 template <class... P, class... Q>
