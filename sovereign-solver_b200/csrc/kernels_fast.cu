@@ -187,33 +187,44 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? PDHG_SHORT_MIN_CTAS :
         return;
     }
     // rounds of four entries per lane: the index and value loads of a round
-    // are all in flight before its gathers, the gathers before the adds; the
-    // first round's are loaded before the wait for the pass before
+    // are all in flight before its gathers, the gathers before the adds; EARLY
+    // loads the first round's before the wait for the pass before. The loop
+    // turned that way is the faster one in FP32 anyway (1,000,000 x 2,500,000:
+    // 115 -> 110 us an iteration), in FP64 it is not (badly scaled 500 x 1,200,
+    // rows of up to 512 entries: 8.3 -> 9.3).
     T acc = T(0);
-    int k0 = b + lane;
     int c[4];
     T v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int k = k0 + u * VW;
-        c[u] = k < e ? __ldcs(M.ci + k) : 0;
-        v[u] = k < e ? __ldcs(vals + k) : T(0);
-    }
-    if (EARLY) {
-        pass_wait();
-        if (lane == 0) epi_load_moving<T, PRIMAL>(in, a.it, r, first, fresh, hw);
-    }
-    for (;;) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (k0 + u * VW < e) acc += v[u] * gather_ld<EARLY>(xg + c[u]);
-        k0 += 4 * VW;
-        if (k0 >= e) break;
+    const auto load_round = [&](int k0) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int k = k0 + u * VW;
             c[u] = k < e ? __ldcs(M.ci + k) : 0;
             v[u] = k < e ? __ldcs(vals + k) : T(0);
+        }
+    };
+    const auto add_round = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u * VW < e) acc += v[u] * gather_ld<EARLY>(xg + c[u]);
+    };
+    if (EARLY || std::is_same<T, float>::value) {
+        int k0 = b + lane;
+        load_round(k0);
+        if (EARLY) {
+            pass_wait();
+            if (lane == 0) epi_load_moving<T, PRIMAL>(in, a.it, r, first, fresh, hw);
+        }
+        for (;;) {
+            add_round(k0);
+            k0 += 4 * VW;
+            if (k0 >= e) break;
+            load_round(k0);
+        }
+    } else {
+        for (int k0 = b + lane; k0 < e; k0 += 4 * VW) {
+            load_round(k0);
+            add_round(k0);
         }
     }
     if (VW > 1) acc = group_sum(acc, VW);
