@@ -129,7 +129,7 @@ struct MatDev {
     int64_t nnz_dense = 0;  // entries of the dense rows (columns computed)
     DBuf<int2> runs;        // column runs of rows of two entries, if in use
     int64_t nnz_runs = 0;   // entries whose columns they give
-    ResParts parts;         // of at most kResPartRows rows (else empty)
+    ResParts parts;         // if wanted (bin_matrix) and of at most kResPartRows rows, else empty
     DevCsr view() const {
         DevCsr d;
         d.rows = rows;
@@ -272,7 +272,8 @@ inline int build_items(const std::vector<int4>& ext, int min_len, int min_seg, i
 // row (about half the mean short-row length, a power of two in [1, 32]), the
 // warp-row list of the ordered kernels, and the throughput kernels' tiers:
 // short rows up to short_max, the two warp-row lists and the CTA work items.
-inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err) {
+// want_parts: M.parts too.
+inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err, bool want_parts = false) {
     cudaError_t e = M.long_rows.alloc(static_cast<size_t>(M.rows) + 1);
     if (e != cudaSuccess) return cuda_fail(err, e, "bin_matrix");
     if ((e = M.wrows.alloc(static_cast<size_t>(M.rows) + 1)) != cudaSuccess ||
@@ -283,7 +284,7 @@ inline int bin_matrix(MatDev& M, cudaStream_t s, std::string* err) {
     constexpr size_t kPartWords = (sizeof(ResParts) + 7) / 8;  // the parts travel with the counters
     if ((e = cnt.alloc(9 + kPartWords)) != cudaSuccess) return cuda_fail(err, e, "bin_matrix");
     cudaMemsetAsync(cnt.p, 0, 9 * sizeof(unsigned long long), s);
-    const bool parts = M.rows > 0 && M.rows <= kResPartRows;
+    const bool parts = want_parts && M.rows > 0 && M.rows <= kResPartRows;
     if (parts) launch_parts(M.rp.p, M.rows, reinterpret_cast<ResParts*>(cnt.p + 9), s);
     launch_bin(M.rp.p, M.rows, kLongRow, M.long_rows.p, cnt.p, s);
     launch_bin(M.rp.p, M.rows, kWarpRow, M.wrows.p, cnt.p + 3, s);
@@ -573,21 +574,22 @@ inline int build_dense_rows(MatDev& M, cudaStream_t s, std::string* err) {
 inline int build_col_runs(MatDev& M, cudaStream_t s, std::string* err) {
     const char* knob = std::getenv("PDHG_B200_DENSE_ROWS");  // "0": load every column index
     M.nnz_runs = 0;
-    M.runs.release();
-    if (M.rp_stride != 2 || (knob != nullptr && knob[0] == '0')) return PDHG_OK;
+    if (M.rp_stride != 2 || (knob != nullptr && knob[0] == '0')) {
+        M.runs.release();
+        return PDHG_OK;
+    }
     const size_t n = (static_cast<size_t>(M.rows) + 31) / 32;
-    if (M.runs.alloc(n) != cudaSuccess) {  // no room: the columns are loaded
+    if (M.runs.alloc(n + 1) != cudaSuccess) {  // no room: the columns are loaded
         M.runs.release();
         cudaGetLastError();
         return PDHG_OK;
     }
-    DBuf<unsigned long long> cnt;
+    unsigned long long* const cnt = reinterpret_cast<unsigned long long*>(M.runs.p + n);
     unsigned long long h = 0;
     cudaError_t e;
-    if ((e = cnt.alloc(1)) != cudaSuccess || (e = cudaMemsetAsync(cnt.p, 0, sizeof h, s)) != cudaSuccess)
-        return cuda_fail(err, e, "build_col_runs");
-    launch_col_runs(M.ci.p, M.rows, M.runs.p, cnt.p, s);
-    if ((e = cudaMemcpyAsync(&h, cnt.p, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+    if ((e = cudaMemsetAsync(cnt, 0, sizeof h, s)) != cudaSuccess) return cuda_fail(err, e, "build_col_runs");
+    launch_col_runs(M.ci.p, M.rows, M.runs.p, cnt, s);
+    if ((e = cudaMemcpyAsync(&h, cnt, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_fail(err, e, "build_col_runs");
     if (4 * h < 3 * n) M.runs.release();

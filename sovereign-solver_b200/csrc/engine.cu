@@ -273,9 +273,9 @@ int ensure_scaled(Ctx& c, const ScalingParams& sp) {
     pc.mark("scale: values");
     CK(to_float(c.As.v32, c.As.v64, s));
     CK(to_float(c.ATs.v32, c.ATs.v64, s));
-    int rc = bin_matrix(c.As, s, &c.err);
+    int rc = bin_matrix(c.As, s, &c.err, true);
     if (rc != PDHG_OK) return rc;
-    rc = bin_matrix(c.ATs, s, &c.err);
+    rc = bin_matrix(c.ATs, s, &c.err, true);
     if (rc != PDHG_OK) return rc;
     rc = build_slices(c.As, s, &c.err);
     if (rc != PDHG_OK) return rc;
