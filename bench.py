@@ -305,9 +305,9 @@ def barrier(world: int):
         dist.barrier()
 
 
-def traffic_from_profile() -> float | None:
-    """DRAM bytes per launch of the primal kernel from the committed ncu summary."""
-    path = os.path.join(ROOT, "profiles", "primal_transportation_10M.json")
+def traffic_from_profile(kernel: str) -> float | None:
+    """DRAM bytes per launch of the primal or dual pass from the committed ncu summary."""
+    path = os.path.join(ROOT, "profiles", f"{kernel}_transportation_10M.json")
     try:
         with open(path) as f:
             return float(json.load(f)["dram_bytes_per_launch"])
@@ -790,7 +790,7 @@ def main() -> None:
     roofline = {"bound": "hbm", "kernel": dom["name"], "achieved": achieved,
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                 "peak_source": peaks["source"],
-                "traffic": traffic_from_profile() if dom["name"] == "primal" else None,
+                "traffic": traffic_from_profile(dom["name"]),
                 "algorithmic_bytes_per_launch": dom["bytes"],
                 "bytes_note": "this LP's: the row pointer (every column has 2 entries) and the "
                               "column bounds (all 0 <= x) carry no information and are not loaded",
